@@ -141,7 +141,8 @@ def _design(seed, nx, ny, nz, volfrac):
     d = torch.minimum(torch.minimum(z + 0 * x, (z - top).abs()), torch.minimum(web[0], web[1]))
     d = (d * torch.exp(0.25 * _smooth_field(g, (nx, nz, ny), max(2.0, ny / 16)))).reshape(-1)
     cut = torch.sort(d).values[int(volfrac * (d.numel() - 1))]
-    return (0.03 + 0.97 * torch.sigmoid(3.0 * (1.0 - d / cut))).contiguous()
+    rim = torch.clamp(cut / 3.0, min=1.2 / nz)   # about an element at least, as the filter leaves it
+    return (0.03 + 0.97 * torch.sigmoid((cut - d) / rim)).contiguous()
 
 
 def _cell(seed, nx, ny, nz):
