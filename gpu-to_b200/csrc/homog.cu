@@ -10,8 +10,11 @@
 //    (i, j, k) has the corners (i + x_a, j + y_a, k + z_a) mod n in the
 //    reference's local order.  Node 0 is held (its three dofs) to remove the
 //    rigid translations, the periodic operator's only null space;
-//  * vectors: [dof][6] with dof = 3 node + d, the six load cases of a dof
-//    next to each other, so one thread applies the operator to all six;
+//  * vectors: nine planes of load-case pairs, plane 3 d + p holding component
+//    d of cases 2p and 2p + 1 as one float2 / double2 per node, so that a warp
+//    along y reads and writes whole 128-byte lines in every kernel (with the
+//    six cases of a dof adjacent, a warp's loads were 72 or 144 bytes apart
+//    and the sweeps were bound by L1 wavefronts);
 //  * load case r (Voigt xx, yy, zz, yz, xz, xy; engineering shears): the
 //    fluctuation chi_r solves K chi_r = -sum_e CX_e Ke u0_r, u0_r the affine
 //    field of unit strain r at an element's local corners;
@@ -66,129 +69,206 @@ template <> __device__ __forceinline__ float pke<float>(int idx) { return cPKe32
 
 enum PMode { P_APPLY = 0, P_DEFECT = 1, P_JACOBI = 2, P_PRE = 3 };
 
-// One operator sweep over all six load cases, thread per node.  Modes as the
-// fine sweeps: K u (with the per-case p'q partials), f - K u, damped Jacobi
-// z = u + omega (f - K u) / diag, and the pre-relaxation that starts from
-// u = prerelax f / diag.  Node 0's dofs are held at zero residual.
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256)
-psweep_kernel(PGrid g, const T *__restrict__ CX, const T *__restrict__ u, const T *__restrict__ f,
-              const T *__restrict__ rdiag, T *__restrict__ out, T omega, T prerelax, double *__restrict__ partial,
+template <typename T> struct Pair;
+template <> struct Pair<float> {
+    using V = float2;
+};
+template <> struct Pair<double> {
+    using V = double2;
+};
+__device__ __forceinline__ float2 pfma(float b, float2 v, float2 a) { return __ffma2_rn(make_float2(b, b), v, a); }
+__device__ __forceinline__ double2 pfma(double b, double2 v, double2 a)
+{
+    return make_double2(fma(b, v.x, a.x), fma(b, v.y, a.y));
+}
+__device__ __forceinline__ float2 pscale(float b, float2 v) { return make_float2(b * v.x, b * v.y); }
+__device__ __forceinline__ double2 pscale(double b, double2 v) { return make_double2(b * v.x, b * v.y); }
+
+// One operator sweep over all six load cases, thread per NX nodes along x.
+// Modes as the fine sweeps: K u (with the per-case p'q partials), f - K u,
+// damped Jacobi z = u + omega (f - K u) / diag, and the pre-relaxation that
+// starts from u = prerelax f / diag.  Node 0's dofs are held at zero residual.
+//
+// Per node 576 FMAs form the 27 blocks and 1458 apply them to the six cases
+// (as 729 paired FP32 instructions): 118 us of FMA pipe at 128^3 in FP32 and
+// 237 us in FP64, above the 70 and 93 us of HBM traffic.  The 27 x 9
+// neighbour pairs come through L1, coalesced along y; a CTA covers 32 (y) x 8
+// (z) columns so that most of them hit (the apply takes 256 consecutive nodes,
+// the order of its p'q sums).  In FP32 a thread takes two nodes on large
+// grids, which share two of their three neighbour planes (18 instead of 27
+// plane reads per node).  The neighbours' loads are kept three at a time:
+// left to itself the compiler hoists them all and spills.
+// Measured at 128^3: FP32 Jacobi sweep 232 us (FMA pipe 54 % active; 727 us
+// with the cases of a dof adjacent, bound by L1 wavefronts), FP64 apply 402 us
+// (1272 us); the same bits.  One node per thread at three CTAs per SM gave the
+// same time as two nodes at two CTAs, two nodes at three CTAs spilled (6 %
+// slower per solve), and keeping the node's own values in registers for the
+// epilogue cost the FP64 apply its second CTA (4 % slower per solve).
+template <typename T, int MODE, int NX>
+__global__ void __launch_bounds__(256, 2)
+psweep_kernel(PGrid g, int ty, int ntj, int nt, const T *__restrict__ CX, const T *__restrict__ u_, const T *__restrict__ f_,
+              const T *__restrict__ rdiag, T *__restrict__ out_, T omega, T prerelax, double *__restrict__ partial,
               const int *__restrict__ done)
 {
     if (done && *done) return;
-    const long long nn = g.nnod();
-    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    double dsum[NR];
+    using V = typename Pair<T>::V;
+    const V *__restrict__ u = reinterpret_cast<const V *>(u_);
+    const V *__restrict__ f = reinterpret_cast<const V *>(f_);
+    V *__restrict__ out = reinterpret_cast<V *>(out_);
+    const int nn = (int)g.nnod();
+    const size_t N = (size_t)nn;
+    int i0, j, k;
+    bool mine;
+    if (MODE == P_APPLY) {   // 256 consecutive nodes: the p'q partials sum in node order
+        const int n = (int)(blockIdx.x * 256 + threadIdx.x), t = n / g.ny;
+        j = n - t * g.ny;
+        i0 = t / g.nz;
+        k = t - i0 * g.nz;
+        mine = n < nn;
+    } else {
+        const int tz = 256 / ty;
+        const int bi = (int)(blockIdx.x / (unsigned)nt), bt = (int)blockIdx.x - bi * nt;   // x step, (y, z) tile
+        const int tk = bt / ntj, tj = bt - tk * ntj;
+        const int lk = (int)threadIdx.x / ty;
+        j = tj * ty + ((int)threadIdx.x - lk * ty);
+        k = tk * tz + lk;
+        i0 = bi * NX;
+        mine = j < g.ny && lk < tz && k < g.nz;
+    }
+    V dsum[3];
 #pragma unroll
-    for (int r = 0; r < NR; ++r) dsum[r] = 0.0;
-    if (n < nn) {
-        const int j = (int)(n % g.ny);
-        const long long t = n / g.ny;
-        const int k = (int)(t % g.nz), i = (int)(t / g.nz);
-        const int xi[3] = {wrap(i - 1, g.nx), i, wrap(i + 1, g.nx)};
+    for (int p = 0; p < 3; ++p) dsum[p].x = dsum[p].y = T(0);
+    if (mine) {
+        const int ps = g.nz * g.ny;
         const int yj[3] = {wrap(j - 1, g.ny), j, wrap(j + 1, g.ny)};
-        const int zk[3] = {wrap(k - 1, g.nz), k, wrap(k + 1, g.nz)};
-        // the eight elements around the node: element (i - 1 + ex, j - 1 + ey, k - 1 + ez)
-        T cxe[8];
+        const int zk[3] = {wrap(k - 1, g.nz) * g.ny, k * g.ny, wrap(k + 1, g.nz) * g.ny};
+        int xi[NX + 2];   // planes i0 - 1 .. i0 + NX
+        xi[0] = wrap(i0 - 1, g.nx) * ps;
 #pragma unroll
-        for (int ex = 0; ex < 2; ++ex)
+        for (int q = 1; q < NX + 2; ++q) {
+            int v = i0 + q - 1;
+            v = v >= g.nx ? v - g.nx : v;
+            xi[q] = v * ps;
+        }
+        // the elements around the nodes: element (i0 - 1 + ex, j - 1 + ey, k - 1 + ez)
+        T cxe[NX + 1][2][2];
+#pragma unroll
+        for (int ex = 0; ex < NX + 1; ++ex)
 #pragma unroll
             for (int ey = 0; ey < 2; ++ey)
 #pragma unroll
-                for (int ez = 0; ez < 2; ++ez) cxe[(ex * 2 + ey) * 2 + ez] = CX[g.node(xi[ex], yj[ey], zk[ez])];
-        T acc[3][NR], uc[3][NR];
+                for (int ez = 0; ez < 2; ++ez) cxe[ex][ey][ez] = CX[xi[ex] + zk[ez] + yj[ey]];
+        V acc[NX][9];   // [3 d + p]
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
+        for (int m = 0; m < NX; ++m)
 #pragma unroll
-            for (int r = 0; r < NR; ++r) acc[d][r] = T(0);
+            for (int q = 0; q < 9; ++q) acc[m][q].x = acc[m][q].y = T(0);
 #pragma unroll
-        for (int dx = -1; dx <= 1; ++dx)
+        for (int px = 0; px < NX + 2; ++px)
 #pragma unroll
-            for (int dy = -1; dy <= 1; ++dy)
+            for (int dy = -1; dy <= 1; ++dy) {
+                asm volatile("" ::: "memory");   // keep the loads of three neighbours in flight, not of all
 #pragma unroll
                 for (int dz = -1; dz <= 1; ++dz) {
-                    // 3x3 block between the node and neighbour (dx, dy, dz)
-                    T B[3][3];
-#pragma unroll
-                    for (int a = 0; a < 3; ++a)
-#pragma unroll
-                        for (int b = 0; b < 3; ++b) B[a][b] = T(0);
-#pragma unroll
-                    for (int ex = 0; ex < 2; ++ex)
-#pragma unroll
-                        for (int ey = 0; ey < 2; ++ey)
-#pragma unroll
-                            for (int ez = 0; ez < 2; ++ez) {
-                                const int bx = dx + 1 - ex, by = dy + 1 - ey, bz = dz + 1 - ez;
-                                if (bx < 0 || bx > 1 || by < 0 || by > 1 || bz < 0 || bz > 1) continue;
-                                const int ca = corner_of(1 - ex, 1 - ey, 1 - ez), cb = corner_of(bx, by, bz);
-                                const T c = cxe[(ex * 2 + ey) * 2 + ez];
-#pragma unroll
-                                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                                    for (int b = 0; b < 3; ++b)
-                                        B[a][b] = fma(c, pke<T>((3 * ca + a) * 24 + 3 * cb + b), B[a][b]);
-                            }
-                    const long long nb = g.node(xi[dx + 1], yj[dy + 1], zk[dz + 1]);
-                    T v[3][NR];
+                    const int nb = xi[px] + zk[dz + 1] + yj[dy + 1];
+                    V v[9];
 #pragma unroll
                     for (int b = 0; b < 3; ++b) {
-                        const long long base = (3 * nb + b) * NR;
                         if (MODE == P_PRE) {
-                            const T s = prerelax * rdiag[3 * nb + b];
+                            const T s = prerelax * rdiag[3 * (size_t)nb + b];
 #pragma unroll
-                            for (int r = 0; r < NR; ++r) v[b][r] = s * f[base + r];
+                            for (int p = 0; p < 3; ++p) v[3 * b + p] = pscale(s, f[(3 * b + p) * N + nb]);
                         } else {
 #pragma unroll
-                            for (int r = 0; r < NR; ++r) v[b][r] = u[base + r];
+                            for (int p = 0; p < 3; ++p) v[3 * b + p] = u[(3 * b + p) * N + nb];
                         }
                     }
-                    if (dx == 0 && dy == 0 && dz == 0) {
 #pragma unroll
-                        for (int b = 0; b < 3; ++b)
+                    for (int m = 0; m < NX; ++m) {
+                        const int dx = px - 1 - m;   // offset from node i0 + m
+                        if (dx < -1 || dx > 1) continue;
+                        // 3x3 block between the node and neighbour (dx, dy, dz)
+                        T B[3][3];
 #pragma unroll
-                            for (int r = 0; r < NR; ++r) uc[b][r] = v[b][r];
+                        for (int a = 0; a < 3; ++a)
+#pragma unroll
+                            for (int b = 0; b < 3; ++b) B[a][b] = T(0);
+#pragma unroll
+                        for (int ex = 0; ex < 2; ++ex)
+#pragma unroll
+                            for (int ey = 0; ey < 2; ++ey)
+#pragma unroll
+                                for (int ez = 0; ez < 2; ++ez) {
+                                    const int bx = dx + 1 - ex, by = dy + 1 - ey, bz = dz + 1 - ez;
+                                    if (bx < 0 || bx > 1 || by < 0 || by > 1 || bz < 0 || bz > 1) continue;
+                                    const int ca = corner_of(1 - ex, 1 - ey, 1 - ez), cb = corner_of(bx, by, bz);
+                                    const T c = cxe[m + ex][ey][ez];
+#pragma unroll
+                                    for (int a = 0; a < 3; ++a)
+#pragma unroll
+                                        for (int b = 0; b < 3; ++b)
+                                            B[a][b] = fma(c, pke<T>((3 * ca + a) * 24 + 3 * cb + b), B[a][b]);
+                                }
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+#pragma unroll
+                            for (int b = 0; b < 3; ++b)
+#pragma unroll
+                                for (int p = 0; p < 3; ++p)
+                                    acc[m][3 * a + p] = pfma(B[a][b], v[3 * b + p], acc[m][3 * a + p]);
                     }
-#pragma unroll
-                    for (int a = 0; a < 3; ++a)
-#pragma unroll
-                        for (int b = 0; b < 3; ++b)
-#pragma unroll
-                            for (int r = 0; r < NR; ++r) acc[a][r] = fma(B[a][b], v[b][r], acc[a][r]);
                 }
-        const bool held = n == 0;
+            }
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const long long base = (3 * n + d) * NR;
+        for (int m = 0; m < NX; ++m) {
+            if (i0 + m >= g.nx) break;
+            const int n = (i0 + m) * ps + k * g.ny + j;
+            const bool held = n == 0;
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                if (MODE == P_APPLY) {
-                    const T q = held ? T(0) : acc[d][r];
-                    out[base + r] = q;
-                    dsum[r] = fma((double)uc[d][r], (double)q, dsum[r]);
-                } else if (MODE == P_DEFECT) {
-                    out[base + r] = held ? T(0) : f[base + r] - acc[d][r];
-                } else {
-                    const T res = held ? T(0) : f[base + r] - acc[d][r];
-                    out[base + r] = uc[d][r] + omega * res * rdiag[3 * n + d];
+            for (int d = 0; d < 3; ++d) {
+                const T rd = (MODE == P_JACOBI || MODE == P_PRE) ? rdiag[3 * (size_t)n + d] : T(0);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const size_t at = (3 * d + p) * N + n;
+                    const V ku = acc[m][3 * d + p];
+                    // the node's own value, read again (L1): keeping it cost registers that a second CTA needs
+                    const V uu = MODE == P_PRE ? pscale(prerelax * rd, f[at]) : u[at];
+                    V o;
+                    if (MODE == P_APPLY) {
+                        o.x = held ? T(0) : ku.x;
+                        o.y = held ? T(0) : ku.y;
+                        dsum[p].x = fma(uu.x, o.x, dsum[p].x);
+                        dsum[p].y = fma(uu.y, o.y, dsum[p].y);
+                    } else {
+                        const V fv = f[at];
+                        o.x = held ? T(0) : fv.x - ku.x;
+                        o.y = held ? T(0) : fv.y - ku.y;
+                        if (MODE != P_DEFECT) {
+                            o.x = fma(omega * o.x, rd, uu.x);
+                            o.y = fma(omega * o.y, rd, uu.y);
+                        }
+                    }
+                    out[at] = o;
                 }
             }
         }
     }
-    if (MODE == P_APPLY && partial) {
+    if (MODE == P_APPLY && partial) {   // partial[CTA][case]
         __shared__ double red[8][NR];
+        double ds[NR];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) ds[2 * p] = (double)dsum[p].x, ds[2 * p + 1] = (double)dsum[p].y;
 #pragma unroll
         for (int r = 0; r < NR; ++r)
-            for (int o = 16; o > 0; o >>= 1) dsum[r] += __shfl_xor_sync(0xffffffffu, dsum[r], o);
+            for (int o = 16; o > 0; o >>= 1) ds[r] += __shfl_xor_sync(0xffffffffu, ds[r], o);
         if ((threadIdx.x & 31) == 0)
 #pragma unroll
-            for (int r = 0; r < NR; ++r) red[threadIdx.x >> 5][r] = dsum[r];
+            for (int r = 0; r < NR; ++r) red[threadIdx.x >> 5][r] = ds[r];
         __syncthreads();
         if (threadIdx.x < NR) {
             double s = 0.0;
             for (int w = 0; w < 8; ++w) s += red[w][threadIdx.x];
-            partial[blockIdx.x * NR + threadIdx.x] = s;
+            partial[(size_t)blockIdx.x * NR + threadIdx.x] = s;
         }
     }
 }
@@ -230,19 +310,21 @@ __global__ void pcoarse_cx_kernel(PGrid gc, const double *__restrict__ CXf, doub
 
 // Full-weighting restriction (the transpose of the trilinear prolongation):
 // coarse node (I, J, K) gathers fine nodes (2I + dx, ...) with weights
-// 1, 1/2 per direction; node 0 gets zero.
-__global__ void prestrict_kernel(PGrid gc, const float *__restrict__ rf, float *__restrict__ fc, const int *done)
+// 1, 1/2 per direction; node 0 gets zero.  Thread per coarse node and
+// component (blockIdx.y), the three load-case pairs of that component.
+__global__ void __launch_bounds__(256)
+prestrict_kernel(PGrid gc, const float *__restrict__ rf, float *__restrict__ fc, const int *done)
 {
     if (done && *done) return;
-    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= gc.nnod()) return;
+    const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x), nc = (int)gc.nnod();
+    if (n >= nc) return;
     const PGrid gf{2 * gc.nx, 2 * gc.ny, 2 * gc.nz};
-    const int J = (int)(n % gc.ny);
-    const long long t = n / gc.ny;
-    const int K = (int)(t % gc.nz), I = (int)(t / gc.nz);
-    float acc[3 * NR];
+    const size_t Nf = (size_t)gf.nnod();
+    const float2 *src = reinterpret_cast<const float2 *>(rf) + 3 * blockIdx.y * Nf;
+    const int J = n % gc.ny, t = n / gc.ny, K = t % gc.nz, I = t / gc.nz;
+    float2 acc[3];
 #pragma unroll
-    for (int q = 0; q < 3 * NR; ++q) acc[q] = 0.f;
+    for (int p = 0; p < 3; ++p) acc[p] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int dx = -1; dx <= 1; ++dx)
 #pragma unroll
@@ -250,44 +332,57 @@ __global__ void prestrict_kernel(PGrid gc, const float *__restrict__ rf, float *
 #pragma unroll
             for (int dy = -1; dy <= 1; ++dy) {
                 const float w = (dx ? 0.5f : 1.f) * (dy ? 0.5f : 1.f) * (dz ? 0.5f : 1.f);
-                const long long fn = gf.node(wrap(2 * I + dx, gf.nx), wrap(2 * J + dy, gf.ny), wrap(2 * K + dz, gf.nz));
-                const float *src = rf + fn * 3 * NR;
+                const size_t fn = (size_t)gf.node(wrap(2 * I + dx, gf.nx), wrap(2 * J + dy, gf.ny),
+                                                  wrap(2 * K + dz, gf.nz));
 #pragma unroll
-                for (int q = 0; q < 3 * NR; ++q) acc[q] = fmaf(w, src[q], acc[q]);
+                for (int p = 0; p < 3; ++p) acc[p] = pfma(w, src[p * Nf + fn], acc[p]);
             }
-    float *dst = fc + n * 3 * NR;
+    float2 *dst = reinterpret_cast<float2 *>(fc) + 3 * blockIdx.y * (size_t)nc + n;
 #pragma unroll
-    for (int q = 0; q < 3 * NR; ++q) dst[q] = n == 0 ? 0.f : acc[q];
+    for (int p = 0; p < 3; ++p) dst[p * (size_t)nc] = n == 0 ? make_float2(0.f, 0.f) : acc[p];
 }
 
-// u_f += P u_c (trilinear, periodic); node 0 stays zero.
-__global__ void pprolong_kernel(PGrid gf, const float *__restrict__ uc, float *__restrict__ uf, const int *done)
+// u_f += P u_c (trilinear, periodic); node 0 stays zero.  Thread per fine
+// node and component (blockIdx.y).
+__global__ void __launch_bounds__(256)
+pprolong_kernel(PGrid gf, const float *__restrict__ uc, float *__restrict__ uf, const int *done)
 {
     if (done && *done) return;
-    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= gf.nnod()) return;
+    const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x), nf = (int)gf.nnod();
+    if (n >= nf) return;
     const PGrid gc{gf.nx / 2, gf.ny / 2, gf.nz / 2};
-    const int j = (int)(n % gf.ny);
-    const long long t = n / gf.ny;
-    const int k = (int)(t % gf.nz), i = (int)(t / gf.nz);
+    const size_t Nc = (size_t)gc.nnod();
+    const float2 *src = reinterpret_cast<const float2 *>(uc) + 3 * blockIdx.y * Nc;
+    float2 *dst = reinterpret_cast<float2 *>(uf) + 3 * blockIdx.y * (size_t)nf + n;
+    const int j = n % gf.ny, t = n / gf.ny, k = t % gf.nz, i = t / gf.nz;
+    float2 old[3];
+#pragma unroll
+    for (int p = 0; p < 3; ++p) old[p] = dst[p * (size_t)nf];
     const int ix[2] = {i >> 1, (i & 1) ? wrap((i >> 1) + 1, gc.nx) : (i >> 1)};
     const int iy[2] = {j >> 1, (j & 1) ? wrap((j >> 1) + 1, gc.ny) : (j >> 1)};
     const int iz[2] = {k >> 1, (k & 1) ? wrap((k >> 1) + 1, gc.nz) : (k >> 1)};
     const int mx = (i & 1) ? 2 : 1, my = (j & 1) ? 2 : 1, mz = (k & 1) ? 2 : 1;
     const float w = 1.f / (float)(mx * my * mz);
-    float acc[3 * NR];
+    float2 acc[3];
 #pragma unroll
-    for (int q = 0; q < 3 * NR; ++q) acc[q] = 0.f;
-    for (int a = 0; a < mx; ++a)
-        for (int c = 0; c < mz; ++c)
-            for (int b = 0; b < my; ++b) {
-                const float *src = uc + gc.node(ix[a], iy[b], iz[c]) * 3 * NR;
+    for (int p = 0; p < 3; ++p) acc[p] = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int q = 0; q < 3 * NR; ++q) acc[q] += src[q];
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                if (a >= mx || c >= mz || b >= my) continue;
+                const size_t q = (size_t)gc.node(ix[a], iy[b], iz[c]);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const float2 v = src[p * Nc + q];
+                    acc[p].x += v.x;
+                    acc[p].y += v.y;
+                }
             }
-    float *dst = uf + n * 3 * NR;
 #pragma unroll
-    for (int q = 0; q < 3 * NR; ++q) dst[q] = n == 0 ? 0.f : fmaf(w, acc[q], dst[q]);
+    for (int p = 0; p < 3; ++p) dst[p * (size_t)nf] = n == 0 ? make_float2(0.f, 0.f) : pfma(w, acc[p], old[p]);
 }
 
 // Dense coarsest matrix (row per thread, no atomics); node 0's rows and
@@ -320,8 +415,16 @@ __global__ void pdense_kernel(PGrid g, const double *__restrict__ CX, double *__
             }
 }
 
+// Index of dof c = 3 n + d, load case r, in the pair planes of a grid of N nodes.
+__device__ __forceinline__ long long pidx(int c, int r, int N)
+{
+    const int n = c / 3, d = c - 3 * n;
+    return 2 * ((long long)(3 * d + (r >> 1)) * N + n) + (r & 1);
+}
+
 // y = M x on the coarsest grid for the six cases (warp per row; lower: the
-// lower triangle of M, else the upper).
+// lower triangle of M, else the upper).  The FP32 side is in pair planes, the
+// FP64 intermediate as [dof][case].
 template <typename Tin, typename Tout>
 __global__ void pgemv6_kernel(int n, const double *__restrict__ M, const Tin *__restrict__ x, Tout *__restrict__ y,
                               int lower, const int *done)
@@ -337,7 +440,8 @@ __global__ void pgemv6_kernel(int n, const double *__restrict__ M, const Tin *__
     for (int c = lo + lane; c < hi; c += 32) {
         const double m = mr[c];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) s[r] = fma(m, (double)x[(long long)c * NR + r], s[r]);
+        for (int r = 0; r < NR; ++r)
+            s[r] = fma(m, (double)x[sizeof(Tin) == 4 ? pidx(c, r, n / 3) : (long long)c * NR + r], s[r]);
     }
 #pragma unroll
     for (int r = 0; r < NR; ++r)
@@ -347,7 +451,7 @@ __global__ void pgemv6_kernel(int n, const double *__restrict__ M, const Tin *__
 #pragma unroll
         for (int r = 1; r < NR; ++r)
             if (lane == r) v = s[r];
-        y[(long long)row * NR + lane] = (Tout)v;
+        y[sizeof(Tout) == 4 ? pidx(row, lane, n / 3) : (long long)row * NR + lane] = (Tout)v;
     }
 }
 
@@ -368,8 +472,11 @@ __global__ void pload_kernel(PGrid g, const double *__restrict__ CX, double *__r
                 for (int d = 0; d < 3; ++d)
                     for (int r = 0; r < NR; ++r) f[d][r] -= c * cPG[(3 * ca + d) * NR + r];
             }
+    const size_t N = (size_t)g.nnod();
     for (int d = 0; d < 3; ++d)
-        for (int r = 0; r < NR; ++r) F[(3 * n + d) * NR + r] = n == 0 ? 0.0 : f[d][r];
+        for (int p = 0; p < 3; ++p)
+            reinterpret_cast<double2 *>(F)[(3 * d + p) * N + n] =
+                n == 0 ? make_double2(0.0, 0.0) : make_double2(f[d][2 * p], f[d][2 * p + 1]);
 }
 
 // ---- PCG over the six cases (FP64) ----------------------------------------
@@ -379,9 +486,10 @@ struct HScal {
     int done_r[NR], nit[NR];
     double tol;
     int iter, maxit, done, status;
+    int pending;   // the last iteration's U += alpha P is still to be applied
 };
 
-// Per-block partial sums of K values per dof group -> partial[block][K].
+// Per-CTA sums of K values -> partial[CTA][K].
 template <int K>
 __device__ __forceinline__ void block_partials(double (&v)[K], double *partial)
 {
@@ -400,29 +508,40 @@ __device__ __forceinline__ void block_partials(double (&v)[K], double *partial)
     }
 }
 
+// The vector kernels: a thread takes dofs c = 3 n + d a grid stride apart, all
+// six cases of each (the order of the sums), so a warp reads 11 consecutive
+// nodes of three planes per pair.  All are bound by HBM: at 128^3 pupdate 203
+// us for 1.06 GB, pdot2 98 us for 0.60 GB, ppupdate 220 us for 1.51 GB (with
+// the cases adjacent, 48 bytes between a warp's lanes, and U updated here:
+// 589, 95 and 269 us).
+
 // U = 0, R = F, float(R), |F_r|^2 partials.
-__global__ void __launch_bounds__(256) pinit_kernel(long long nd, const double *__restrict__ F, double *__restrict__ U,
-                                                    double *__restrict__ R, float *__restrict__ Rf,
+__global__ void __launch_bounds__(256) pinit_kernel(size_t N, const double2 *__restrict__ F, double2 *__restrict__ U,
+                                                    double2 *__restrict__ R, float2 *__restrict__ Rf,
                                                     double *__restrict__ partial)
 {
     double s[NR] = {};
-    for (long long d = (long long)blockIdx.x * blockDim.x + threadIdx.x; d < nd; d += (long long)gridDim.x * blockDim.x)
+    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < 3 * N; c += (size_t)gridDim.x * blockDim.x) {
+        const size_t n = c / 3, d = c - 3 * n;
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const double f = F[d * NR + r];
-            U[d * NR + r] = 0.0;
-            R[d * NR + r] = f;
-            Rf[d * NR + r] = (float)f;
-            s[r] = fma(f, f, s[r]);
+        for (int p = 0; p < 3; ++p) {
+            const size_t q = (3 * d + p) * N + n;
+            const double2 f = F[q];
+            U[q] = make_double2(0.0, 0.0);
+            R[q] = f;
+            Rf[q] = make_float2((float)f.x, (float)f.y);
+            s[2 * p] = fma(f.x, f.x, s[2 * p]);
+            s[2 * p + 1] = fma(f.y, f.y, s[2 * p + 1]);
         }
+    }
     block_partials<NR>(s, partial);
 }
 
-// U += alpha P, R -= alpha Q, float(R), |R_r|^2 partials.
-__global__ void __launch_bounds__(256) pupdate_kernel(long long nd, double *__restrict__ U, double *__restrict__ R,
-                                                      const double *__restrict__ P, const double *__restrict__ Q,
-                                                      float *__restrict__ Rf, const HScal *__restrict__ sc,
-                                                      double *__restrict__ partial)
+// R -= alpha Q, float(R), |R_r|^2 partials.  U += alpha P waits for
+// ppupdate_kernel, which reads P anyway.
+__global__ void __launch_bounds__(256) pupdate_kernel(size_t N, double2 *__restrict__ R,
+                                                      const double2 *__restrict__ Q, float2 *__restrict__ Rf,
+                                                      const HScal *__restrict__ sc, double *__restrict__ partial)
 {
     if (sc->done) return;
     double al[NR], s[NR];
@@ -431,82 +550,150 @@ __global__ void __launch_bounds__(256) pupdate_kernel(long long nd, double *__re
         al[r] = sc->alpha[r];
         s[r] = 0.0;
     }
-    for (long long d = (long long)blockIdx.x * blockDim.x + threadIdx.x; d < nd; d += (long long)gridDim.x * blockDim.x)
+    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < 3 * N; c += (size_t)gridDim.x * blockDim.x) {
+        const size_t n = c / 3, d = c - 3 * n;
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const long long q = d * NR + r;
-            U[q] = fma(al[r], P[q], U[q]);
-            const double rv = fma(-al[r], Q[q], R[q]);
-            R[q] = rv;
-            Rf[q] = (float)rv;
-            s[r] = fma(rv, rv, s[r]);
+        for (int p = 0; p < 3; ++p) {
+            const size_t q = (3 * d + p) * N + n;
+            const double2 r = R[q], a = Q[q];
+            const double2 v = make_double2(fma(-al[2 * p], a.x, r.x), fma(-al[2 * p + 1], a.y, r.y));
+            R[q] = v;
+            Rf[q] = make_float2((float)v.x, (float)v.y);
+            s[2 * p] = fma(v.x, v.x, s[2 * p]);
+            s[2 * p + 1] = fma(v.y, v.y, s[2 * p + 1]);
         }
+    }
     block_partials<NR>(s, partial);
 }
 
 // r'z and r'z_old per case.
-__global__ void __launch_bounds__(256) pdot2_kernel(long long nd, const double *__restrict__ R,
-                                                    const float *__restrict__ Z, const float *__restrict__ Zo,
+__global__ void __launch_bounds__(256) pdot2_kernel(size_t N, const double2 *__restrict__ R,
+                                                    const float2 *__restrict__ Z, const float2 *__restrict__ Zo,
                                                     double *__restrict__ partial, const HScal *__restrict__ sc)
 {
     if (sc && sc->done) return;
     double s[2 * NR] = {};
-    for (long long d = (long long)blockIdx.x * blockDim.x + threadIdx.x; d < nd; d += (long long)gridDim.x * blockDim.x)
+    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < 3 * N; c += (size_t)gridDim.x * blockDim.x) {
+        const size_t n = c / 3, d = c - 3 * n;
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const long long q = d * NR + r;
-            const double rv = R[q];
-            s[r] = fma(rv, (double)Z[q], s[r]);
-            if (Zo) s[NR + r] = fma(rv, (double)Zo[q], s[NR + r]);
+        for (int p = 0; p < 3; ++p) {
+            const size_t q = (3 * d + p) * N + n;
+            const double2 r = R[q];
+            const float2 z = Z[q];
+            s[2 * p] = fma(r.x, (double)z.x, s[2 * p]);
+            s[2 * p + 1] = fma(r.y, (double)z.y, s[2 * p + 1]);
+            if (Zo) {
+                const float2 o = Zo[q];
+                s[NR + 2 * p] = fma(r.x, (double)o.x, s[NR + 2 * p]);
+                s[NR + 2 * p + 1] = fma(r.y, (double)o.y, s[NR + 2 * p + 1]);
+            }
         }
+    }
     block_partials<2 * NR>(s, partial);
 }
 
-// P = z + beta P (beta = 0: P = z), z_old = z.
-__global__ void __launch_bounds__(256) ppupdate_kernel(long long nd, const float *__restrict__ Z, double *__restrict__ P,
-                                                       float *__restrict__ Zo, const HScal *__restrict__ sc, int first)
+// U += alpha P, P = z + beta P, z_old = z (first: P = z and z_old = z alone).
+// Once done, only a pending U update.  blockIdx.y = load-case pair.
+__global__ void __launch_bounds__(256) ppupdate_kernel(size_t N, const float2 *__restrict__ Z, double2 *__restrict__ P,
+                                                       double2 *__restrict__ U, float2 *__restrict__ Zo,
+                                                       const HScal *__restrict__ sc, int first)
 {
-    if (sc->done && !first) return;
-    double be[NR];
+    const bool done = sc->done != 0, up = !first && sc->pending != 0;
+    if (!first && !up) return;
+    const int p = blockIdx.y;
+    const double bx = first ? 0.0 : sc->beta[2 * p], by = first ? 0.0 : sc->beta[2 * p + 1];
+    const double ax = up ? sc->alpha[2 * p] : 0.0, ay = up ? sc->alpha[2 * p + 1] : 0.0;
+    for (size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x; n < N; n += (size_t)gridDim.x * blockDim.x)
 #pragma unroll
-    for (int r = 0; r < NR; ++r) be[r] = first ? 0.0 : sc->beta[r];
-    for (long long d = (long long)blockIdx.x * blockDim.x + threadIdx.x; d < nd; d += (long long)gridDim.x * blockDim.x)
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const long long q = d * NR + r;
-            const float z = Z[q];
-            P[q] = first ? (double)z : fma(be[r], P[q], (double)z);
+        for (int d = 0; d < 3; ++d) {
+            const size_t q = (3 * d + p) * N + n;
+            const double2 pv = P[q];
+            if (up) {
+                const double2 u = U[q];
+                U[q] = make_double2(fma(ax, pv.x, u.x), fma(ay, pv.y, u.y));
+            }
+            if (done && !first) continue;
+            const float2 z = Z[q];
+            P[q] = first ? make_double2((double)z.x, (double)z.y)
+                         : make_double2(fma(bx, pv.x, (double)z.x), fma(by, pv.y, (double)z.y));
             Zo[q] = z;
         }
 }
 
+// The fluctuations from the pair planes to the caller's [3 node + d][case].
+__global__ void __launch_bounds__(256) pchi_kernel(size_t N, const double2 *__restrict__ U, double *__restrict__ chi)
+{
+    __shared__ double t[256 * 19];   // odd row length: no bank conflicts
+    const size_t n0 = (size_t)blockIdx.x * 256, n = n0 + threadIdx.x;
+    if (n < N)
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {   // plane 3 d + p -> row entry 6 d + 2 p
+            const double2 v = U[q * N + n];
+            t[threadIdx.x * 19 + 2 * q] = v.x;
+            t[threadIdx.x * 19 + 2 * q + 1] = v.y;
+        }
+    __syncthreads();
+    const int cnt = (int)min((size_t)256, N - n0) * 18;
+    for (int q = threadIdx.x; q < cnt; q += 256) chi[n0 * 18 + q] = t[(q / 18) * 19 + q % 18];
+}
+
 enum PFinish { PF_INIT = 0, PF_RHO0 = 1, PF_ALPHA = 2, PF_END = 3 };
 
-// Sums the per-block partials in fixed order and moves the scalars (one
-// block).  INIT: res0; RHO0: rho; ALPHA: alpha = rho / p'q (0 for finished
-// cases); END (partials: r'z, r'z_old; rr from the update): beta, relres,
-// convergence per case, iteration count.
-__global__ void __launch_bounds__(256) pfinish_kernel(int nb, const double *__restrict__ partial,
-                                                      const double *__restrict__ partial_rr, HScal *sc, int which)
+constexpr int kFinThreads = 1024;
+constexpr int kFinChunk = 3072;   // partials staged in shared memory at a time (24 KB), a multiple of 2 NR
+
+// tot[q] = sum over CTAs b, in order, of partial[b][K].  The sum of a row is
+// one serial chain of additions (its order is part of the result), so the
+// partials are staged in shared memory by the whole CTA and thread q runs the
+// chain from there, eight loads ahead: 60 us over the apply's 8192 partials
+// (bound by the chain of additions), where one thread per row reading global
+// memory took 400 us.
+template <int K>
+__device__ __forceinline__ void row_sums(int nb, const double *__restrict__ partial, double *st, double *tot)
 {
-    if (which >= PF_ALPHA && sc->done) return;
-    // pdot2 writes 2 NR partials per block (INIT: pinit, ALPHA: the apply, NR each)
-    const int K = (which == PF_END || which == PF_RHO0) ? 2 * NR : NR;
-    __shared__ double tot[2 * NR], tot_rr[NR];
-    // thread q sums column q (fixed order: deterministic)
-    if (threadIdx.x < K) {
-        double s = 0.0;
-        for (int b = 0; b < nb; ++b) s += partial[(long long)b * K + threadIdx.x];
-        tot[threadIdx.x] = s;
+    double s = 0.0;
+    const long long n = (long long)nb * K;
+    for (long long c0 = 0; c0 < n; c0 += kFinChunk) {
+        const int m = (int)min((long long)kFinChunk, n - c0);
+        __syncthreads();
+        for (int q = threadIdx.x; q < m; q += kFinThreads) st[q] = partial[c0 + q];
+        __syncthreads();
+        if (threadIdx.x < K) {
+            const int rows = m / K;
+            int b = 0;
+            for (; b + 8 <= rows; b += 8) {
+                double v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = st[(b + e) * K + threadIdx.x];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) s += v[e];
+            }
+            for (; b < rows; ++b) s += st[b * K + threadIdx.x];
+        }
     }
-    if (which == PF_END && threadIdx.x >= 32 && threadIdx.x < 32 + NR) {
-        double s = 0.0;
-        for (int b = 0; b < nb; ++b) s += partial_rr[(long long)b * NR + threadIdx.x - 32];
-        tot_rr[threadIdx.x - 32] = s;
+    if (threadIdx.x < K) tot[threadIdx.x] = s;
+}
+
+// Sums the CTA partials and moves the scalars (one CTA).  INIT: res0; RHO0:
+// rho; ALPHA: alpha = rho / p'q (0 for finished cases); END (partials: r'z,
+// r'z_old; rr from the update): beta, relres, convergence per case,
+// iteration count.
+template <int WHICH>
+__global__ void __launch_bounds__(kFinThreads) pfinish_kernel(int nb, const double *__restrict__ partial,
+                                                              const double *__restrict__ partial_rr, HScal *sc)
+{
+    if (WHICH >= PF_ALPHA && sc->done) {
+        if (WHICH == PF_ALPHA && threadIdx.x == 0) sc->pending = 0;
+        return;
     }
+    // pdot2 writes 2 NR rows (INIT: pinit, ALPHA: the apply, NR each)
+    constexpr int K = (WHICH == PF_END || WHICH == PF_RHO0) ? 2 * NR : NR;
+    __shared__ double st[kFinChunk], tot[2 * NR], tot_rr[NR];
+    row_sums<K>(nb, partial, st, tot);
+    if (WHICH == PF_END) row_sums<NR>(nb, partial_rr, st, tot_rr);
     __syncthreads();
     if (threadIdx.x != 0) return;
-    if (which == PF_INIT) {
+    if (WHICH == PF_INIT) {
         for (int r = 0; r < NR; ++r) {
             sc->res0[r] = sqrt(tot[r]);
             sc->relres[r] = 1.0;
@@ -525,9 +712,10 @@ __global__ void __launch_bounds__(256) pfinish_kernel(int nb, const double *__re
         for (int r = 0; r < NR; ++r) all &= sc->done_r[r];
         sc->done = all || sc->status || sc->maxit <= 0;
         sc->iter = 0;
-    } else if (which == PF_RHO0) {
+    } else if (WHICH == PF_RHO0) {
         for (int r = 0; r < NR; ++r) sc->rho[r] = tot[r];
-    } else if (which == PF_ALPHA) {
+    } else if (WHICH == PF_ALPHA) {
+        sc->pending = 0;
         for (int r = 0; r < NR; ++r) {
             const double a = sc->rho[r] / tot[r];
             if (sc->done_r[r]) {
@@ -563,6 +751,7 @@ __global__ void __launch_bounds__(256) pfinish_kernel(int nb, const double *__re
             }
             all &= sc->done_r[r];
         }
+        sc->pending = 1;
         sc->iter = it + 1;
         if (all || sc->status || it + 1 >= sc->maxit) sc->done = 1;
     }
@@ -573,6 +762,7 @@ __global__ void __launch_bounds__(256) pfinish_kernel(int nb, const double *__re
 __global__ void __launch_bounds__(256) pceff_kernel(PGrid g, const double *__restrict__ CX,
                                                     const double *__restrict__ U, double *__restrict__ partial)
 {
+    const long long N = g.nnod();
     double c[21] = {};
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < g.nnod();
          e += (long long)gridDim.x * blockDim.x) {
@@ -592,7 +782,7 @@ __global__ void __launch_bounds__(256) pceff_kernel(PGrid g, const double *__res
             for (int a = 0; a < 8; ++a)
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
-                    w[3 * a + d] = cPU0[r * 24 + 3 * a + d] + U[(3 * nodes[a] + d) * NR + r];
+                    w[3 * a + d] = cPU0[r * 24 + 3 * a + d] + U[2 * ((3 * d + (r >> 1)) * N + nodes[a]) + (r & 1)];
 #pragma unroll
             for (int m = 0; m < 24; ++m) {
                 double s = 0.0;
@@ -607,7 +797,8 @@ __global__ void __launch_bounds__(256) pceff_kernel(PGrid g, const double *__res
                 for (int a = 0; a < 8; ++a)
 #pragma unroll
                     for (int d = 0; d < 3; ++d)
-                        dot = fma(cPU0[s2 * 24 + 3 * a + d] + U[(3 * nodes[a] + d) * NR + s2], kw[3 * a + d], dot);
+                        dot = fma(cPU0[s2 * 24 + 3 * a + d] + U[2 * ((3 * d + (s2 >> 1)) * N + nodes[a]) + (s2 & 1)],
+                                  kw[3 * a + d], dot);
                 // q indexes the upper triangle in row order
 #pragma unroll
                 for (int z = 0; z < 21; ++z)
@@ -631,10 +822,10 @@ struct Homog {
     cudaStream_t own_stream = nullptr;
     std::vector<void *> owned;
     size_t bytes = 0;
-    // FP64 outer vectors [ndof][6]
+    // FP64 outer vectors (pair planes)
     double *F = nullptr, *U = nullptr, *R = nullptr, *P = nullptr, *Q = nullptr;
     float *Rf = nullptr, *Zold = nullptr;
-    // per level: element scales (FP64 natural, FP32), 1/diag (FP64, FP32), FP32 buffers [ndof_l][6]
+    // per level: element scales (FP64 natural, FP32), 1/diag (FP64, FP32), FP32 buffers (pair planes)
     double *CXd[kMaxLevels]{}, *rdd[kMaxLevels]{};
     float *CXf[kMaxLevels]{}, *rdf[kMaxLevels]{};
     float *u0[kMaxLevels]{}, *u1[kMaxLevels]{}, *fl[kMaxLevels]{}, *rl[kMaxLevels]{};
@@ -643,7 +834,7 @@ struct Homog {
     int *info = nullptr;
     HScal *sc = nullptr, *h_sc = nullptr;
     double *part = nullptr, *part_rr = nullptr, *part_c = nullptr;
-    int nb_red = 0;
+    int nb_red = 0, nb_apply = 0;   // CTAs of the vector kernels and of the operator apply
     cudaGraphExec_t graph = nullptr;
     cudaStream_t graph_stream = nullptr;
 
@@ -727,7 +918,7 @@ struct Homog {
         if (!s) s = alloc(&info, 4);
         if (!s) s = alloc(&sc, 1);
         nb_red = (int)std::min<long long>(kHBlocks, std::max(1LL, (g[0].ndof() + 255) / 256));
-        const int nb_apply = (int)nblk(g[0].nnod());
+        nb_apply = (int)nblk(g[0].nnod());
         if (!s) s = alloc(&part, (long long)std::max(nb_apply, nb_red) * 2 * NR);
         if (!s) s = alloc(&part_rr, (long long)nb_red * NR);
         if (!s) s = alloc(&part_c, (long long)nb_red * 21);
@@ -796,11 +987,35 @@ struct Homog {
         return GPUTO_OK;
     }
 
+    // Tiles of a sweep: 32 (y) x 8 (z) node columns per CTA, or the whole
+    // (shorter) y row by 256 / ny, and nx planes per thread.
+    struct SweepGrid {
+        unsigned grid;
+        int ty, ntj, nt;
+    };
+    static SweepGrid sweep_grid(const PGrid &q, int nxt)
+    {
+        const int ty = std::min(q.ny, 32), tz = 256 / ty;
+        const int ntj = (q.ny + ty - 1) / ty, ntk = (q.nz + tz - 1) / tz;
+        return SweepGrid{(unsigned)(ntj * ntk) * (unsigned)((q.nx + nxt - 1) / nxt), ty, ntj, ntj * ntk};
+    }
+
+    // Two nodes per thread halve the CTAs and the plane reads: from about one
+    // wave of CTAs on (2 x 148 of 512 nodes).  Below that the sweeps are bound
+    // by latency (7-8 us) and more CTAs are worth more.
     template <int MODE>
     void sweep(int l, const float *u, const float *f, float *out, const int *done, cudaStream_t st)
     {
-        psweep_kernel<float, MODE><<<nblk(g[l].nnod()), 256, 0, st>>>(
-            g[l], CXf[l], u, f, rdf[l], out, (float)opt.omega, (float)opt.prerelax, nullptr, done);
+        const float om = (float)opt.omega, pr = (float)opt.prerelax;
+        if (g[l].nnod() >= 2LL * 148 * 512) {
+            const SweepGrid s = sweep_grid(g[l], 2);
+            psweep_kernel<float, MODE, 2>
+                <<<s.grid, 256, 0, st>>>(g[l], s.ty, s.ntj, s.nt, CXf[l], u, f, rdf[l], out, om, pr, nullptr, done);
+        } else {
+            const SweepGrid s = sweep_grid(g[l], 1);
+            psweep_kernel<float, MODE, 1>
+                <<<s.grid, 256, 0, st>>>(g[l], s.ty, s.ntj, s.nt, CXf[l], u, f, rdf[l], out, om, pr, nullptr, done);
+        }
         count_launches(1);
     }
 
@@ -815,7 +1030,7 @@ struct Homog {
         for (int l = 0; l < nl; ++l) {
             const float *f = l == 0 ? r0 : fl[l];
             if (l > 0) {
-                prestrict_kernel<<<nblk(g[l].nnod()), 256, 0, st>>>(g[l], rl[l - 1], fl[l], done);
+                prestrict_kernel<<<dim3(nblk(g[l].nnod()), 3), 256, 0, st>>>(g[l], rl[l - 1], fl[l], done);
                 count_launches(1);
             }
             if (l < nl - 1) {
@@ -834,7 +1049,7 @@ struct Homog {
         for (int l = nl - 2; l >= 0; --l) {
             const float *f = l == 0 ? r0 : fl[l];
             int cur = (ns - 1) & 1;
-            pprolong_kernel<<<nblk(g[l].nnod()), 256, 0, st>>>(g[l], buf(l + 1, 1), buf(l, cur), done);
+            pprolong_kernel<<<dim3(nblk(g[l].nnod()), 3), 256, 0, st>>>(g[l], buf(l + 1, 1), buf(l, cur), done);
             count_launches(1);
             // starting from buffer (ns - 1) & 1, ns sweeps end in buffer 1
             for (int s = 0; s < ns; ++s) {
@@ -847,16 +1062,17 @@ struct Homog {
     // One flexible PCG iteration of all six cases.
     void iteration(cudaStream_t st)
     {
-        const long long nd = g[0].ndof();
+        const size_t N = (size_t)g[0].nnod();
         const int *done = &sc->done;
-        const int nb = (int)nblk(g[0].nnod());
-        psweep_kernel<double, P_APPLY><<<nb, 256, 0, st>>>(g[0], CXd[0], P, nullptr, nullptr, Q, 1.0, 0.0, part, done);
-        pfinish_kernel<<<1, 256, 0, st>>>(nb, part, nullptr, sc, PF_ALPHA);
-        pupdate_kernel<<<nb_red, 256, 0, st>>>(nd, U, R, P, Q, Rf, sc, part_rr);
+        const dim3 gp((unsigned)(nb_red + 2) / 3, 3);
+        psweep_kernel<double, P_APPLY, 1><<<nb_apply, 256, 0, st>>>(g[0], 0, 0, 0, CXd[0], P, nullptr, nullptr, Q, 1.0,
+                                                                    0.0, part, done);
+        pfinish_kernel<PF_ALPHA><<<1, kFinThreads, 0, st>>>(nb_apply, part, nullptr, sc);
+        pupdate_kernel<<<nb_red, 256, 0, st>>>(N, (double2 *)R, (const double2 *)Q, (float2 *)Rf, sc, part_rr);
         vcycle(Rf, u1[0], done, st);
-        pdot2_kernel<<<nb_red, 256, 0, st>>>(nd, R, u1[0], Zold, part, sc);
-        pfinish_kernel<<<1, 256, 0, st>>>(nb_red, part, part_rr, sc, PF_END);
-        ppupdate_kernel<<<nb_red, 256, 0, st>>>(nd, u1[0], P, Zold, sc, 0);
+        pdot2_kernel<<<nb_red, 256, 0, st>>>(N, (const double2 *)R, (const float2 *)u1[0], (const float2 *)Zold, part, sc);
+        pfinish_kernel<PF_END><<<1, kFinThreads, 0, st>>>(nb_red, part, part_rr, sc);
+        ppupdate_kernel<<<gp, 256, 0, st>>>(N, (const float2 *)u1[0], (double2 *)P, (double2 *)U, (float2 *)Zold, sc, 0);
         count_launches(7);
     }
 
@@ -884,17 +1100,18 @@ struct Homog {
             set_error("maxit must be >= 0 and tol >= 0");
             return GPUTO_ERR_ARG;
         }
-        const long long nd = g[0].ndof();
+        const size_t N = (size_t)g[0].nnod();
+        const dim3 gp((unsigned)(nb_red + 2) / 3, 3);
         HScal z{};
         z.tol = tol;
         z.maxit = maxit;
         GPUTO_CUDA(cudaMemcpyAsync(sc, &z, sizeof(HScal), cudaMemcpyHostToDevice, st));
-        pinit_kernel<<<nb_red, 256, 0, st>>>(nd, F, U, R, Rf, part);
-        pfinish_kernel<<<1, 256, 0, st>>>(nb_red, part, nullptr, sc, PF_INIT);
+        pinit_kernel<<<nb_red, 256, 0, st>>>(N, (const double2 *)F, (double2 *)U, (double2 *)R, (float2 *)Rf, part);
+        pfinish_kernel<PF_INIT><<<1, kFinThreads, 0, st>>>(nb_red, part, nullptr, sc);
         vcycle(Rf, u1[0], &sc->done, st);
-        pdot2_kernel<<<nb_red, 256, 0, st>>>(nd, R, u1[0], nullptr, part, nullptr);
-        pfinish_kernel<<<1, 256, 0, st>>>(nb_red, part, nullptr, sc, PF_RHO0);
-        ppupdate_kernel<<<nb_red, 256, 0, st>>>(nd, u1[0], P, Zold, sc, 1);
+        pdot2_kernel<<<nb_red, 256, 0, st>>>(N, (const double2 *)R, (const float2 *)u1[0], nullptr, part, nullptr);
+        pfinish_kernel<PF_RHO0><<<1, kFinThreads, 0, st>>>(nb_red, part, nullptr, sc);
+        ppupdate_kernel<<<gp, 256, 0, st>>>(N, (const float2 *)u1[0], (double2 *)P, (double2 *)U, (float2 *)Zold, sc, 1);
         count_launches(5);
         GPUTO_CUDA(cudaStreamSynchronize(st));   // the host struct z is on the stack
         int it = 0;
@@ -987,8 +1204,11 @@ int gputo_homog_solve_dev(gputo_homog *hh, const double *Ke0, const double *CX, 
     if (!s) s = h.setup(CX, st);
     if (!s) s = h.solve(tol, maxit, Ceff, relres, nit, st);
     if (!s && chi) {
-        GPUTO_CUDA(cudaMemcpyAsync(chi, h.U, sizeof(double) * h.g[0].ndof() * gputo::NR, cudaMemcpyDeviceToDevice, st));
+        const size_t N = (size_t)h.g[0].nnod();
+        gputo::pchi_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(N, (const double2 *)h.U, chi);
+        gputo::count_launches(1);
         GPUTO_CUDA(cudaStreamSynchronize(st));
+        GPUTO_CUDA(cudaGetLastError());
     }
     return s;
 }

@@ -76,3 +76,28 @@ def test_random_field_cell_at_32_cubed_is_within_the_bounds(oracle, gputo, torch
     assert np.linalg.eigvalsh(C - R).min() >= -1e-9 * np.abs(C).max()
     C2, rr2, nit2 = h.solve(Ke, _dev(torch, CX), tol=1e-6, maxit=2000)
     assert np.array_equal(C, C2) and np.array_equal(nit, nit2)
+
+
+@pytest.mark.parametrize("shape,nl", [((64, 48, 56), 4), ((24, 16, 40), 3), ((12, 36, 20), 3)])
+def test_rotated_cell_gives_the_rotated_tensor(gputo, torch, shape, nl):
+    """The axes of a random cell permuted cyclically permute its tensor: every
+    direction of the sweeps, transfers and sums has to index alike, on rows
+    shorter and longer than a tile of 32 columns, on sizes that leave part of a
+    tile empty, and on a grid large enough (from 151,552 nodes) for two nodes
+    per thread.  Solves to 1e-9 leave a second-order error in C (below 1e-12 at
+    this contrast of 1e3): 1e-8 as for the oracle."""
+    nx, ny, nz = shape
+    x = gputo.random_field_density(nx, ny, nz, seed=8, corr_len=4.0, lo=0.1, hi=1.0).reshape(nx, nz, ny)
+    Ke = gputo.hex8_stiffness(0.3)
+
+    def tensor(a):   # a in (x, z, y) order
+        h = gputo.Homog(a.shape[0], a.shape[2], a.shape[1], nl)
+        C, rr, nit = h.solve(Ke, _dev(torch, a.reshape(-1) ** 3), tol=1e-9, maxit=500)
+        assert (rr < 1e-9).all()
+        return C
+
+    C = tensor(x)
+    # x' = y, y' = z, z' = x: (x', z', y') = (y, x, z)
+    Cr = tensor(np.ascontiguousarray(x.transpose(2, 0, 1)))
+    p = [1, 2, 0, 4, 5, 3]
+    assert np.abs(Cr - C[np.ix_(p, p)]).max() <= 1e-8 * np.abs(C).max()
