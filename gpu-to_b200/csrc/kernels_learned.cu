@@ -8,17 +8,32 @@
 // FP32.  Flat parameter layout per layer: w[co][ci][tap] then b[co], tap =
 // 9 (dx+1) + 3 (dz+1) + (dy+1).
 //
-// Convolutions are direct: one thread per node computes a chunk of output
-// channels, the chunk's weights sit in shared memory and every thread of a
-// warp reads the same weight at the same time (broadcast), the input reads
-// are coalesced along Y.  Weight gradients are reduced per (co, ci) pair by
-// one CTA in a fixed order, so training is deterministic.
+// The 16 -> 32 and 32 -> 64 convolutions and their data gradients are implicit
+// GEMMs on the 5th-generation tensor cores (conv_tc_kernel); the first layer,
+// the 1x1x1 head and the weight gradients run on the CUDA cores.
+//
+// Activations and gradients between the layers are stored as "split rows":
+//  * a grid node is row r = guard + ((s (X + 1) + x) (Z + 1) + z) (Y + 1) + y;
+//    one zero row after each y line, one zero line after each z plane, one
+//    zero plane after each sample and `guard` zero rows in front and behind
+//    stand in for the zero padding, so every tap of every node is a fixed row
+//    offset and needs no test;
+//  * each FP32 value is the exact sum of three BF16 parts (hi, mid, lo: the 24
+//    significand bits, split by truncation), kept in planes
+//    [part][channel / 8][row][8]: 16 bytes per row, the K-major operand rows
+//    of the tensor cores, which a bulk copy brings in as they are and whose
+//    shift by a row is a shift of the operand's address by 16 bytes.
+// Products of the parts with the BF16 weights are exact in FP32, so three
+// BF16 MMAs give the FP32 convolution up to the order of its sums.  Weight
+// gradients are reduced in a fixed order, so training is deterministic.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "gputo_internal.h"
+#include "tma.h"
 
 namespace gputo {
 
@@ -29,208 +44,755 @@ __host__ __device__ constexpr int net_k(int l) { return l == 3 ? 1 : 3; }
 
 __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-constexpr int kNetThreads = 128;
+constexpr int kRows = 128;                       // rows of one tile (TMEM lanes)
+constexpr uint32_t kNetWaitNs = 2000000000u;     // bounded waits give up after 2 s
 
-// Offset of tap t of a 3x3x3 stencil, and whether it stays inside the grid.
-__device__ __forceinline__ bool tap_in(int t, int xi, int zi, int yi, const NetDims &d, long long &off)
+// Eight FP32 values -> their three BF16 parts, eight per 16-byte row entry
+// (the same truncating split as kernels_tc.cu's).
+__device__ __forceinline__ void split8(const float (&v)[8], uint4 (&o)[3])
 {
-    const int dx = t / 9 - 1, dz = (t / 3) % 3 - 1, dy = t % 3 - 1;
-    off = ((long long)dx * d.Z + dz) * d.Y + dy;
-    return (unsigned)(xi + dx) < (unsigned)d.X && (unsigned)(zi + dz) < (unsigned)d.Z && (unsigned)(yi + dy) < (unsigned)d.Y;
-}
-
-template <int CIN, int COT, int K, bool RELU>
-__global__ void __launch_bounds__(kNetThreads)
-conv_fwd_kernel(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
-                float *__restrict__ y, NetDims d, int cout)
-{
-    constexpr int K3 = K * K * K;
-    extern __shared__ float ws[];   // [CIN][K3][COT], BF16-rounded
-    const int co0 = blockIdx.y * COT;
-    for (int idx = threadIdx.x; idx < CIN * K3 * COT; idx += blockDim.x) {
-        const int c = idx % COT, rest = idx / COT, t = rest % K3, ci = rest / K3;
-        const int co = co0 + c;
-        ws[idx] = co < cout ? bf16r(w[((long long)co * CIN + ci) * K3 + t]) : 0.f;
-    }
-    __syncthreads();
-    const long long N = d.n();
-    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    const int yi = (int)(n % d.Y);
-    const long long r = n / d.Y;
-    const int zi = (int)(r % d.Z), xi = (int)(r / d.Z);
-    float acc[COT];
+    uint32_t w[3][4];
 #pragma unroll
-    for (int c = 0; c < COT; ++c) acc[c] = co0 + c < cout ? b[co0 + c] : 0.f;
-    for (int ci = 0; ci < CIN; ++ci) {
-        const float *xc = x + (long long)ci * N;
+    for (int q = 0; q < 4; ++q) {
+        uint32_t a[3], b[3];
 #pragma unroll
-        for (int t = 0; t < K3; ++t) {
-            long long off = 0;
-            const bool in = K == 1 ? true : tap_in(t, xi, zi, yi, d, off);
-            const float v = in ? xc[n + off] : 0.f;
-            const float *wr = ws + (ci * K3 + t) * COT;
-#pragma unroll
-            for (int c = 0; c < COT; ++c) acc[c] = fmaf(wr[c], v, acc[c]);
+        for (int e = 0; e < 2; ++e) {
+            const float x = v[2 * q + e];
+            const uint32_t b0 = __float_as_uint(x);
+            // an infinity stays one: its remainder would be a NaN
+            const float r1 = (b0 & 0x7F800000u) == 0x7F800000u ? 0.f : x - __uint_as_float(b0 & 0xFFFF0000u);
+            const uint32_t b1 = __float_as_uint(r1);
+            const float r2 = r1 - __uint_as_float(b1 & 0xFFFF0000u);
+            uint32_t *t = e ? b : a;
+            t[0] = b0;
+            t[1] = b1;
+            t[2] = __float_as_uint(r2);
         }
+#pragma unroll
+        for (int p = 0; p < 3; ++p) w[p][q] = __byte_perm(a[p], b[p], 0x7632);
     }
 #pragma unroll
-    for (int c = 0; c < COT; ++c)
-        if (co0 + c < cout) y[(long long)(co0 + c) * N + n] = RELU ? fmaxf(acc[c], 0.f) : acc[c];
+    for (int p = 0; p < 3; ++p) o[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
 }
 
-// gx[ci](n) = sum_co sum_tap w[co][ci][tap] g[co](n - offset(tap))
-template <int COUT, int CIT, int K>
-__global__ void __launch_bounds__(kNetThreads)
-conv_bwd_data_kernel(const float *__restrict__ g, const float *__restrict__ w, float *__restrict__ gx, NetDims d,
-                     int cin)
+__device__ __forceinline__ void add_part(float (&v)[8], const uint4 &u)
 {
-    constexpr int K3 = K * K * K;
-    extern __shared__ float ws[];   // [COUT][K3][CIT]
-    const int ci0 = blockIdx.y * CIT;
-    for (int idx = threadIdx.x; idx < COUT * K3 * CIT; idx += blockDim.x) {
-        const int c = idx % CIT, rest = idx / CIT, t = rest % K3, co = rest / K3;
-        const int ci = ci0 + c;
-        ws[idx] = ci < cin ? bf16r(w[((long long)co * cin + ci) * K3 + t]) : 0.f;
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        v[2 * q] += __uint_as_float(w[q] << 16);
+        v[2 * q + 1] += __uint_as_float(w[q] & 0xFFFF0000u);
     }
-    __syncthreads();
-    const long long N = d.n();
-    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    const int yi = (int)(n % d.Y);
-    const long long r = n / d.Y;
-    const int zi = (int)(r % d.Z), xi = (int)(r / d.Z);
-    float acc[CIT];
-#pragma unroll
-    for (int c = 0; c < CIT; ++c) acc[c] = 0.f;
-    for (int co = 0; co < COUT; ++co) {
-        const float *gc = g + (long long)co * N;
-#pragma unroll
-        for (int t = 0; t < K3; ++t) {
-            long long off = 0;
-            // output node n - offset(t): the mirrored tap of n
-            const bool in = K == 1 ? true : tap_in(K3 - 1 - t, xi, zi, yi, d, off);
-            const float v = in ? gc[n + off] : 0.f;
-            const float *wr = ws + (co * K3 + t) * CIT;
-#pragma unroll
-            for (int c = 0; c < CIT; ++c) acc[c] = fmaf(wr[c], v, acc[c]);
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < CIT; ++c)
-        if (ci0 + c < cin) gx[(long long)(ci0 + c) * N + n] = acc[c];
 }
 
-// gw[co][ci][tap] += sum_n g[co](n) x[ci](n + offset(tap)): one CTA per (co, ci)
-template <int K>
+// Geometry of the split rows of S samples.
+struct RowGeo {
+    int X, Z, Y, S;
+    int py, pz;            // row offsets of dz = 1 and dx = 1
+    long long rows;        // S (X + 1) (Z + 1) (Y + 1)
+    long long guard, R;    // zero rows in front; rows of a plane (a whole number of tiles, guards included)
+    int ntiles;
+};
+
+RowGeo row_geo(const NetDims &d, int S)
+{
+    RowGeo q;
+    q.X = d.X, q.Z = d.Z, q.Y = d.Y, q.S = S;
+    q.py = d.Y + 1;
+    q.pz = (d.Z + 1) * (d.Y + 1);
+    q.rows = (long long)S * (d.X + 1) * q.pz;
+    q.guard = ((long long)q.pz + q.py + 1 + 7) / 8 * 8;
+    q.ntiles = (int)((q.rows + kRows - 1) / kRows);
+    q.R = 2 * q.guard + (long long)q.ntiles * kRows;
+    return q;
+}
+
+// Row r (without the guard) -> sample, node; false on padding rows.
+__device__ __forceinline__ bool row_node(const RowGeo &q, long long r, int &s, int &x, int &z, int &y)
+{
+    const long long line = r / q.py;
+    y = (int)(r - line * q.py);
+    const long long plane = line / (q.Z + 1);
+    z = (int)(line - plane * (q.Z + 1));
+    s = (int)(plane / (q.X + 1));
+    x = (int)(plane - (long long)s * (q.X + 1));
+    return s < q.S && x < q.X && z < q.Z && y < q.Y;
+}
+
+// Zeroes the guard rows of up to five sets of planes.
+struct GuardSets {
+    uint4 *p[5];
+    int planes[5];
+};
+
+__global__ void __launch_bounds__(256) zero_guards_kernel(GuardSets g, RowGeo q)
+{
+    uint4 *p = g.p[blockIdx.y];
+    const long long n = 2 * q.guard * g.planes[blockIdx.y];
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const long long pl = i / (2 * q.guard), k = i - pl * 2 * q.guard;
+        p[pl * q.R + (k < q.guard ? k : q.R - 2 * q.guard + k)] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
+// The BF16 weight operands of the four tensor-core convolutions, as the
+// shared-memory image [tap][K / 8][N][8] that a CTA copies whole:
+//   forward l: K = ci, N = co; data gradient l: K = co, N = ci, tap mirrored.
+constexpr int kImg2 = 27 * 16 * 32, kImg3 = 27 * 32 * 64;   // elements
+
 __global__ void __launch_bounds__(256)
-conv_bwd_weight_kernel(const float *__restrict__ g, const float *__restrict__ x, float *__restrict__ gw, NetDims d,
-                       int cin)
+pack_weights_kernel(const float *__restrict__ w2, const float *__restrict__ w3, __nv_bfloat16 *__restrict__ img)
 {
-    constexpr int K3 = K * K * K;
-    const int co = blockIdx.x / cin, ci = blockIdx.x % cin;
-    const long long N = d.n();
-    const float *gc = g + (long long)co * N, *xc = x + (long long)ci * N;
-    float acc[K3];
-#pragma unroll
-    for (int t = 0; t < K3; ++t) acc[t] = 0.f;
-    for (long long n = threadIdx.x; n < N; n += blockDim.x) {
-        const float gv = gc[n];
-        if (gv == 0.f) continue;
-        const int yi = (int)(n % d.Y);
-        const long long r = n / d.Y;
-        const int zi = (int)(r % d.Z), xi = (int)(r / d.Z);
-#pragma unroll
-        for (int t = 0; t < K3; ++t) {
-            long long off = 0;
-            const bool in = K == 1 ? true : tap_in(t, xi, zi, yi, d, off);
-            if (in) acc[t] = fmaf(gv, xc[n + off], acc[t]);
+    int i = blockIdx.x * 256 + threadIdx.x;   // images: forward 2, forward 3, data 3, data 2
+    if (i >= 2 * (kImg2 + kImg3)) return;
+    const int out = i;
+    int l = 2, back = 0;
+    if (i >= kImg2) {
+        i -= kImg2;
+        l = 3;
+        if (i >= kImg3) {
+            i -= kImg3;
+            back = 1;
+            if (i >= kImg3) {
+                i -= kImg3;
+                l = 2;
+            }
         }
     }
-    __shared__ float red[8][K3];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int ci_n = l == 2 ? 16 : 32, co_n = l == 2 ? 32 : 64;
+    const int K = back ? co_n : ci_n, N = back ? ci_n : co_n;
+    const int e = i & 7, n = (i >> 3) % N, rest = (i >> 3) / N, kc = rest % (K / 8), t = rest / (K / 8);
+    const int k = 8 * kc + e;
+    const int co = back ? k : n, ci = back ? n : k, tap = back ? 26 - t : t;
+    const float *w = l == 2 ? w2 : w3;
+    img[out] = __float2bfloat16_rn(w[(co * ci_n + ci) * 27 + tap]);
+}
+
+// Layer 1 (4 -> 16): the 108 taps from the caller's dense input, weights
+// broadcast from shared memory, output pairs on paired FP32 instructions;
+// writes the split rows of its 16 channels (zeros on padding).  4 x 27 x 16
+// FMAs per node are too few channels for the tensor cores.  A thread takes
+// kC1R rows a CTA width apart, which share each weight read: with one row the
+// kernel was bound by those reads (94 us at 129 x 65 x 65, 72 us now).
+constexpr int kC1R = 4;
+
+__global__ void __launch_bounds__(128)
+conv1_kernel(const float *__restrict__ xin, const float *__restrict__ w, const float *__restrict__ b,
+             uint4 *__restrict__ out, RowGeo q)
+{
+    __shared__ __align__(16) float ws[4 * 27 * 16];
+    __shared__ float bs[16];
+    for (int i = threadIdx.x; i < 4 * 27 * 16; i += 128) {
+        const int c = i & 15, t = i >> 4;   // t = ci 27 + tap
+        ws[i] = bf16r(w[c * 108 + t]);
+    }
+    if (threadIdx.x < 16) bs[threadIdx.x] = b[threadIdx.x];
+    __syncthreads();
+    const long long r0 = (long long)blockIdx.x * (128 * kC1R) + threadIdx.x, nr = (long long)q.ntiles * kRows;
+    const int N = q.X * q.Z * q.Y;
+    const float *xs[kC1R];
+    unsigned ok[kC1R];   // bits 0-8: the (dx, dz) line is inside, 9 and 10: y - 1 and y + 1 are; 0 on padding
+    float2 acc[kC1R][8];
 #pragma unroll
-    for (int t = 0; t < K3; ++t) {
-        float v = acc[t];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[wid][t] = v;
+    for (int k = 0; k < kC1R; ++k) {
+        int s, x, z, y;
+        const bool in = row_node(q, r0 + 128 * k, s, x, z, y);
+        xs[k] = in ? xin + (size_t)s * 4 * N + ((size_t)x * q.Z + z) * q.Y + y : xin;
+        ok[k] = 0;
+        if (in) {
+#pragma unroll
+            for (int g = 0; g < 9; ++g)
+                if ((unsigned)(x + g / 3 - 1) < (unsigned)q.X && (unsigned)(z + g % 3 - 1) < (unsigned)q.Z) ok[k] |= 1u << g;
+            ok[k] |= (y > 0 ? 1u << 9 : 0u) | (y < q.Y - 1 ? 1u << 10 : 0u);
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[k][c] = make_float2(bs[2 * c], bs[2 * c + 1]);
     }
-    __syncthreads();
-    if (threadIdx.x < K3) {
-        float s = 0.f;
-        for (int q = 0; q < 8; ++q) s += red[q][threadIdx.x];
-        gw[((long long)co * cin + ci) * K3 + threadIdx.x] += s;
+#pragma unroll 1
+    for (int ci = 0; ci < 4; ++ci)
+#pragma unroll 1
+        for (int dx = 0; dx < 3; ++dx) {
+            float v[kC1R][9];
+#pragma unroll
+            for (int k = 0; k < kC1R; ++k)
+#pragma unroll
+                for (int dz = 0; dz < 3; ++dz) {
+                    const bool in = (ok[k] >> (3 * dx + dz)) & 1u;
+                    const float *p = xs[k] + (size_t)ci * N + (ptrdiff_t)((dx - 1) * q.Z + dz - 1) * q.Y;
+                    v[k][3 * dz] = in && (ok[k] & (1u << 9)) ? p[-1] : 0.f;
+                    v[k][3 * dz + 1] = in ? p[0] : 0.f;
+                    v[k][3 * dz + 2] = in && (ok[k] & (1u << 10)) ? p[1] : 0.f;
+                }
+            const float4 *wr = reinterpret_cast<const float4 *>(ws + (ci * 27 + 9 * dx) * 16);
+#pragma unroll
+            for (int t = 0; t < 9; ++t)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float4 m = wr[4 * t + c];
+#pragma unroll
+                    for (int k = 0; k < kC1R; ++k) {
+                        const float2 vv = make_float2(v[k][t], v[k][t]);
+                        acc[k][2 * c] = __ffma2_rn(make_float2(m.x, m.y), vv, acc[k][2 * c]);
+                        acc[k][2 * c + 1] = __ffma2_rn(make_float2(m.z, m.w), vv, acc[k][2 * c + 1]);
+                    }
+                }
+        }
+#pragma unroll
+    for (int k = 0; k < kC1R; ++k) {
+        const long long r = r0 + 128 * k;
+        if (r >= nr) break;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                v[2 * e] = ok[k] ? fmaxf(acc[k][4 * c + e].x, 0.f) : 0.f;
+                v[2 * e + 1] = ok[k] ? fmaxf(acc[k][4 * c + e].y, 0.f) : 0.f;
+            }
+            uint4 o[3];
+            split8(v, o);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) out[(size_t)(p * 2 + c) * q.R + q.guard + r] = o[p];
+        }
     }
 }
 
-// gb[co] += sum_n g[co](n)
-__global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict__ g, float *__restrict__ gb, NetDims d)
+// What conv_tc_kernel does with a finished row of N sums.
+enum ConvEpi {
+    EPI_RELU = 0,   // + bias, ReLU -> split rows
+    EPI_HEAD = 1,   // + bias, ReLU (stored in FP32 when training), then the 64 -> 3 head -> dense output
+    EPI_MASK = 2    // data gradient: zero where the layer's activation is -> split rows
+};
+
+struct ConvArgs {
+    const uint4 *a;          // input split rows, 3 K / 8 planes
+    const uint4 *img;        // weight operand image
+    const float *bias;
+    uint4 *out;              // split rows, 3 N / 8 planes
+    const uint4 *mask;       // EPI_MASK: the activation's split rows (its hi planes decide)
+    const float *w4, *b4;    // EPI_HEAD
+    float *y, *act;          // EPI_HEAD: dense output [S][3][n]; FP32 rows [N / 8][rows of the tiles][8] or null
+    int *err;                // set when a bounded wait gives up
+};
+
+// One convolution as an implicit GEMM: D[row][N] = sum over 27 taps, K input
+// channels and 3 parts.  Per tile of 128 rows and (dx, dz) pair ("segment"),
+// 130 rows of every plane are brought in by bulk copies; the three dy taps are
+// the same rows shifted by one, i.e. operand addresses 16 bytes apart.
+//
+// Warp 4's first thread issues the copies, warp 5's first thread the MMAs,
+// warps 0-3 add the segment sums from TMEM (double-buffered) into FP32
+// registers and run the epilogue.  Draining every segment keeps the tensor
+// core's accumulation chains short (its adds truncate): the smallest parts go
+// in first, so 3 K / 16 adds per segment happen at full magnitude, and the
+// nine segment sums are rounded FP32 adds.  Against 64 bits the network's
+// error is below that of the FP32 FMA chains (3.3e-7 against 6.4e-7 at 129 x
+// 65 x 65).
+//
+// Persistent, weights resident (110 KB for 32 x 64).  Bound by the operand
+// reads from shared memory (4 KB of A and N 32 bytes of B per MMA) and the
+// nine reads of the activations from L2.  Measured at 129 x 65 x 65: 32 -> 64
+// with the head 249 us (0.9 PFLOP/s of BF16 MMAs; 3167 + 50 us as direct
+// FP32 convolutions on the CUDA cores), 16 -> 32 97 us (733 us); data gradients
+// of eight 33^3 samples 230 and 132 us (2988 and 784 us).
+template <int CK, int CN> struct ConvCfg {
+    static constexpr int C8 = CK / 8;
+    static constexpr int RS = kRows + 2;                    // rows of a segment
+    static constexpr int STAGE = 3 * C8 * RS * 16;          // bytes
+    static constexpr int BBYTES = 27 * CK * CN * 2;
+    static constexpr int NST = CK == 64 ? 2 : 4;
+    static constexpr int COLS = 2 * CN < 32 ? 32 : 2 * CN;  // TMEM columns (a power of two)
+    static constexpr int BARS = BBYTES + NST * STAGE;
+    static constexpr size_t SMEM = BARS + 8 * (2 * NST + 5) + 16 + 200 * 4;
+    static_assert(BBYTES % 128 == 0 && STAGE % 16 == 0 && BARS % 16 == 0, "bulk copies need 16-byte alignment");
+    static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
+};
+
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
-    const long long N = d.n();
-    const float *gc = g + (long long)blockIdx.x * N;
-    float v = 0.f;
-    for (long long n = threadIdx.x; n < N; n += blockDim.x) v += gc[n];
-    __shared__ float red[8];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+__device__ __forceinline__ void tc_commit(uint64_t *bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+
+// K-major BF16 operand without swizzle: 8 rows x 16 bytes contiguous, the
+// next 8 rows 128 bytes on (SBO), the next 8 channels lbo bytes on (LBO).
+__device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo)
+{
+    return ((uint64_t)(addr >> 4) & 0x3FFFull) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) | ((uint64_t)(128 >> 4) << 32) |
+           ((uint64_t)1 << 46);
+}
+
+template <int CK, int CN, int EPI>
+__global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
+{
+    using C = ConvCfg<CK, CN>;
+    extern __shared__ __align__(128) unsigned char sm[];
+    unsigned char *sB = sm, *sA = sm + C::BBYTES;
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + C::BARS), *empty = full + C::NST, *tfull = empty + C::NST,
+             *tempty = tfull + 2, *bbar = tempty + 2;
+    uint32_t *tbase = reinterpret_cast<uint32_t *>(bbar + 1);
+    float *hw = reinterpret_cast<float *>(tbase + 4);   // head weights [64][3] and bias
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tbase)),
+                     "r"(C::COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 128) {
+        for (int s = 0; s < C::NST; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&tfull[s], 1);
+            mbar_init(&tempty[s], 128);
+        }
+        mbar_init(bbar, 1);
+        fence_barrier_init();
+    }
+    if (EPI == EPI_HEAD)
+        for (int i = tid; i < 195; i += 192) hw[i] = i < 192 ? bf16r(A.w4[(i % 3) * 64 + i / 3]) : A.b4[i - 192];
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.f;
-        for (int q = 0; q < 8; ++q) s += red[q];
-        gb[blockIdx.x] += s;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tbase;
+    bool bad = false;
+    auto wait = [&](uint64_t *b, uint32_t parity) {
+        if (!bad && !mbar_wait_for(b, parity, kNetWaitNs)) {
+            bad = true;
+            if (A.err) *(volatile int *)A.err = GPUTO_ERR_TIMEOUT;
+        }
+    };
+    if (warp == 4) {
+        if (lane == 0) {
+            mbar_arrive_expect_tx(bbar, C::BBYTES);
+            bulk_load(sB, A.img, C::BBYTES, bbar);
+            int it = 0, issued = 0;
+            for (int tile = blockIdx.x; tile < q.ntiles && !bad; tile += gridDim.x)
+                for (int seg = 0; seg < 9; ++seg, ++it) {
+                    const int s = it % C::NST;
+                    if (it >= C::NST) wait(&empty[s], (uint32_t)((it / C::NST - 1) & 1));
+                    if (bad) break;
+                    const long long row =
+                        q.guard + (long long)tile * kRows + (long long)(seg / 3 - 1) * q.pz + (seg % 3 - 1) * q.py - 1;
+                    mbar_arrive_expect_tx(&full[s], C::STAGE);
+                    unsigned char *dst = sA + s * C::STAGE;
+                    for (int pl = 0; pl < 3 * C::C8; ++pl)
+                        bulk_load(dst + pl * (C::RS * 16), A.a + pl * q.R + row, C::RS * 16, &full[s]);
+                    ++issued;
+                }
+            // copies in flight land before the CTA leaves (they already have unless a wait gave up)
+            if (bad) {
+                mbar_wait_for(bbar, 0, kNetWaitNs);
+                for (int k = issued > C::NST ? issued - C::NST : 0; k < issued; ++k)
+                    mbar_wait_for(&full[k % C::NST], (uint32_t)((k / C::NST) & 1), kNetWaitNs);
+            }
+        }
+    } else if (warp == 5) {
+        if (lane == 0) {
+            constexpr uint32_t idesc =
+                (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(CN >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+            const uint32_t b0 = smem_u32(sB), a0 = smem_u32(sA);
+            wait(bbar, 0);
+            int it = 0;
+            for (int tile = blockIdx.x; tile < q.ntiles && !bad; tile += gridDim.x)
+                for (int seg = 0; seg < 9; ++seg, ++it) {
+                    const int s = it % C::NST, tb = it & 1;
+                    wait(&full[s], (uint32_t)((it / C::NST) & 1));
+                    if (it >= 2) wait(&tempty[tb], (uint32_t)((it / 2 - 1) & 1));
+                    if (bad) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t d = tmem + (uint32_t)(tb * CN);
+                    uint32_t acc = 0;
+#pragma unroll
+                    for (int part = 2; part >= 0; --part)
+#pragma unroll
+                        for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                            for (int ks = 0; ks < CK / 16; ++ks) {
+                                const uint64_t da = tc_desc(
+                                    a0 + s * C::STAGE + ((part * C::C8 + 2 * ks) * C::RS + dy) * 16, C::RS * 16);
+                                const uint64_t db =
+                                    tc_desc(b0 + ((3 * seg + dy) * C::C8 + 2 * ks) * CN * 16, CN * 16);
+                                asm volatile(
+                                    "{\n\t.reg .pred p;\n\t"
+                                    "setp.ne.b32 p, %4, 0;\n\t"
+                                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d),
+                                    "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+                                    : "memory");
+                                acc = 1;
+                            }
+                    tc_commit(&empty[s]);
+                    tc_commit(&tfull[tb]);
+                }
+            // MMAs in flight end before TMEM is freed
+            if (bad && it > 0) mbar_wait_for(&tfull[(it - 1) & 1], (uint32_t)(((it - 1) / 2) & 1), kNetWaitNs);
+        }
+    } else {
+        const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
+        int it = 0;
+        for (int tile = blockIdx.x; tile < q.ntiles && !bad; tile += gridDim.x) {
+            float acc[CN];
+#pragma unroll
+            for (int c = 0; c < CN; ++c) acc[c] = 0.f;
+            for (int seg = 0; seg < 9; ++seg, ++it) {
+                const int tb = it & 1;
+                wait(&tfull[tb], (uint32_t)((it / 2) & 1));
+                if (__any_sync(0xffffffffu, bad)) {   // the TMEM loads are warp-wide
+                    bad = true;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int c0 = 0; c0 < CN; c0 += 16) {
+                    uint32_t r[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+                        "tcgen05.wait::ld.sync.aligned;"
+                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+                          "=r"(r[14]), "=r"(r[15])
+                        : "r"(tmem + lane_off + (uint32_t)(tb * CN + c0))
+                        : "memory");
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) acc[c0 + c] += __uint_as_float(r[c]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[tb])) : "memory");
+            }
+            if (bad) break;
+            const long long r = (long long)tile * kRows + warp * 32 + lane;
+            int s, x, z, y;
+            const bool in = row_node(q, r, s, x, z, y);
+            if (EPI == EPI_HEAD) {
+                float o3[3] = {hw[192], hw[193], hw[194]};
+#pragma unroll
+                for (int c = 0; c < CN; ++c) {
+                    acc[c] = in ? fmaxf(acc[c] + A.bias[c], 0.f) : 0.f;
+#pragma unroll
+                    for (int o = 0; o < 3; ++o) o3[o] = fmaf(hw[3 * c + o], acc[c], o3[o]);
+                }
+                if (in) {
+                    const long long n = (long long)q.X * q.Z * q.Y, at = ((long long)x * q.Z + z) * q.Y + y;
+#pragma unroll
+                    for (int o = 0; o < 3; ++o) A.y[(3LL * s + o) * n + at] = o3[o];
+                }
+                if (A.act) {
+                    float4 *dst = reinterpret_cast<float4 *>(A.act);
+                    const size_t nr = (size_t)q.ntiles * kRows;
+#pragma unroll
+                    for (int c = 0; c < CN / 8; ++c)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            dst[2 * (c * nr + r) + h] = make_float4(acc[8 * c + 4 * h], acc[8 * c + 4 * h + 1],
+                                                                    acc[8 * c + 4 * h + 2], acc[8 * c + 4 * h + 3]);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < CN / 8; ++c) {
+                    float v[8];
+                    if (EPI == EPI_RELU) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] = in ? fmaxf(acc[8 * c + e] + A.bias[8 * c + e], 0.f) : 0.f;
+                    } else {
+                        const uint4 m = A.mask[(size_t)c * q.R + q.guard + r];
+                        const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            v[e] = in && ((e & 1) ? (mw[e >> 1] >> 16) : (mw[e >> 1] & 0xFFFFu)) ? acc[8 * c + e] : 0.f;
+                    }
+                    uint4 o[3];
+                    split8(v, o);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) A.out[(size_t)(p * (CN / 8) + c) * q.R + q.guard + r] = o[p];
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::COLS) : "memory");
+}
+
+// Backward through the head and layer 3's ReLU: from the output gradient gy
+// (dense [S][3][n]) and the FP32 activations, the split rows of layer 3's
+// gradient, g3 = [act > 0] w4' gy, and the CTA's partial sums of the head's
+// weight and bias gradients, part[CTA][195] (co 64 + ci, then co).
+constexpr int kHeadPart = 195;
+
+__global__ void __launch_bounds__(256)
+head_backward_kernel(const float *__restrict__ gy, const float *__restrict__ act, const float *__restrict__ w4,
+                     uint4 *__restrict__ g3, float *__restrict__ part, RowGeo q)
+{
+    __shared__ float as[kRows][65], gs[kRows][4], hw[192];
+    const int tid = threadIdx.x;
+    if (tid < 192) hw[tid] = bf16r(w4[tid]);
+    const long long n = (long long)q.X * q.Z * q.Y;
+    const size_t nr = (size_t)q.ntiles * kRows;
+    float sum = 0.f;
+    for (int tile = blockIdx.x; tile < q.ntiles; tile += gridDim.x) {
+        __syncthreads();
+        if (tid < kRows) {
+            int s, x, z, y;
+            const bool in = row_node(q, (long long)tile * kRows + tid, s, x, z, y);
+            const long long at = ((long long)x * q.Z + z) * q.Y + y;
+#pragma unroll
+            for (int o = 0; o < 3; ++o) gs[tid][o] = in ? gy[(3LL * s + o) * n + at] : 0.f;
+        }
+        __syncthreads();
+        for (int i = tid; i < 8 * kRows; i += 256) {   // (chunk, row)
+            const int c = i / kRows, rr = i - c * kRows;
+            const size_t r = (size_t)tile * kRows + rr;
+            const float4 *src = reinterpret_cast<const float4 *>(act) + 2 * (c * nr + r);
+            const float4 lo = src[0], hi = src[1];
+            const float a[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                as[rr][8 * c + e] = a[e];
+                float g = hw[8 * c + e] * gs[rr][0];
+                g = fmaf(hw[64 + 8 * c + e], gs[rr][1], g);
+                g = fmaf(hw[128 + 8 * c + e], gs[rr][2], g);
+                v[e] = a[e] > 0.f ? g : 0.f;
+            }
+            uint4 o[3];
+            split8(v, o);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) g3[(size_t)(p * 8 + c) * q.R + q.guard + r] = o[p];
+        }
+        __syncthreads();
+        if (tid < 192) {
+            const int co = tid >> 6, ci = tid & 63;
+#pragma unroll 8
+            for (int rr = 0; rr < kRows; ++rr) sum = fmaf(gs[rr][co], as[rr][ci], sum);
+        } else if (tid < kHeadPart) {
+            for (int rr = 0; rr < kRows; ++rr) sum += gs[rr][tid - 192];
+        }
+    }
+    if (tid < kHeadPart) part[(size_t)blockIdx.x * kHeadPart + tid] = sum;
+}
+
+// Weight gradients gw[co][ci][tap] = sum over rows of g[row][co]
+// x[row + offset(tap)][ci] and bias gradients, one CTA per (row range, dx).
+// A thread keeps G output channels x the 9 (dz, dy) taps of one input channel
+// in registers: per row it reads its G gradients (the same for a warp) and
+// three new input values (the dy taps slide along the row), for 9 G FMAs as
+// paired instructions, so it runs near the FMA rate.  The CTAs' sums go to
+// part[range][(co CI + ci) 27 + tap] and are added in a fixed order
+// (sum_parts_kernel).  Eight 33^3 samples: 892, 290 and 153 us for the three
+// layers (the 32 -> 64 one at 53 % of the FMA rate), 8616 us together with one
+// CTA per (co, ci) pair and per sample.  Layer 1 reads its input from the dense [S][4][n].
+constexpr int kWgRows = 48;   // rows staged at a time
+
+template <int CO, int CI, int G, bool DENSE>
+__global__ void __launch_bounds__((CO / G) * CI)
+wgrad_kernel(const uint4 *__restrict__ g, const uint4 *__restrict__ xr, const float *__restrict__ xd,
+             float *__restrict__ part, float *__restrict__ bpart, RowGeo q, int tiles_per)
+{
+    constexpr int NT = (CO / G) * CI, GP = CO + 4, XP = CI + 4;
+    __shared__ __align__(16) float gs[kWgRows][GP];
+    __shared__ __align__(16) float xs[3][kWgRows + 2][XP];
+    const int tid = threadIdx.x, ci = tid % CI, cg = tid / CI;
+    const int dx = (int)blockIdx.y - 1;
+    const long long ntile = (q.rows + kWgRows - 1) / kWgRows;
+    const long long t0 = (long long)blockIdx.x * tiles_per, t1 = min(t0 + tiles_per, ntile);
+    float2 acc[G / 2][9], bsum[G / 2];
+#pragma unroll
+    for (int c = 0; c < G / 2; ++c) {
+        bsum[c] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int t = 0; t < 9; ++t) acc[c][t] = make_float2(0.f, 0.f);
+    }
+    for (long long tile = t0; tile < t1; ++tile) {
+        const long long r0 = tile * kWgRows;
+        __syncthreads();
+        for (int i = tid; i < kWgRows * (CO / 8); i += NT) {
+            const int c = i / kWgRows, rr = i - c * kWgRows;
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (r0 + rr < q.rows)
+#pragma unroll
+                for (int p = 2; p >= 0; --p) add_part(v, g[(size_t)(p * (CO / 8) + c) * q.R + q.guard + r0 + rr]);
+            float4 *d = reinterpret_cast<float4 *>(&gs[rr][8 * c]);
+            d[0] = make_float4(v[0], v[1], v[2], v[3]);
+            d[1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+        if constexpr (DENSE) {
+            const long long n = (long long)q.X * q.Z * q.Y;
+            for (int i = tid; i < 3 * (kWgRows + 2) * CI; i += NT) {
+                const int rr = i % (kWgRows + 2), rest = i / (kWgRows + 2), c = rest % CI, dz = rest / CI;
+                const long long r = r0 + rr - 1 + (long long)dx * q.pz + (dz - 1) * q.py;
+                int s, x, z, y;
+                const bool in = r >= 0 && row_node(q, r, s, x, z, y);
+                xs[dz][rr][c] = in ? xd[(4LL * s + c) * n + ((long long)x * q.Z + z) * q.Y + y] : 0.f;
+            }
+        } else {
+            for (int i = tid; i < 3 * (kWgRows + 2) * (CI / 8); i += NT) {
+                const int rr = i % (kWgRows + 2), rest = i / (kWgRows + 2), c = rest % (CI / 8), dz = rest / (CI / 8);
+                const long long r = q.guard + r0 + rr - 1 + (long long)dx * q.pz + (dz - 1) * q.py;
+                float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                if (r < q.R)   // the last tile's overhang meets zero gradients
+#pragma unroll
+                    for (int p = 2; p >= 0; --p) add_part(v, xr[(size_t)(p * (CI / 8) + c) * q.R + r]);
+                float4 *d = reinterpret_cast<float4 *>(&xs[dz][rr][8 * c]);
+                d[0] = make_float4(v[0], v[1], v[2], v[3]);
+                d[1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        }
+        __syncthreads();
+        float xw[3][3];   // [dz][row mod 3]
+#pragma unroll
+        for (int dz = 0; dz < 3; ++dz) {
+            xw[dz][0] = xs[dz][0][ci];
+            xw[dz][1] = xs[dz][1][ci];
+        }
+#pragma unroll 1
+        for (int rb = 0; rb < kWgRows; rb += 3)
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                const int rr = rb + u;
+                float2 gv[G / 2];
+                if constexpr (G >= 4) {
+#pragma unroll
+                    for (int c = 0; c < G / 4; ++c) {
+                        const float4 f = *reinterpret_cast<const float4 *>(&gs[rr][cg * G + 4 * c]);
+                        gv[2 * c] = make_float2(f.x, f.y);
+                        gv[2 * c + 1] = make_float2(f.z, f.w);
+                    }
+                } else {
+                    gv[0] = *reinterpret_cast<const float2 *>(&gs[rr][cg * G]);
+                }
+#pragma unroll
+                for (int dz = 0; dz < 3; ++dz) xw[dz][(u + 2) % 3] = xs[dz][rr + 2][ci];
+                if (dx == -1)
+#pragma unroll
+                    for (int c = 0; c < G / 2; ++c) bsum[c] = __fadd2_rn(bsum[c], gv[c]);
+#pragma unroll
+                for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+                    for (int dy = 0; dy < 3; ++dy) {
+                        const float v = xw[dz][(u + dy) % 3];
+#pragma unroll
+                        for (int c = 0; c < G / 2; ++c)
+                            acc[c][3 * dz + dy] = __ffma2_rn(gv[c], make_float2(v, v), acc[c][3 * dz + dy]);
+                    }
+            }
+    }
+    float *dst = part + (size_t)blockIdx.x * (CO * CI * 27) + 9 * blockIdx.y;
+#pragma unroll
+    for (int c = 0; c < G / 2; ++c)
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {
+            dst[((cg * G + 2 * c) * CI + ci) * 27 + t] = acc[c][t].x;
+            dst[((cg * G + 2 * c + 1) * CI + ci) * 27 + t] = acc[c][t].y;
+        }
+    if (dx == -1 && ci == 0)
+#pragma unroll
+        for (int c = 0; c < G / 2; ++c) {
+            bpart[(size_t)blockIdx.x * CO + cg * G + 2 * c] = bsum[c].x;
+            bpart[(size_t)blockIdx.x * CO + cg * G + 2 * c + 1] = bsum[c].y;
+        }
+}
+
+// grads[i] += sum over ranges of part[range][i]: a CTA takes 32 entries, its
+// eight warps every eighth range, and the warps' sums are added in order.
+__global__ void __launch_bounds__(256)
+sum_parts_kernel(const float *__restrict__ part, int n, int ranges, float *__restrict__ grads)
+{
+    __shared__ float red[8][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    float s = 0.f;
+    if (i < n)
+#pragma unroll 8
+        for (int b = w; b < ranges; b += 8) s += part[(size_t)b * n + i];
+    red[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && i < n) {
+        s = red[0][lane];
+        for (int k = 1; k < 8; ++k) s += red[k][lane];
+        grads[i] += s;
     }
 }
 
-// g <- g where the layer's ReLU output is positive, else 0
-__global__ void relu_mask_kernel(float *__restrict__ g, const float *__restrict__ y, long long n)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !(y[i] > 0.f)) g[i] = 0.f;
-}
-
-// Masked mean square error of one sample: partial sums per CTA, then a
-// single-CTA finish that also writes the gradient scale; fixed order.
+// Masked mean square error: partial sums per CTA (blockIdx.y = sample), then
+// a single-CTA finish (a warp per sample, lanes in order of the CTAs) that
+// adds the losses and writes the gradients' scales; fixed order.
 __global__ void __launch_bounds__(256)
 mse_partial_kernel(const float *__restrict__ y, const float *__restrict__ t, const float *__restrict__ m, long long n,
                    double *__restrict__ part)
 {
+    const long long o = (long long)blockIdx.y * n;
     double s = 0.0, c = 0.0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const double r = (double)y[i] - (double)t[i];
-        s += (double)m[i] * r * r;
-        c += (double)m[i];
+        const double r = (double)y[o + i] - (double)t[o + i];
+        s += (double)m[o + i] * r * r;
+        c += (double)m[o + i];
     }
     __shared__ double rs[8], rc[8];
-    for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-        c += __shfl_xor_sync(0xffffffffu, c, o);
+    for (int w = 16; w > 0; w >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, w);
+        c += __shfl_xor_sync(0xffffffffu, c, w);
     }
     if ((threadIdx.x & 31) == 0) rs[threadIdx.x >> 5] = s, rc[threadIdx.x >> 5] = c;
     __syncthreads();
     if (threadIdx.x == 0) {
         double a = 0.0, b = 0.0;
-        for (int q = 0; q < 8; ++q) a += rs[q], b += rc[q];
-        part[2 * blockIdx.x] = a;
-        part[2 * blockIdx.x + 1] = b;
+        for (int w = 0; w < 8; ++w) a += rs[w], b += rc[w];
+        double *p = part + 2 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x);
+        p[0] = a;
+        p[1] = b;
     }
 }
 
-__global__ void mse_finish_kernel(const double *__restrict__ part, int nb, double *__restrict__ loss_acc,
-                                  float *__restrict__ gscale)
+__global__ void __launch_bounds__(1024)
+mse_finish_kernel(const double *__restrict__ part, int nb, int samples, double *__restrict__ loss_acc,
+                  float *__restrict__ gscale)
 {
-    if (threadIdx.x != 0) return;
-    double a = 0.0, b = 0.0;
-    for (int q = 0; q < nb; ++q) a += part[2 * q], b += part[2 * q + 1];
-    const double den = b > 1.0 ? b : 1.0;
-    *loss_acc += a / den;
-    *gscale = (float)(2.0 / den);
+    __shared__ double ls[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < samples; s0 += 32) {
+        const int s = s0 + warp;
+        double a = 0.0, b = 0.0;
+        if (s < samples)
+            for (int k = lane; k < nb; k += 32) {
+                a += part[2 * ((size_t)s * nb + k)];
+                b += part[2 * ((size_t)s * nb + k) + 1];
+            }
+        for (int w = 16; w > 0; w >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, w);
+            b += __shfl_xor_sync(0xffffffffu, b, w);
+        }
+        const double den = b > 1.0 ? b : 1.0;
+        if (lane == 0) {
+            ls[warp] = s < samples ? a / den : 0.0;
+            if (s < samples) gscale[s] = (float)(2.0 / den);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double l = *loss_acc;
+            for (int w = 0; w < 32; ++w) l += ls[w];
+            *loss_acc = l;
+        }
+        __syncthreads();
+    }
 }
 
 __global__ void mse_grad_kernel(const float *__restrict__ y, const float *__restrict__ t, const float *__restrict__ m,
                                 long long n, const float *__restrict__ gscale, float *__restrict__ g)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) g[i] = *gscale * m[i] * (y[i] - t[i]);
+    const long long o = (long long)blockIdx.y * n + i;
+    if (i < n) g[o] = gscale[blockIdx.y] * m[o] * (y[o] - t[o]);
 }
 
 __global__ void adam_kernel(float *__restrict__ p, float *__restrict__ g, float *__restrict__ m1, float *__restrict__ m2,
@@ -247,30 +809,42 @@ __global__ void adam_kernel(float *__restrict__ p, float *__restrict__ g, float 
     g[i] = 0.f;
 }
 
-template <int CIN, int COT, int K, bool RELU>
-void launch_fwd(const float *x, const float *w, const float *b, float *y, const NetDims &d, int cout, cudaStream_t st)
+// Persistent grids: CTAs per SM by shared memory (1 for K N >= 2048, else 2).
+template <int CK, int CN, int EPI>
+void launch_conv(const ConvArgs &a, const RowGeo &q, int sms, cudaStream_t st)
 {
-    constexpr int K3 = K * K * K;
-    const size_t smem = sizeof(float) * CIN * K3 * COT;
-    const dim3 grid((unsigned)((d.n() + kNetThreads - 1) / kNetThreads), (unsigned)((cout + COT - 1) / COT));
-    conv_fwd_kernel<CIN, COT, K, RELU><<<grid, kNetThreads, smem, st>>>(x, w, b, y, d, cout);
+    using C = ConvCfg<CK, CN>;
+    const int per = C::SMEM <= 113 * 1024 ? 2 : 1;
+    conv_tc_kernel<CK, CN, EPI><<<std::min(q.ntiles, per * sms), 192, C::SMEM, st>>>(a, q);
     count_launches(1);
 }
 
-template <int COUT, int CIT, int K>
-void launch_bwd_data(const float *g, const float *w, float *gx, const NetDims &d, int cin, cudaStream_t st)
+// Row ranges of the weight-gradient kernels (a CTA per range and dx): two CTAs
+// of 256 threads per SM for 64 x 32 channels, and as many more of the smaller
+// CTAs of the other layers (98 ranges for those left most of the chip idle:
+// 353 and 848 us on eight 33^3 samples).
+constexpr int kWgRanges = 98;
+constexpr int kWgMaxWeights = kWgRanges * 64 * 32 * 27, kWgMaxBias = 8 * kWgRanges * 16;
+
+template <int CO, int CI, int G, bool DENSE>
+void launch_wgrad(const uint4 *g, const uint4 *xr, const float *xd, float *part, float *bpart, float *gw, float *gb,
+                  const RowGeo &q, cudaStream_t st)
 {
-    constexpr int K3 = K * K * K;
-    const size_t smem = sizeof(float) * COUT * K3 * CIT;
-    const dim3 grid((unsigned)((d.n() + kNetThreads - 1) / kNetThreads), (unsigned)((cin + CIT - 1) / CIT));
-    conv_bwd_data_kernel<COUT, CIT, K><<<grid, kNetThreads, smem, st>>>(g, w, gx, d, cin);
-    count_launches(1);
+    constexpr int NT = (CO / G) * CI, MAXR = kWgRanges * (256 / NT);   // 98, 196, 784
+    static_assert(MAXR * CO * CI * 27 <= kWgMaxWeights && MAXR * CO <= kWgMaxBias, "partial sums");
+    const long long ntile = (q.rows + kWgRows - 1) / kWgRows;
+    const int per = (int)((ntile + MAXR - 1) / MAXR), ranges = (int)((ntile + per - 1) / per);
+    wgrad_kernel<CO, CI, G, DENSE><<<dim3((unsigned)ranges, 3), NT, 0, st>>>(g, xr, xd, part, bpart, q, per);
+    const int n = CO * CI * 27;
+    sum_parts_kernel<<<(n + 31) / 32, 256, 0, st>>>(part, n, ranges, gw);
+    sum_parts_kernel<<<(CO + 31) / 32, 256, 0, st>>>(bpart, CO, ranges, gb);
+    count_launches(3);
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Net: parameters, Adam state and activation buffers on one device
+// Net: parameters, Adam state and work buffers on one device
 // ---------------------------------------------------------------------------
 
 long long Net::num_params()
@@ -291,24 +865,30 @@ long long Net::param_offset(int l, bool bias)
 Net::~Net()
 {
     for (void *p : owned) cudaFree(p);
-    for (int l = 1; l <= 4; ++l) cudaFree(act[l]);
-    cudaFree(gA);
-    cudaFree(gB);
+    if (h_err) cudaFreeHost(h_err);
 }
 
 int Net::create(unsigned long long seed)
 {
     GPUTO_CUDA(cudaGetDevice(&device));
+    GPUTO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const long long np = num_params();
     for (float **p : {&params, &grads, &m1, &m2}) {
         GPUTO_CUDA(cudaMalloc(p, sizeof(float) * np));
         owned.push_back(*p);
         GPUTO_CUDA(cudaMemset(*p, 0, sizeof(float) * np));
     }
-    GPUTO_CUDA(cudaMalloc(&part, sizeof(double) * 2 * 1024 + sizeof(double) + sizeof(float)));
+    // part: kNetPart doubles of reduction scratch, the summed loss, a gradient scale per sample of a group
+    GPUTO_CUDA(cudaMalloc(&part, sizeof(double) * (kNetPart + 1) + sizeof(float) * kNetGroup));
     owned.push_back(part);
-    loss_acc = part + 2 * 1024;   // part: 2048 doubles of reduction scratch
+    loss_acc = part + kNetPart;
     gscale = reinterpret_cast<float *>(loss_acc + 1);
+    GPUTO_CUDA(cudaMalloc(&img, 2 * 2 * (size_t)(kImg2 + kImg3)));
+    owned.push_back(img);
+    // where a kernel's bounded wait reports that it gave up: read by the host after a synchronisation
+    GPUTO_CUDA(cudaHostAlloc((void **)&h_err, sizeof(int), cudaHostAllocMapped));
+    *h_err = 0;
+    GPUTO_CUDA(cudaHostGetDevicePointer((void **)&d_err, h_err, 0));
     // He-normal initial weights (last layer scaled by 0.1), zero biases;
     // a fixed generator so that a seed reproduces the network
     std::vector<float> h((size_t)np, 0.f);
@@ -330,19 +910,41 @@ int Net::create(unsigned long long seed)
     return GPUTO_OK;
 }
 
-int Net::reserve(long long n)
+// Work buffers for S samples of a grid at once (train: also the backward
+// pass's).  They only grow; a buffer that is outgrown stays allocated until
+// the network goes, since a solver's captured graph may still use it.
+int Net::reserve(const NetDims &d, int S, bool train)
 {
-    if (n <= cap_n) return GPUTO_OK;
-    for (int l = 1; l <= 4; ++l) cudaFree(act[l]), act[l] = nullptr;
-    cudaFree(gA), cudaFree(gB);
-    gA = gB = nullptr;
-    cap_n = 0;
-    const int chs[5] = {4, 16, 32, 64, 3};
-    for (int l = 1; l <= 4; ++l) GPUTO_CUDA(cudaMalloc(&act[l], sizeof(float) * chs[l] * n));
-    GPUTO_CUDA(cudaMalloc(&gA, sizeof(float) * 64 * n));
-    GPUTO_CUDA(cudaMalloc(&gB, sizeof(float) * 64 * n));
-    cap_n = n;
-    return GPUTO_OK;
+    const RowGeo q = row_geo(d, S);
+    auto grow = [&](auto **p, size_t &cap, size_t bytes) -> int {
+        if (bytes <= cap) return GPUTO_OK;
+        void *v = nullptr;
+        GPUTO_CUDA(cudaMalloc(&v, bytes));
+        owned.push_back(v);
+        *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(v);
+        cap = bytes;
+        return GPUTO_OK;
+    };
+    const size_t plane = 16 * (size_t)q.R, dense = sizeof(float) * 3 * (size_t)d.n() * S;
+    int s = grow(&rows1, cap[0], 6 * plane);
+    if (!s) s = grow(&rows2, cap[1], 12 * plane);
+    if (!s) s = grow(&y, cap[2], dense);
+    if (train) {
+        if (!s) s = grow(&gy, cap[3], dense);
+        if (!s) s = grow(&act3, cap[4], sizeof(float) * 64 * (size_t)q.ntiles * kRows);
+        if (!s) s = grow(&g3, cap[5], 24 * plane);
+        if (!s) s = grow(&g2, cap[6], 12 * plane);
+        if (!s) s = grow(&g1, cap[7], 6 * plane);
+        if (!s) s = grow(&wpart, cap[8], sizeof(float) * ((size_t)kWgMaxWeights + kWgMaxBias +
+                                                          (size_t)2 * sms * kHeadPart));
+    }
+    return s;
+}
+
+int Net::group(const NetDims &d, int ns) const
+{
+    const long long per = row_geo(d, 1).rows;
+    return (int)std::max(1LL, std::min<long long>({(long long)ns, (long long)kNetGroup, (1LL << 20) / per}));
 }
 
 int init_net_kernels()
@@ -351,43 +953,71 @@ int init_net_kernels()
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && done[dev]) return GPUTO_OK;
-    GPUTO_CUDA(cudaFuncSetAttribute(conv_fwd_kernel<32, 16, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    32 * 27 * 16 * 4));
-    GPUTO_CUDA(cudaFuncSetAttribute(conv_bwd_data_kernel<64, 16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    64 * 27 * 16 * 4));
-    GPUTO_CUDA(cudaFuncSetAttribute(conv_bwd_data_kernel<32, 16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    32 * 27 * 16 * 4));
+    auto set = [](auto *k, size_t b) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+    };
+    GPUTO_CUDA(set(conv_tc_kernel<16, 32, EPI_RELU>, ConvCfg<16, 32>::SMEM));
+    GPUTO_CUDA(set(conv_tc_kernel<32, 64, EPI_HEAD>, ConvCfg<32, 64>::SMEM));
+    GPUTO_CUDA(set(conv_tc_kernel<64, 32, EPI_MASK>, ConvCfg<64, 32>::SMEM));
+    GPUTO_CUDA(set(conv_tc_kernel<32, 16, EPI_MASK>, ConvCfg<32, 16>::SMEM));
     if (dev < 64) done[dev] = true;
     return GPUTO_OK;
 }
 
-int Net::forward(const float *x, const NetDims &d, float *y, cudaStream_t st)
+int Net::check()
 {
-    int s = reserve(d.n());
+    if (!*(volatile int *)h_err) return GPUTO_OK;
+    const int e = *(volatile int *)h_err;
+    *(volatile int *)h_err = 0;
+    set_error("a bounded wait of the network's convolution gave up");
+    return e;
+}
+
+int Net::forward(const float *x, const NetDims &d, int S, float *yout, bool train, cudaStream_t st)
+{
+    int s = reserve(d, S, train);
     if (s) return s;
-    act[0] = const_cast<float *>(x);
+    const RowGeo q = row_geo(d, S);
     const float *p = params;
-    launch_fwd<4, 16, 3, true>(x, p + param_offset(0, false), p + param_offset(0, true), act[1], d, 16, st);
-    launch_fwd<16, 16, 3, true>(act[1], p + param_offset(1, false), p + param_offset(1, true), act[2], d, 32, st);
-    launch_fwd<32, 16, 3, true>(act[2], p + param_offset(2, false), p + param_offset(2, true), act[3], d, 64, st);
-    launch_fwd<64, 3, 1, false>(act[3], p + param_offset(3, false), p + param_offset(3, true), y ? y : act[4], d, 3,
-                                st);
+    GuardSets gs{{rows1, rows2, g3, g2, nullptr}, {6, 12, 24, 12, 0}};
+    zero_guards_kernel<<<dim3(64, train ? 4 : 2), 256, 0, st>>>(gs, q);
+    pack_weights_kernel<<<(2 * (kImg2 + kImg3) + 255) / 256, 256, 0, st>>>(p + param_offset(1, false),
+                                                                          p + param_offset(2, false),
+                                                                          (__nv_bfloat16 *)img);
+    conv1_kernel<<<(q.ntiles + kC1R - 1) / kC1R, 128, 0, st>>>(x, p + param_offset(0, false), p + param_offset(0, true), rows1, q);
+    count_launches(3);
+    const uint4 *im = reinterpret_cast<const uint4 *>(img);
+    ConvArgs a{};
+    a.err = d_err;
+    a.a = rows1;
+    a.img = im;
+    a.bias = p + param_offset(1, true);
+    a.out = rows2;
+    launch_conv<16, 32, EPI_RELU>(a, q, sms, st);
+    a.a = rows2;
+    a.img = im + kImg2 / 8;
+    a.bias = p + param_offset(2, true);
+    a.w4 = p + param_offset(3, false);
+    a.b4 = p + param_offset(3, true);
+    a.y = yout ? yout : y;
+    a.act = train ? act3 : nullptr;
+    launch_conv<32, 64, EPI_HEAD>(a, q, sms, st);
     return GPUTO_OK;
 }
 
-// Loss of one sample (x, target t, mask m) added to loss_acc, gradients
+// Losses of S samples (x, target t, mask m) added to loss_acc, gradients
 // added to grads.
-int Net::accumulate(const float *x, const float *t, const float *m, const NetDims &d, cudaStream_t st)
+int Net::accumulate(const float *x, const float *t, const float *m, const NetDims &d, int S, cudaStream_t st)
 {
-    int s = forward(x, d, nullptr, st);
+    int s = forward(x, d, S, nullptr, true, st);
     if (s) return s;
-    const long long N = d.n(), n3 = 3 * N;
-    const int nb = (int)std::min<long long>(1024, (n3 + 255) / 256);
-    mse_partial_kernel<<<nb, 256, 0, st>>>(act[4], t, m, n3, part);
-    mse_finish_kernel<<<1, 32, 0, st>>>(part, nb, loss_acc, gscale);
-    mse_grad_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>(act[4], t, m, n3, gscale, gA);
+    const long long n3 = 3 * d.n();
+    const int nb = (int)std::max(1LL, std::min<long long>(kNetPart / 2 / S, (n3 + 255) / 256));
+    mse_partial_kernel<<<dim3((unsigned)nb, (unsigned)S), 256, 0, st>>>(y, t, m, n3, part);
+    mse_finish_kernel<<<1, 1024, 0, st>>>(part, nb, S, loss_acc, gscale);
+    mse_grad_kernel<<<dim3((unsigned)((n3 + 255) / 256), (unsigned)S), 256, 0, st>>>(y, t, m, n3, gscale, gy);
     count_launches(3);
-    return backward_from(d, st);
+    return backward_from(x, d, S, st);
 }
 
 int Net::adam(float lr, int nsamples, cudaStream_t st)
@@ -398,6 +1028,39 @@ int Net::adam(float lr, int nsamples, cudaStream_t st)
     adam_kernel<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(params, grads, m1, m2, np, lr,
                                                              1.f / (float)std::max(nsamples, 1), bc1, bc2);
     count_launches(1);
+    return GPUTO_OK;
+}
+
+// The backward pass of the last training forward from the output gradient in
+// gy; adds to grads.
+int Net::backward_from(const float *x, const NetDims &d, int S, cudaStream_t st)
+{
+    const RowGeo q = row_geo(d, S);
+    const float *p = params;
+    float *bpart = wpart + kWgMaxWeights, *hpart = bpart + kWgMaxBias;
+    const int hb = std::min(q.ntiles, 2 * sms);
+    head_backward_kernel<<<hb, 256, 0, st>>>(gy, act3, p + param_offset(3, false), g3, hpart, q);
+    // the head's 192 weights and 3 biases are adjacent in grads
+    sum_parts_kernel<<<(kHeadPart + 31) / 32, 256, 0, st>>>(hpart, kHeadPart, hb, grads + param_offset(3, false));
+    count_launches(2);
+    const uint4 *im = reinterpret_cast<const uint4 *>(img);
+    ConvArgs a{};
+    a.err = d_err;
+    a.a = g3;
+    a.img = im + (kImg2 + kImg3) / 8;
+    a.mask = rows2;
+    a.out = g2;
+    launch_conv<64, 32, EPI_MASK>(a, q, sms, st);
+    a.a = g2;
+    a.img = im + (kImg2 + 2 * kImg3) / 8;
+    a.mask = rows1;
+    a.out = g1;
+    launch_conv<32, 16, EPI_MASK>(a, q, sms, st);
+    auto gw = [&](int l) { return grads + param_offset(l, false); };
+    auto gb = [&](int l) { return grads + param_offset(l, true); };
+    launch_wgrad<64, 32, 8, false>(g3, rows2, nullptr, wpart, bpart, gw(2), gb(2), q, st);
+    launch_wgrad<32, 16, 4, false>(g2, rows1, nullptr, wpart, bpart, gw(1), gb(1), q, st);
+    launch_wgrad<16, 4, 2, true>(g1, nullptr, x, wpart, bpart, gw(0), gb(0), q, st);
     return GPUTO_OK;
 }
 
@@ -686,36 +1349,6 @@ int launch_net_energy(const Lay &L2, const float *y, const float *q, const float
     net_energy_kernel<<<nb, 256, 0, st>>>(L2, y, q, diag2, gt, mask2, gy, part);
     net_energy_finish_kernel<<<1, 32, 0, st>>>(part, nb, loss_acc);
     count_launches(2);
-    return GPUTO_OK;
-}
-
-// The backward pass from a given output gradient gA (3 channels); adds to grads.
-int Net::backward_from(const NetDims &d, cudaStream_t st)
-{
-    const long long N = d.n();
-    float *g = gA, *gn = gB;
-    for (int l = 3; l >= 0; --l) {
-        const int cin = net_ch(l), cout = net_ch(l + 1);
-        float *gw = grads + param_offset(l, false), *gb = grads + param_offset(l, true);
-        if (l < 3) {
-            relu_mask_kernel<<<(unsigned)((cout * N + 255) / 256), 256, 0, st>>>(g, act[l + 1], cout * N);
-            count_launches(1);
-        }
-        if (net_k(l) == 3)
-            conv_bwd_weight_kernel<3><<<cout * cin, 256, 0, st>>>(g, act[l], gw, d, cin);
-        else
-            conv_bwd_weight_kernel<1><<<cout * cin, 256, 0, st>>>(g, act[l], gw, d, cin);
-        bias_grad_kernel<<<cout, 256, 0, st>>>(g, gb, d);
-        count_launches(2);
-        if (l == 0) break;
-        const float *w = params + param_offset(l, false);
-        switch (l) {
-        case 3: launch_bwd_data<3, 16, 1>(g, w, gn, d, 64, st); break;
-        case 2: launch_bwd_data<64, 16, 3>(g, w, gn, d, 32, st); break;
-        default: launch_bwd_data<32, 16, 3>(g, w, gn, d, 16, st); break;
-        }
-        std::swap(g, gn);
-    }
     return GPUTO_OK;
 }
 

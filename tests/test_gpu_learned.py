@@ -68,6 +68,38 @@ def test_mse_gradient_matches_oracle(gputo):
     assert np.array_equal(net.get_params(), th)
 
 
+@pytest.mark.parametrize("dims,ns", [((1, 1, 1), 1), ((2, 1, 2), 257), ((3, 2, 129), 2), ((7, 12, 31), 3), ((4, 40, 1), 2)])
+def test_tiles_and_samples_match_oracle(gputo, dims, ns):
+    """Forward and gradients where the 128-row tiles and the stacked samples can
+    go wrong: grids smaller than a tile, lines longer than one, single lines and
+    planes, tiles that end inside a line, and more samples than one pass takes.
+    Sums of up to 864 products in FP32: 864 2^-24 = 5e-5 of the largest, within
+    the tolerances of the tests above."""
+    import torch
+    rng = np.random.default_rng(int(np.prod(dims)) + ns)
+    th = learned.init_params(3)
+    th[learned.num_params() - 3:] = [0.1, -0.2, 0.3]
+    xs = rng.standard_normal((ns, 4) + dims).astype(np.float32)
+    ts = rng.standard_normal((ns, 3) + dims).astype(np.float32)
+    ms = (rng.random((ns, 3) + dims) > 0.3).astype(np.float32)
+    net = gputo.Net(seed=0)
+    net.set_params(th)
+    y = torch.empty(3 * int(np.prod(dims)), dtype=torch.float32, device="cuda")
+    net.forward(_f32(xs[0]), dims, y)
+    ref, _ = learned.forward(xs[0], th)
+    assert np.abs(y.cpu().numpy().reshape(ref.shape) - ref).max() <= 1e-4 * np.abs(ref).max()
+    g = np.zeros(learned.num_params(), dtype=np.float32)
+    loss = net.train_step(_f32(xs), _f32(ts), _f32(ms), ns, dims, 0.0, grads_out=g)
+    ref_g, ref_l = np.zeros(learned.num_params()), 0.0
+    for q in range(ns):
+        yq, acts = learned.forward(xs[q], th)
+        l, gy = learned.loss(yq, ts[q], ms[q])
+        ref_l += l / ns
+        ref_g += learned.backward(acts, th, gy)
+    assert abs(loss - ref_l) <= 1e-4 * abs(ref_l)
+    assert np.abs(g - ref_g).max() <= 1e-3 * np.abs(ref_g).max()
+
+
 def _problem(gputo, shape=(64, 32, 32), nl=4, seed=0):
     import torch
     F, fixed = gputo.cantilever(*shape)
