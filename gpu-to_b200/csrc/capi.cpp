@@ -940,17 +940,16 @@ int gputo_simp_dev(const double *xPhys, long long n, double penal, double E0, do
 namespace {
 // Scratch of the OC update, grown on demand and kept for later calls.
 struct OcScratch {
-    double *ocp = nullptr, *partial = nullptr, *lmid_dev = nullptr;
-    unsigned *ticket = nullptr;
-    void *state = nullptr;
+    double *ocp = nullptr, *partial = nullptr;
+    void *sync = nullptr, *state = nullptr;
     long long cap = 0;
     int reserve(long long n)
     {
         if (!partial) {
-            GPUTO_CUDA(cudaMalloc(&partial, sizeof(double) * 2048));
-            GPUTO_CUDA(cudaMalloc(&ticket, 16));
-            GPUTO_CUDA(cudaMemset(ticket, 0, 16));
+            GPUTO_CUDA(cudaMalloc(&sync, gputo::kLoopSyncBytes));
+            GPUTO_CUDA(cudaMemset(sync, 0, gputo::kLoopSyncBytes));
             GPUTO_CUDA(cudaMalloc(&state, 64));
+            GPUTO_CUDA(cudaMalloc(&partial, sizeof(double) * gputo::kLoopPartials));
         }
         if (n > cap) {
             cudaFree(ocp);
@@ -978,13 +977,21 @@ int gputo_oc_update_dev(const double *x, const double *dc, const double *dV0, lo
     st = g_oc.reserve(n);
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
-    gputo::launch_oc_update(n, x, dc, dV0, volfrac, move, g_oc.ocp, xnew, g_oc.partial,
-                            g_oc.ticket, g_oc.state, 64, s);
-    double hst[3] = {0, 0, 0};
-    GPUTO_CUDA(cudaMemcpyAsync(hst, g_oc.state, sizeof(hst), cudaMemcpyDeviceToHost, s));
+    st = gputo::launch_oc_update(n, x, dc, dV0, volfrac, move, g_oc.ocp, xnew, g_oc.partial, g_oc.sync, g_oc.state, 64,
+                                 s);
+    if (st) return st;
+    struct {
+        double l1, l2, lmid;
+        int steps, done;
+    } hst{};
+    GPUTO_CUDA(cudaMemcpyAsync(&hst, g_oc.state, sizeof(hst), cudaMemcpyDeviceToHost, s));
     GPUTO_CUDA(cudaStreamSynchronize(s));
     GPUTO_CUDA(cudaGetLastError());
-    if (lmid) *lmid = hst[2];
+    if (hst.done == 2) {
+        gputo::set_error("OC update: a grid barrier gave up");
+        return GPUTO_ERR_TIMEOUT;
+    }
+    if (lmid) *lmid = hst.lmid;
     return GPUTO_OK;
 }
 
@@ -999,8 +1006,9 @@ int gputo_heaviside_dev(const double *xTilde, long long n, double volfrac, doubl
     st = g_oc.reserve(n);
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
-    gputo::launch_heaviside(n, xTilde, volfrac, beta, *eta, xPhys, dprj, g_oc.partial, g_oc.ticket, g_oc.state,
-                            kHeavisideSteps, s);
+    st = gputo::launch_heaviside(n, xTilde, volfrac, beta, *eta, xPhys, dprj, g_oc.ocp, g_oc.partial, g_oc.sync,
+                                 g_oc.state, kHeavisideSteps, s);
+    if (st) return st;
     struct {
         double eta;
         int steps, done;
@@ -1008,6 +1016,10 @@ int gputo_heaviside_dev(const double *xTilde, long long n, double volfrac, doubl
     GPUTO_CUDA(cudaMemcpyAsync(&hst, g_oc.state, sizeof(hst), cudaMemcpyDeviceToHost, s));
     GPUTO_CUDA(cudaStreamSynchronize(s));
     GPUTO_CUDA(cudaGetLastError());
+    if (hst.done == 2) {
+        gputo::set_error("Heaviside threshold: a grid barrier gave up");
+        return GPUTO_ERR_TIMEOUT;
+    }
     *eta = hst.eta;
     if (!hst.done) {
         gputo::set_error("Heaviside threshold: the eta Newton iteration did not reach |f| <= 1e-6");

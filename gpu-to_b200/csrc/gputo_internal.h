@@ -337,12 +337,17 @@ void launch_simp(long long n, const double *x, double penal, double E0, double E
                  double *dsK, cudaStream_t st);
 int oc_state_bytes();
 int proj_state_bytes();
-void launch_heaviside(long long n, const double *xt, double volfrac, double beta, double eta0, double *xphys,
-                      double *dprj, double *partial, unsigned *ticket, void *state, int max_steps, cudaStream_t st);
+// The projection and the OC update: one cooperative launch each.  ex / ocp: n
+// doubles of scratch; partial: kLoopPartials doubles; sync: kLoopSyncBytes zeroed once.
+constexpr long long kLoopMaxBlocks = 512;
+constexpr int kLoopPartials = 2 * 7 * (int)kLoopMaxBlocks, kLoopSyncBytes = 16;
+int launch_heaviside(long long n, const double *xt, double volfrac, double beta, double eta0, double *xphys,
+                     double *dprj, double *ex, double *partial, void *sync, void *state, int max_steps,
+                     cudaStream_t st);
 void launch_mul(long long n, const double *a, const double *b, double *out, cudaStream_t st);
-void launch_oc_update(long long n, const double *x, const double *dc, const double *dv0,
-                      double volfrac, double move, double *ocp, double *xnew, double *partial,
-                      unsigned *ticket, void *state, int max_steps, cudaStream_t st);
+int launch_oc_update(long long n, const double *x, const double *dc, const double *dv0, double volfrac, double move,
+                     double *ocp, double *xnew, double *partial, void *sync, void *state, int max_steps,
+                     cudaStream_t st);
 
 // Counter of kernel launches issued by this library (per process).
 void count_launches(long long n);

@@ -33,6 +33,53 @@ def test_heaviside_matches_oracle_newton(oracle, gputo, torch):
     np.testing.assert_allclose(Z.cpu().numpy(), P.cpu().numpy() * D.cpu().numpy(), rtol=0, atol=0)
 
 
+@pytest.mark.parametrize("n", [5, 4097, 300001])
+@pytest.mark.parametrize("beta", [0.5, 64.0, 400.0])
+def test_projection_loop_sizes_and_betas(oracle, gputo, torch, n, beta):
+    """Fewer elements than a CTA, a partial last pass, more than one pass; beta
+    on the exponential and (above 300, and where it overflows) the direct
+    formulas.  The sums differ from numpy's by rounding (1e-16 n^(1/2) at
+    most), which the Newton steps carry into eta: 1e-12."""
+    xt = np.random.default_rng(n).random(n)
+    xt[:2] = 0.0, 1.0
+    volfrac, eta0 = 0.4, 0.55
+    eta = eta0
+    for _ in range(60):
+        f = oracle.prj(xt, eta, beta).mean() - volfrac
+        if abs(f) <= 1e-6:
+            break
+        eta = eta - f / oracle.deta(xt, eta, beta).mean()
+    converged = abs(f) <= 1e-6
+    X = torch.as_tensor(xt, dtype=torch.float64, device="cuda")
+    P = torch.empty_like(X)
+    if not converged:   # no threshold gives this volume: the steps run into NaNs or the call says it did not converge
+        try:
+            gputo.heaviside_dev(X, P, volfrac, beta, eta0)
+            assert torch.isnan(P).any()
+        except gputo.GputoError as e:
+            assert e.status == gputo.GPUTO_ERR_BREAKDOWN
+        return
+    eta_g = gputo.heaviside_dev(X, P, volfrac, beta, eta0)
+    assert abs(eta_g - eta) <= 1e-12 * abs(eta)
+    np.testing.assert_allclose(P.cpu().numpy(), oracle.prj(xt, eta, beta), rtol=0, atol=1e-12 * max(1.0, beta))
+
+
+@pytest.mark.parametrize("n", [1, 700, 4097, 300001])
+def test_oc_loop_sizes(oracle, gputo, torch, n):
+    """The OC update on fewer elements than a CTA, a partial last pass and
+    several passes: the multiplier's path is the numpy loop's (its start differs
+    by rounding only)."""
+    rng = np.random.default_rng(n)
+    x, dc = rng.random(n), -np.exp(rng.standard_normal(n))
+    dv = np.full(n, 1.0 / n)
+    ref, lref = oracle.oc_update(x, dc, dv, 0.3, 0.2)
+    X, D, V = (torch.as_tensor(a, dtype=torch.float64, device="cuda") for a in (x, dc, dv))
+    out = torch.empty_like(X)
+    lm = gputo.oc_update_dev(X, D, V, out, 0.3, 0.2)
+    assert abs(lm - lref) <= 1e-13 * abs(lref)
+    np.testing.assert_allclose(out.cpu().numpy(), ref, rtol=0, atol=1e-13)
+
+
 def test_design_loop_with_projection_matches_oracle(oracle, gputo, torch):
     """Six iterations of the 32x16x16 cantilever with ft = 3 on the GPU against
     the oracle loop with the same settings: compliance history within 1e-6,
