@@ -38,69 +38,12 @@ constexpr int kMaxFilterRadius = 6;           // stencil up to 13^3
 constexpr int kFilterW = 2 * kMaxFilterRadius + 1;
 __constant__ double cFilterH[kFilterW * kFilterW * kFilterW];
 
-// ce_e = u_e^T Ke u_e, dc_e = dsK_e ce_e, and sum_e CX_e ce_e.  Thread per
-// element.  U is in the solver frame: the driver's U(cMat) gather
-// (top3D125modCuda.m:39-41,139) lists element nodes in an order mirrored in y,
-// which matches the y-negated U the MEX hands back, so both give the same ce.
-// HAD: u_e' Ke u_e as (T u_e)' (S / 64) (T u_e) in the element's Hadamard
-// basis (about 140 FP64 operations, so the pass is bound by memory); else
-// the dense 24x24 product with Ke from constant memory (1152 FLOP).
-template <bool HAD>
-__global__ void __launch_bounds__(256)
-element_energy_kernel(Grid g, HC<double> hc, const double *__restrict__ U, const double *__restrict__ CX,
-                      const double *__restrict__ dsK, double *__restrict__ ce,
-                      double *__restrict__ dc, double *__restrict__ partial, unsigned *ticket,
-                      double *compliance)
+// The CTAs' compliance partials, summed by the last CTA to finish with all its
+// threads, in a fixed order.
+__device__ __forceinline__ void sum_compliance(double csum, double *partial, unsigned *ticket, double *compliance)
 {
     __shared__ double red[8];
     __shared__ bool is_last;
-    const long long nel = g.nel();
-    double csum = 0.0;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nel;
-         e += (long long)gridDim.x * blockDim.x) {
-        const long long t = e / g.ny;
-        const int j = (int)(e - t * g.ny);
-        const int i = (int)(t / g.nz);
-        const int k = (int)(t - (long long)i * g.nz);
-        double s = 0.0;
-        if constexpr (HAD) {
-            // corners (cx, cy, cz) into the two x faces, [(2 cy + cz) 4 + d]
-            double Fp[HF], Fn[HF];
-#pragma unroll
-            for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-                for (int cz = 0; cz < 2; ++cz) {
-                    const long long n0 = g.node(i, j + cy, k + cz), n1 = g.node(i + 1, j + cy, k + cz);
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        Fp[(2 * cy + cz) * 4 + d] = U[3 * n0 + d];
-                        Fn[(2 * cy + cz) * 4 + d] = U[3 * n1 + d];
-                    }
-                }
-            face_h(Fp);
-            face_h(Fn);
-            s = element_energy_h(Fp, Fn, hc);
-        } else {
-            double ue[24];
-#pragma unroll
-            for (int a = 0; a < 8; ++a) {
-                const long long n = g.node(i + local_x(a), j + local_y(a), k + local_z(a));
-#pragma unroll
-                for (int d = 0; d < 3; ++d) ue[3 * a + d] = U[3 * n + d];
-            }
-#pragma unroll 4
-            for (int m = 0; m < 24; ++m) {
-                double tm = 0.0;
-#pragma unroll
-                for (int q = 0; q < 24; ++q) tm = fma(cKeD[m * 24 + q], ue[q], tm);
-                s = fma(ue[m], tm, s);
-            }
-        }
-        if (ce) ce[e] = s;
-        if (dc) dc[e] = dsK[e] * s;
-        if (CX) csum = fma(CX[e], s, csum);
-    }
-    if (!compliance) return;
     for (int o = 16; o > 0; o >>= 1) csum += __shfl_xor_sync(0xffffffffu, csum, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = csum;
     __syncthreads();
@@ -112,16 +55,197 @@ element_energy_kernel(Grid g, HC<double> hc, const double *__restrict__ U, const
         is_last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
     }
     __syncthreads();
-    if (is_last && threadIdx.x == 0) {
-        __threadfence();
-        double v = 0.0;
-        for (unsigned b = 0; b < gridDim.x; ++b) v += partial[b];
+    if (!is_last) return;
+    __threadfence();
+    double v = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) v += __ldcg(partial + b);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        v = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[w];
         *compliance = v;
         *ticket = 0;
     }
 }
 
-// Same kernel with an explicit number of CTAs (one partial slot per CTA).
+// ce_e = u_e^T Ke u_e, dc_e = dsK_e ce_e, and sum_e CX_e ce_e, dense 24x24
+// product with Ke from constant memory (1152 FLOP), thread per element: any Ke
+// without the cube element's Hadamard pattern.  U is in the solver frame: the
+// driver's U(cMat) gather (top3D125modCuda.m:39-41,139) lists element nodes in
+// an order mirrored in y, which matches the y-negated U the MEX hands back, so
+// both give the same ce.
+__global__ void __launch_bounds__(256)
+element_energy_kernel(Grid g, const double *__restrict__ U, const double *__restrict__ CX,
+                      const double *__restrict__ dsK, double *__restrict__ ce,
+                      double *__restrict__ dc, double *__restrict__ partial, unsigned *ticket,
+                      double *compliance)
+{
+    const long long nel = g.nel();
+    double csum = 0.0;
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nel;
+         e += (long long)gridDim.x * blockDim.x) {
+        const long long t = e / g.ny;
+        const int j = (int)(e - t * g.ny);
+        const int i = (int)(t / g.nz);
+        const int k = (int)(t - (long long)i * g.nz);
+        double s = 0.0, ue[24];
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            const long long n = g.node(i + local_x(a), j + local_y(a), k + local_z(a));
+#pragma unroll
+            for (int d = 0; d < 3; ++d) ue[3 * a + d] = U[3 * n + d];
+        }
+#pragma unroll 4
+        for (int m = 0; m < 24; ++m) {
+            double tm = 0.0;
+#pragma unroll
+            for (int q = 0; q < 24; ++q) tm = fma(cKeD[m * 24 + q], ue[q], tm);
+            s = fma(ue[m], tm, s);
+        }
+        if (ce) ce[e] = s;
+        if (dc) dc[e] = dsK[e] * s;
+        if (CX) csum = fma(CX[e], s, csum);
+    }
+    if (compliance) sum_compliance(csum, partial, ticket, compliance);
+}
+
+__device__ __forceinline__ void cp_async8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// The same for the cube element's Ke, as (T u_e)' (S / 64) (T u_e) in the
+// element's Hadamard basis.  A CTA takes 32 (y) x 4 (z) element columns and
+// marches along x: node planes come by cp.async (8 bytes: rows start anywhere)
+// into a ring of four, two ahead of the one in use, and each face is
+// transformed once for the two elements that share it (about 116 FP64
+// operations per element).  Work items are (tile, x chunk) pairs, so any grid
+// runs on as many CTAs as there are partial slots.  57 bytes and 116 FP64
+// operations per element bound it (36 and 27 us at 256 x 128 x 128); it is
+// held by latency at the 16 warps per SM its registers allow.  Per call at 256
+// x 128 x 128 78 us, on 193 x 97 x 95 (a last y tile of one column) 67 us, on
+// 114 x 82 x 50 31 us; 148, 92 and 62 us with a thread per element gathering
+// its 24 corner values and a one-thread sum of the CTAs' partials.  Tiles of 8
+// rows took 82, 67 and 33 us.
+constexpr int kEnY = 32, kEnZ = 4, kEnT = 32 * kEnZ, kEnRing = 4;
+constexpr int kEnRow = 3 * (kEnY + 1), kEnPlane = kEnRow * (kEnZ + 1), kEnPos = (kEnPlane + kEnT - 1) / kEnT;
+
+__global__ void __launch_bounds__(kEnT, 512 / kEnT)
+element_energy_march_kernel(Grid g, HC<double> hc, int xc, int ntj, int ntk, long long nitems,
+                            const double *__restrict__ U, const double *__restrict__ CX,
+                            const double *__restrict__ dsK, double *__restrict__ ce, double *__restrict__ dc,
+                            double *__restrict__ partial, unsigned *ticket, double *compliance)
+{
+    __shared__ double ring[kEnRing][kEnPlane];
+    const int tid = threadIdx.x, l = tid & 31, w = tid >> 5;
+    const long long ps = 3LL * (g.ny + 1) * (g.nz + 1);   // values per node plane
+    double csum = 0.0;
+    for (long long item = blockIdx.x; item < nitems; item += gridDim.x) {
+        const long long tile = item % ((long long)ntj * ntk);
+        const int i0 = (int)(item / ((long long)ntj * ntk)) * xc, i1 = min(i0 + xc, g.nx);
+        const int j0 = (int)(tile % ntj) * kEnY, k0 = (int)(tile / ntj) * kEnZ;
+        const int np = i1 - i0 + 1;
+        long long off[kEnPos];   // this thread's values of a plane tile, clamped to the grid
+#pragma unroll
+        for (int q = 0; q < kEnPos; ++q) {
+            const int p = tid + kEnT * q, kk = p / kEnRow, c = p - kk * kEnRow;
+            const int v = min(3 * j0 + c, 3 * g.ny + 2);
+            off[q] = (long long)min(k0 + kk, g.nz) * (3 * (g.ny + 1)) + v;
+        }
+        auto fetch = [&](int t) {
+            if (t < np) {
+                const double *src = U + (i0 + t) * ps;
+                double *dst = ring[t % kEnRing];
+#pragma unroll
+                for (int q = 0; q < kEnPos; ++q)
+                    if (tid + kEnT * q < kEnPlane) cp_async8(dst + tid + kEnT * q, src + off[q]);
+            }
+            cp_async_commit();
+        };
+        const int j = j0 + l, k = k0 + w;
+        const bool mine = j < g.ny && k < g.nz;
+        const long long es = (long long)g.ny * g.nz;
+        long long e = (long long)i0 * es + (long long)k * g.ny + j;   // element in front of plane t
+        __syncthreads();   // the ring is free
+#pragma unroll
+        for (int t = 0; t < kEnRing - 1; ++t) fetch(t);
+        auto face = [&](int t, double (&F)[HF]) {
+            cp_async_wait<kEnRing - 2>();
+            __syncthreads();   // plane t has landed for everyone; slot (t - 1) is free
+            fetch(t + kEnRing - 1);
+            const double *P = ring[t % kEnRing] + w * kEnRow + 3 * l;
+#pragma unroll
+            for (int cy = 0; cy < 2; ++cy)
+#pragma unroll
+                for (int cz = 0; cz < 2; ++cz)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) F[(2 * cy + cz) * 4 + d] = P[cz * kEnRow + 3 * cy + d];
+            face_h(F);
+        };
+        auto element = [&](const double (&Fp)[HF], const double (&Fn)[HF], double cx, double ds) {
+            if (mine) {
+                const double s = element_energy_h(Fp, Fn, hc);
+                if (ce) ce[e] = s;
+                if (dc) dc[e] = ds * s;
+                csum = fma(cx, s, csum);
+            }
+            e += es;
+        };
+        double Fa[HF], Fb[HF];
+        // the scales of the element after the next face, a step ahead
+        double cx = mine && CX ? CX[e] : 0.0, ds = mine && dc ? dsK[e] : 0.0, cn = 0.0, dn = 0.0;
+        auto ahead = [&](int t) {
+            if (mine && t + 1 < np) {
+                if (CX) cn = CX[e + es];
+                if (dc) dn = dsK[e + es];
+            }
+        };
+        face(0, Fa);
+        for (int t = 1; t < np; t += 2) {   // two planes a trip: no face is copied
+            ahead(t);
+            face(t, Fb);
+            element(Fa, Fb, cx, ds);
+            if (t + 1 < np) {
+                cx = cn, ds = dn;
+                ahead(t + 1);
+                face(t + 1, Fa);
+                element(Fb, Fa, cx, ds);
+                cx = cn, ds = dn;
+            }
+        }
+        cp_async_wait<0>();   // the empty trailing groups
+    }
+    if (compliance) sum_compliance(csum, partial, ticket, compliance);
+}
+
+// Planes per x chunk of a marching kernel: tiles x chunks CTAs run in waves of
+// 'slots', and a CTA takes its planes and 'extra' more (halo planes, filling
+// the ring), so the chunk count with the smallest waves x (planes + extra):
+// one full wave on large grids, a plane or two per CTA where latency counts
+// (the radius-2 filter of 64 x 32 x 32 elements 26.5 -> 18.5 us per call).
+static int chunk_planes(int nx, long long tiles, long long slots, int extra)
+{
+    int best = nx;
+    long long cost = -1;
+    for (int c = 1; c <= nx && c <= 512; ++c) {
+        const int xc = (nx + c - 1) / c;
+        const long long n = (nx + xc - 1) / xc, t = ((tiles * n + slots - 1) / slots) * (xc + extra);
+        if (cost < 0 || t < cost) {
+            cost = t;
+            best = xc;
+        }
+    }
+    return best;
+}
+
+// One partial slot per CTA: at most nblocks CTAs.
 void launch_element_energy_blocks(const Grid &g, const double *U, const double *CX,
                                   const double *dsK, double *ce, double *dc, double *partial,
                                   unsigned *ticket, double *compliance, int nblocks,
@@ -134,12 +258,16 @@ void launch_element_energy_blocks(const Grid &g, const double *U, const double *
         std::lock_guard<std::mutex> lock(g_design_hk_mu);
         hk = g_design_hk[dev < 64 ? dev : 63];
     }
-    if (hk.ok)
-        element_energy_kernel<true><<<(unsigned)nblocks, 256, 0, st>>>(g, make_hc<double>(hk), U, CX, dsK, ce, dc,
-                                                                       partial, ticket, compliance);
-    else
-        element_energy_kernel<false><<<(unsigned)nblocks, 256, 0, st>>>(g, HC<double>{}, U, CX, dsK, ce, dc,
-                                                                        partial, ticket, compliance);
+    if (hk.ok) {
+        const int ntj = (g.ny + kEnY - 1) / kEnY, ntk = (g.nz + kEnZ - 1) / kEnZ;
+        const long long tiles = (long long)ntj * ntk;
+        const int xc = chunk_planes(g.nx, tiles, (512 / kEnT) * 148, 5);
+        const long long items = tiles * ((g.nx + xc - 1) / xc);
+        element_energy_march_kernel<<<(unsigned)std::min<long long>(items, nblocks), kEnT, 0, st>>>(
+            g, make_hc<double>(hk), xc, ntj, ntk, items, U, CX, dsK, ce, dc, partial, ticket, compliance);
+    } else {
+        element_energy_kernel<<<(unsigned)nblocks, 256, 0, st>>>(g, U, CX, dsK, ce, dc, partial, ticket, compliance);
+    }
     count_launches(1);
 }
 
@@ -263,54 +391,57 @@ filter_kernel(Grid g, const double *__restrict__ in, const double *__restrict__ 
     }
 }
 
-// The same correlation for 1 <= R <= 3, decomposed by x plane: h[a][b][c] =
-// h[-a][b][c], so plane q contributes P_|a|(q) = sum_{c,b} h[a][b][c] in(q, j+b,
-// k+c) (R + 1 two-dimensional sums over the same (2R + 1)^2 shared-memory
-// values) to the output at plane q - a, for every a in -R..R.  A thread keeps
-// the 2R + 1 outputs still open in registers (a ring indexed at compile time:
-// the march is unrolled by 2 (2R + 1)), so each input plane sits in shared
-// memory once (two slots, one barrier per plane) and costs (2R + 1)^2 shared
-// loads per output instead of (2R + 1)^3.  Output i sums P_R(i - R), ...,
-// P_0(i), ..., P_R(i + R) in plane order.
+// The correlation for R = 2 and 3, decomposed by x plane and by distance: the
+// weight of a tap depends on its offsets' magnitudes alone, so plane q
+// contributes P_a(q) = sum over the classes (m, n), 0 <= m <= n <= R, of
+// h[a][m][n] (the sum of the plane's values at offsets (+-m, +-n) and (+-n,
+// +-m)) to the outputs at planes q - a and q + a.  A thread has ZR output rows
+// along z of one y: it reads its (ZR + 2R) x (2R + 1) window of the plane once,
+// folds each row to its R + 1 values |dy| = 0..R, and forms the class sums of
+// its rows from those.  It keeps the 2R + 1 outputs of each row that are still
+// open in registers (a ring indexed at compile time: the march is unrolled by
+// 2R + 1).  At R = 2 that is 36 FP64 operations and 10-15 shared loads per
+// output and plane, against 80 and 25 without the classes and the row reuse.
+// Output i sums P_R(i - R), ..., P_0(i), ..., P_R(i + R) in plane order.
 // Planes arrive by cp.async into a ring of kFPS shared-memory slots (input,
 // and the divisor when given), kFPS - 1 planes ahead of the one in use, one
-// barrier per plane (two planes ahead in registers reached 0.40 of HBM).
+// barrier per plane (a second one with a divisor, whose quotients are taken in
+// place once per plane).  At 256 x 128 x 128 per call: R = 2 with a divisor 57
+// us (84 us with all 25 taps read and multiplied), without 42 us (73), R = 3 90
+// and 69 us (177 and 165); at 64 x 32 x 32 18.5 and 22 us (27 and 52).
 constexpr int kFPS = 4;
 
-__device__ __forceinline__ void cp_async8(void *dst, const void *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+template <int R, int ZR> struct FiltClass {
+    static constexpr int TYH = kFTY + 2 * R, TZH = 8 * ZR + 2 * R;
+    static constexpr int PLANE = TYH * TZH;
+    static constexpr int NPOS = (PLANE + 255) / 256;
+    static constexpr size_t bytes(bool div) { return sizeof(double) * (div ? 2 : 1) * kFPS * PLANE; }
+};
 
-template <int R>
-__global__ void __launch_bounds__(256)
-filter_plane_kernel(Grid g, const double *__restrict__ in, const double *__restrict__ div,
+template <int R, int ZR, bool DIV>
+__global__ void __launch_bounds__(256, 2)
+filter_class_kernel(Grid g, const double *__restrict__ in, const double *__restrict__ div,
                     double *__restrict__ out, double scale, int xc)
 {
-    using FT = FiltTile<R>;
-    constexpr int W = FT::W;
-    extern __shared__ double fs[];   // [kFPS][PLANE] input planes, then (with a divisor) [kFPS][PLANE] divisor planes
+    using FT = FiltClass<R, ZR>;
+    constexpr int W = 2 * R + 1;
+    extern __shared__ double fs[];   // [kFPS][PLANE] input planes, then (DIV) [kFPS][PLANE] divisor planes
     double *fd = fs + kFPS * FT::PLANE;
-    const int tid = threadIdx.x, ly = tid & 31, lz = tid >> 5;
-    const int j0 = blockIdx.x * kFTY, k0 = blockIdx.y * kFTZ;
+    const int tid = threadIdx.x, ly = tid & 31, lg = tid >> 5;
+    const int j0 = blockIdx.x * kFTY, k0 = blockIdx.y * (8 * ZR);
     const int x0 = blockIdx.z * xc, x1 = min(x0 + xc, g.nx);
     const long long ps = (long long)g.ny * g.nz;
-    long long off[FT::NPOS];
+    int off[FT::NPOS];   // offsets in an x plane (the launcher keeps planes of 2^31 elements away)
 #pragma unroll
     for (int q = 0; q < FT::NPOS; ++q) {
         const int p = tid + 256 * q;
         off[q] = -1;
         if (p < FT::PLANE) {
             const int zz = p / FT::TYH, yy = p - zz * FT::TYH;
-            off[q] = (long long)mirror_index(k0 + zz - R, g.nz) * g.ny + mirror_index(j0 + yy - R, g.ny);
+            off[q] = mirror_index(k0 + zz - R, g.nz) * g.ny + mirror_index(j0 + yy - R, g.ny);
         }
     }
     const int T = x1 - x0 + 2 * R;   // planes x0 - R .. x1 + R - 1
-    // plane t (t < T) into slot t mod kFPS; one commit group per plane, empty past the end
     auto fetch = [&](int t) {
         if (t < T) {
             const long long base = (long long)mirror_index(x0 - R + t, g.nx) * ps;
@@ -319,22 +450,23 @@ filter_plane_kernel(Grid g, const double *__restrict__ in, const double *__restr
             for (int q = 0; q < FT::NPOS; ++q)
                 if (off[q] >= 0) {
                     cp_async8(fs + sl + tid + 256 * q, in + base + off[q]);
-                    if (div) cp_async8(fd + sl + tid + 256 * q, div + base + off[q]);
+                    if (DIV) cp_async8(fd + sl + tid + 256 * q, div + base + off[q]);
                 }
         }
         cp_async_commit();
     };
-    const int j = j0 + ly, k = k0 + lz;
-    const bool mine = j < g.ny && k < g.nz;
-    const long long obase = (long long)k * g.ny + j;
-    double acc[W];
+    const int j = j0 + ly, kr = k0 + ZR * lg;   // output column; first of the thread's rows
+    const bool jok = j < g.ny;
+    double acc[W][ZR];
 #pragma unroll
-    for (int s = 0; s < W; ++s) acc[s] = 0.0;
+    for (int s = 0; s < W; ++s)
+#pragma unroll
+        for (int r = 0; r < ZR; ++r) acc[s][r] = 0.0;
 #pragma unroll
     for (int t = 0; t < kFPS - 1; ++t) fetch(t);
-    for (int t0 = 0; t0 < T; t0 += 2 * W)
+    for (int t0 = 0; t0 < T; t0 += W)
 #pragma unroll
-    for (int u = 0; u < 2 * W; ++u) {
+    for (int u = 0; u < W; ++u) {
         const int t = t0 + u;
         if (t >= T) break;                 // the same for the whole CTA
         const int q = x0 - R + t;          // this plane
@@ -342,50 +474,49 @@ filter_plane_kernel(Grid g, const double *__restrict__ in, const double *__restr
         __syncthreads();                   // everyone's have; slot (t - 1) mod kFPS is free
         fetch(t + kFPS - 1);
         double *P = fs + (t % kFPS) * FT::PLANE;
-        if (div) {   // in / divisor, in place, once per plane
+        if (DIV) {
             const double *D = fd + (t % kFPS) * FT::PLANE;
 #pragma unroll
             for (int v = 0; v < FT::NPOS; ++v)
                 if (off[v] >= 0) P[tid + 256 * v] = P[tid + 256 * v] / D[tid + 256 * v];
             __syncthreads();
         }
-        auto val = [&](int zz, int yy) { return P[zz * FT::TYH + yy]; };
-        double pa[R + 1];
-        if constexpr (R == 1) {
-            // radius 1: the weight of a tap depends only on how many of its
-            // offsets are non-zero (centre, face, edge, corner), so each plane
-            // needs the centre, the sum of its 4 edge neighbours and the sum
-            // of its 4 corners
-            const int zc = lz + 1, yc = ly + 1;
-            const double s0 = val(zc, yc);
-            const double s1 = (val(zc, yc - 1) + val(zc, yc + 1)) + (val(zc - 1, yc) + val(zc + 1, yc));
-            const double s2 = (val(zc - 1, yc - 1) + val(zc - 1, yc + 1)) + (val(zc + 1, yc - 1) + val(zc + 1, yc + 1));
-            const double w0 = cFilterH[13], w1 = cFilterH[12], w2 = cFilterH[9], w3 = cFilterH[0];
-            pa[0] = fma(w2, s2, fma(w1, s1, w0 * s0));
-            pa[1] = fma(w3, s2, fma(w2, s1, w1 * s0));
-        } else {
+        // row folds: e[row][m] = sum of the values at |dy| = m
+        double e[ZR + 2 * R][R + 1];
+#pragma unroll
+        for (int z = 0; z < ZR + 2 * R; ++z) {
+            const double *row = P + (ZR * lg + z) * FT::TYH + ly + R;
+            e[z][0] = row[0];
+#pragma unroll
+            for (int m = 1; m <= R; ++m) e[z][m] = row[-m] + row[m];
+        }
+#pragma unroll
+        for (int r = 0; r < ZR; ++r) {
+            double pa[R + 1];
 #pragma unroll
             for (int a = 0; a <= R; ++a) pa[a] = 0.0;
 #pragma unroll
-            for (int c = -R; c <= R; ++c)
+            for (int m = 0; m <= R; ++m)
 #pragma unroll
-                for (int b = -R; b <= R; ++b) {
-                    const double x = val(lz + R + c, ly + R + b);
+                for (int n = m; n <= R; ++n) {
+                    // rows +-m with |dy| = n and, for m < n, rows +-n with |dy| = m
+                    double c = m ? e[r + R - m][n] + e[r + R + m][n] : e[r + R][n];
+                    if (m < n) c += e[r + R - n][m] + e[r + R + n][m];
 #pragma unroll
-                    for (int a = 0; a <= R; ++a)
-                        pa[a] = fma(cFilterH[((a + R) * W + (b + R)) * W + (c + R)], x, pa[a]);
+                    for (int a = 0; a <= R; ++a) pa[a] = fma(cFilterH[((a + R) * W + (m + R)) * W + (n + R)], c, pa[a]);
                 }
-        }
-        // output q + a (a = -R..R) sits in slot (t + a + R) mod W
+            // output q + a (a = -R..R) sits in slot (u + a + R) mod W
 #pragma unroll
-        for (int a = -R; a <= R; ++a) {
-            const int sl = (u + a + R) % W;
-            acc[sl] += pa[a < 0 ? -a : a];
+            for (int a = -R; a <= R; ++a) acc[(u + a + R) % W][r] += pa[a < 0 ? -a : a];
         }
         // output q - R is complete
-        const int i = q - R, sl = u % W;
-        if (i >= x0 && mine) out[(long long)i * ps + obase] = acc[sl] * scale;
-        acc[sl] = 0.0;
+        const int i = q - R;
+#pragma unroll
+        for (int r = 0; r < ZR; ++r) {
+            if (i >= x0 && jok && kr + r < g.nz)
+                out[(long long)i * ps + (long long)(kr + r) * g.ny + j] = acc[u][r] * scale;
+            acc[u][r] = 0.0;
+        }
     }
     cp_async_wait<0>();   // the empty trailing groups
 }
@@ -394,7 +525,7 @@ filter_plane_kernel(Grid g, const double *__restrict__ in, const double *__restr
 // outputs: a thread reads its 6 x 3 window of each plane once for its four
 // outputs, 4.5 shared loads per output instead of 9 (the 32 x 8 tiles above
 // are bound by shared-memory bandwidth in FP64).  The same ring and the same
-// arithmetic per output as filter_plane_kernel<1>.
+// plane sums as filter_class_kernel with the four weights of radius 1.
 constexpr int kF1Y = 32, kF1Z = 32;
 
 template <bool DIV>
@@ -505,7 +636,6 @@ int filter_launch(const Grid &g, const double *in, const double *div, double *ou
         GPUTO_CUDA(e);
     }
     if constexpr (R == 1) {
-        // tiles of 32 x 32 outputs; x chunks for about 592 CTAs (4 per SM, one wave), at least 6 planes each
         constexpr size_t plane = sizeof(double) * (kF1Y + 2) * (kF1Z + 2);
         const size_t smem = (div ? 2 : 1) * kFPS * plane;
         if (div) {
@@ -521,9 +651,14 @@ int filter_launch(const Grid &g, const double *in, const double *div, double *ou
         }
         const unsigned ty = (unsigned)((g.ny + kF1Y - 1) / kF1Y), tz = (unsigned)((g.nz + kF1Z - 1) / kF1Z);
         const long long tiles = (long long)ty * tz;
+        // x chunks for about 592 CTAs (4 per SM, one wave), at least 6 planes
+        // each (a chunk reads two more than it writes); where those leave SMs
+        // without a CTA the call is bound by latency, and chunks are as short as
+        // give every SM one (64 x 32 x 32: 22.9 -> 18.1 us per call)
         const long long want = std::max(1LL, (592 + tiles - 1) / tiles);
-        int xc = (int)std::max(6LL, ((long long)g.nx + want - 1) / want);
-        if (xc > g.nx) xc = g.nx;
+        long long xl = std::max(6LL, ((long long)g.nx + want - 1) / want);
+        if (tiles * ((g.nx + xl - 1) / xl) < 148) xl = std::max(1LL, (g.nx * tiles + 147) / 148);
+        const int xc = (int)std::min<long long>(xl, g.nx);
         const unsigned tx = (unsigned)((g.nx + xc - 1) / xc);
         if (div)
             filter_r1_kernel<true><<<dim3(ty, tz, tx), 256, smem, st>>>(g, in, div, out, scale, xc);
@@ -539,11 +674,30 @@ int filter_launch(const Grid &g, const double *in, const double *div, double *ou
     int xc = (int)std::max(16LL, ((long long)g.nx + want - 1) / want);
     if (xc > g.nx) xc = g.nx;
     const unsigned tx = (unsigned)((g.nx + xc - 1) / xc);
-    if constexpr (R >= 1 && R <= 3)
-        filter_plane_kernel<R><<<dim3(ty, tz, tx), 256, sizeof(double) * (div ? 2 : 1) * kFPS * FT::PLANE, st>>>(
-            g, in, div, out, scale, xc);
-    else
-        filter_kernel<R><<<dim3(ty, tz, tx), 256, FT::bytes, st>>>(g, in, div, out, scale, xc);
+    filter_kernel<R><<<dim3(ty, tz, tx), 256, FT::bytes, st>>>(g, in, div, out, scale, xc);
+    count_launches(1);
+    return GPUTO_OK;
+}
+
+// R = 2 and 3: ZR output rows per thread.
+template <int R, int ZR, bool DIV>
+int filter_class_launch(const Grid &g, const double *in, const double *div, double *out, double scale, cudaStream_t st)
+{
+    using FT = FiltClass<R, ZR>;
+    static std::once_flag once[64];
+    int dev = 0;
+    GPUTO_CUDA(cudaGetDevice(&dev));
+    cudaError_t e = cudaSuccess;
+    std::call_once(once[dev < 64 ? dev : 63], [&]() {
+        e = cudaFuncSetAttribute(filter_class_kernel<R, ZR, DIV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)FT::bytes(DIV));
+    });
+    GPUTO_CUDA(e);
+    const unsigned ty = (unsigned)((g.ny + kFTY - 1) / kFTY), tz = (unsigned)((g.nz + 8 * ZR - 1) / (8 * ZR));
+    const long long tiles = (long long)ty * tz;
+    const int xc = chunk_planes(g.nx, tiles, 2 * 148, 2 * R + 3);
+    const unsigned tx = (unsigned)((g.nx + xc - 1) / xc);
+    filter_class_kernel<R, ZR, DIV><<<dim3(ty, tz, tx), 256, FT::bytes(DIV), st>>>(g, in, div, out, scale, xc);
     count_launches(1);
     return GPUTO_OK;
 }
@@ -577,11 +731,18 @@ int launch_filter(const Grid &g, const double *in, const double *div, double *ou
         have[slot] = true;
     }
     const double scale = normalize ? 1.0 / hs : 1.0;
+    const bool small_plane = (long long)g.ny * g.nz < (1LL << 31);   // the class kernels' plane offsets are 32-bit
     switch (R) {
     case 0: return filter_launch<0>(g, in, div, out, scale, st);
     case 1: return filter_launch<1>(g, in, div, out, scale, st);
-    case 2: return filter_launch<2>(g, in, div, out, scale, st);
-    case 3: return filter_launch<3>(g, in, div, out, scale, st);
+    case 2:
+        if (!small_plane) return filter_launch<2>(g, in, div, out, scale, st);
+        return div ? filter_class_launch<2, 4, true>(g, in, div, out, scale, st)
+                   : filter_class_launch<2, 4, false>(g, in, div, out, scale, st);
+    case 3:
+        if (!small_plane) return filter_launch<3>(g, in, div, out, scale, st);
+        return div ? filter_class_launch<3, 2, true>(g, in, div, out, scale, st)
+                   : filter_class_launch<3, 2, false>(g, in, div, out, scale, st);
     case 4: return filter_launch<4>(g, in, div, out, scale, st);
     case 5: return filter_launch<5>(g, in, div, out, scale, st);
     default: return filter_launch<6>(g, in, div, out, scale, st);

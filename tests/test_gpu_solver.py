@@ -205,6 +205,24 @@ def test_element_energy_both_element_paths(oracle, gputo, torch, ke):
     assert abs(c - CX @ ce_ref) <= 1e-12 * abs(CX @ ce_ref)
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 33, 5), (70, 31, 9), (40, 65, 4), (9, 2, 300)])
+def test_element_energy_tiles_and_chunks(oracle, gputo, torch, shape):
+    """The marching energy pass at the edges of its 32 x 4 column tiles and x
+    chunks: one element, a last tile of one column or row, several chunks, long
+    z.  Sums of 24 products: 1e-12 of the largest, as above."""
+    nelx, nely, nelz = shape
+    p = oracle.cantilever(nelx, nely, nelz)
+    rng = np.random.default_rng(7)
+    U = rng.standard_normal(p.ndof)
+    CX, dsK = oracle.simp(rng.uniform(0.05, 1.0, p.nel))
+    ce, dc = (torch.empty(p.nel, dtype=torch.float64, device="cuda") for _ in range(2))
+    c = gputo.compliance_sens_dev(p.Ke0, _dev(torch, U), _dev(torch, CX), _dev(torch, dsK), nelx, nely, nelz, ce, dc)
+    ce_ref = oracle.element_energy(p, U)
+    assert np.abs(ce.cpu().numpy() - ce_ref).max() <= 1e-12 * np.abs(ce_ref).max()
+    assert np.abs(dc.cpu().numpy() - dsK * ce_ref).max() <= 1e-12 * np.abs(dsK * ce_ref).max()
+    assert abs(c - CX @ ce_ref) <= 1e-12 * abs(CX @ ce_ref)
+
+
 @pytest.mark.parametrize("rmin", [3 ** 0.5, 2 * 3 ** 0.5, 1.2, 2.5, 4.5, 0.9])
 @pytest.mark.parametrize("shape", [(20, 12, 10), (70, 40, 19), (5, 33, 9)])
 def test_density_filter_matches_oracle(oracle, gputo, rmin, shape):
