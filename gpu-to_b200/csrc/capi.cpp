@@ -238,8 +238,7 @@ int gputo_solver_apply_dev(gputo_solver *h, const double *u, double *r, void *st
     cudaStream_t st = s.stream(stream);
     s.launch_status = GPUTO_OK;
     gputo::launch_pack(s.lay[0], u, s.P, 0, st);
-    s.apply(s.P, s.Q, nullptr, nullptr, st);
-    gputo::launch_unpack(s.lay[0], s.Q, r, 0, st);
+    s.apply_dense(s.P, r, st);
     GPUTO_CUDA(cudaStreamSynchronize(st));
     GPUTO_CUDA(cudaGetLastError());
     if (s.launch_status) return s.launch_status;

@@ -211,12 +211,14 @@ template <typename T> int hsweep_blocks(const Grid &g, int mode = MODE_APPLY, in
 // rdiag: 1/diag (launch_recip); maskp: the Dirichlet bytes with rows padded
 // to 16 bytes (launch_pad_mask; hsweep_mask_bytes of storage).
 // MODE_JACOBI_PRO: uc is the coarse correction in the layout Lc (level 1).
+// dense_out (MODE_APPLY, one element column per lane): out is a dense vector
+// (rows of 3 (ny + 1) values) instead of one in the layout L.
 template <typename T>
 int launch_hsweep(int mode, const Lay &L, const ELay &E, const HadamardKe &hk, const T *CX, const T *u, const T *f,
                   const T *rdiag, const uint8_t *mask, const uint8_t *maskp, T *out, T omega, T prerelax,
                   double *dot_partial, const int *done, int *err, cudaStream_t st, const double *Rd = nullptr,
                   const T *zo = nullptr, const T *uc = nullptr, const Lay *Lc = nullptr, int xchunk = 0,
-                  bool pairs = false);
+                  bool pairs = false, bool dense_out = false);
 template <typename T> bool hsweep_pro_fits(const Grid &g);
 // MODE_ENERGY sweep (FP64): out (optional) = f - K u with fixed rows zero,
 // ce / dc in natural element order, partial pairs (|r|^2, sum CX ce) per CTA.

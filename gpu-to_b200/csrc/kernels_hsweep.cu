@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(32 * WZ, HMinBlocks<T, MODE>::value)
 hsweep_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ CUtensorMap tm_d,
               const __grid_constant__ CUtensorMap tm_f, const __grid_constant__ CUtensorMap tm_c,
               const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_r,
-              const __grid_constant__ CUtensorMap tm_z, Lay L, HC<T> hc, int htx, const T *__restrict__ f,
+              const __grid_constant__ CUtensorMap tm_z, Lay L, long long opitch, HC<T> hc, int htx, const T *__restrict__ f,
               const T *__restrict__ rdiag, const uint8_t *__restrict__ mask, T *__restrict__ out, T omega,
               T prerelax, double *__restrict__ dot_partial, const int *__restrict__ done, int *__restrict__ err,
               const double *__restrict__ Rd, const T *__restrict__ zo, uint32_t wait_ns, int skip_stage,
@@ -296,6 +296,8 @@ hsweep_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ 
     const int nst = nE + 1 + (last_plane ? 1 : 0);   // ring stages
     const bool tail_owner = (r == CY - 1) && (jc0 + HY == g.ny);
     const bool zok = (w >= 1 || zt == 0) && kc0 + w <= g.nz;   // this warp's node row is output here
+    // where a node's output goes: rows of opitch values (the layout's, or 3 (ny + 1) for a dense result)
+    auto obase = [&](int p, int j, int k) { return ((long long)p * (g.nz + 1) + k) * opitch + 3LL * j; };
 
     if (tid == 0) {
         for (int s = 0; s < HRING; ++s) mbar_init(&bar[s], 1);
@@ -449,7 +451,7 @@ hsweep_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ 
             }
         } else if (j <= g.ny) {
             const T uu[3] = {Uu[0], Uu[1], Uu[2]};
-            h_store<T, MODE>(L.at(p, j, k), em[l], R, uu, ef + 3 * l, ed + 3 * l, out, omega, dsum, er + 3 * l,
+            h_store<T, MODE>(obase(p, j, k), em[l], R, uu, ef + 3 * l, ed + 3 * l, out, omega, dsum, er + 3 * l,
                              ez + 3 * l, dsum2);
         }
         if (l == HY - 1) {   // this CTA's part of node column jc0 + HY
@@ -470,7 +472,7 @@ hsweep_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ 
                 }
             } else if (tail_owner) {
                 const T uu[3] = {Uu[8], Uu[9], Uu[10]};
-                h_store<T, MODE>(L.at(p, g.ny, k), em[HY], Sd, uu, ef + 3 * HY, ed + 3 * HY, out, omega, dsum,
+                h_store<T, MODE>(obase(p, g.ny, k), em[HY], Sd, uu, ef + 3 * HY, ed + 3 * HY, out, omega, dsum,
                                  er + 3 * HY, ez + 3 * HY, dsum2);
             }
         }
@@ -605,8 +607,8 @@ hsweep_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ 
                 else
                     uu[d] = (MODE == MODE_APPLY || N::D) ? ug[base + d] : T(0);
             }
-            h_store<T, MODE>(base, mask[g.node(p, jc0, k)], v, uu, f + base, rdiag + base, out, omega, dsum,
-                             Rd + base, zo + base, dsum2);
+            h_store<T, MODE>(obase(p, jc0, k), mask[g.node(p, jc0, k)], v, uu, f + base, rdiag + base, out, omega,
+                             dsum, Rd + base, zo + base, dsum2);
         }
     }
     if ((MODE == MODE_APPLY || MODE == MODE_JACOBI_DOT || MODE == MODE_ENERGY) && dot_partial) {
@@ -1241,7 +1243,7 @@ int hlaunch(const Lay &L, const ELay &E, const HadamardKe &hk, const T *CX, cons
             const uint8_t *mask, const uint8_t *maskp, T *out, T omega, T prerelax, double *dot_partial,
             const int *done, int *err, cudaStream_t st, const double *Rd = nullptr, const T *zo = nullptr,
             double *ce = nullptr, double *dcv = nullptr, const double *dsK = nullptr, const T *uc = nullptr,
-            const Lay *Lc = nullptr, int xchunk = 0)
+            const Lay *Lc = nullptr, int xchunk = 0, bool dense_out = false)
 {
     constexpr int WZ = hwz<T>();
     using N = HNeeds<MODE>;
@@ -1298,7 +1300,8 @@ int hlaunch(const Lay &L, const ELay &E, const HadamardKe &hk, const T *CX, cons
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const SweepFaultHook hook = sweep_fault_hook();
-    GPUTO_CUDA(cudaLaunchKernelEx(&cfg, hsweep_kernel<T, MODE, WZ>, mu, md, mf, mc, mm, mr, mz, L, hc, htx, f, rdiag, mask,
+    GPUTO_CUDA(cudaLaunchKernelEx(&cfg, hsweep_kernel<T, MODE, WZ>, mu, md, mf, mc, mm, mr, mz, L,
+                                  dense_out ? 3LL * (g.ny + 1) : L.pitch, hc, htx, f, rdiag, mask,
                                   out, omega, prerelax, dot_partial, done, err, Rd, zo, hook.wait_ns, hook.skip_stage,
                                   ce, dcv, dsK, uc, Lc ? *Lc : L, u));
     count_launches(1);
@@ -1674,7 +1677,7 @@ template <typename T>
 int launch_hsweep(int mode, const Lay &L, const ELay &E, const HadamardKe &hk, const T *CX, const T *u, const T *f,
                   const T *rdiag, const uint8_t *mask, const uint8_t *maskp, T *out, T omega, T prerelax,
                   double *dot_partial, const int *done, int *err, cudaStream_t st, const double *Rd, const T *zo,
-                  const T *uc, const Lay *Lc, int xchunk, bool pairs)
+                  const T *uc, const Lay *Lc, int xchunk, bool pairs, bool dense_out)
 {
     if constexpr (sizeof(T) == 4) {
         if (pairs && mode != MODE_JACOBI_PRO && hsweep_pairs_fit(L.g)) {
@@ -1723,7 +1726,8 @@ int launch_hsweep(int mode, const Lay &L, const ELay &E, const HadamardKe &hk, c
         return GPUTO_ERR_ARG;
     case MODE_APPLY:
         return hlaunch<T, MODE_APPLY>(L, E, hk, CX, u, f, rdiag, mask, maskp, out, omega, prerelax, dot_partial, done,
-                                      err, st, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xchunk);
+                                      err, st, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xchunk,
+                                      dense_out);
     case MODE_DEFECT:
         return hlaunch<T, MODE_DEFECT>(L, E, hk, CX, u, f, rdiag, mask, maskp, out, omega, prerelax, nullptr, done,
                                        err, st, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xchunk);
@@ -1744,11 +1748,11 @@ template int hsweep_blocks<double>(const Grid &, int, int, bool);
 template int launch_hsweep<float>(int, const Lay &, const ELay &, const HadamardKe &, const float *, const float *,
                                   const float *, const float *, const uint8_t *, const uint8_t *, float *, float,
                                   float, double *, const int *, int *, cudaStream_t, const double *, const float *,
-                                  const float *, const Lay *, int, bool);
+                                  const float *, const Lay *, int, bool, bool);
 template int launch_hsweep<double>(int, const Lay &, const ELay &, const HadamardKe &, const double *,
                                    const double *, const double *, const double *, const uint8_t *,
                                    const uint8_t *, double *, double, double, double *, const int *, int *,
                                    cudaStream_t, const double *, const double *, const double *, const Lay *, int,
-                                   bool);
+                                   bool, bool);
 
 }  // namespace gputo

@@ -582,36 +582,45 @@ void launch_diag_packed(const Lay &L, const T *Apk, T *diag, cudaStream_t st)
 template void launch_diag_packed<double>(const Lay &, const double *, double *, cudaStream_t);
 template void launch_diag_packed<float>(const Lay &, const float *, float *, cudaStream_t);
 
-// dense reference layout <-> padded layout (y optionally negated)
-__global__ void pack_kernel(Lay L, double *__restrict__ dense, double *__restrict__ padded,
-                            int flip_y, int to_padded)
+// dense reference layout <-> padded layout (y optionally negated): a warp per
+// node row, eight entries in flight per lane.  Bound by HBM: 247 us for 1.63 GB
+// at 512 x 256 x 256 (one thread per value with a 64-bit division for its row
+// took 415 us).
+template <bool TO_PADDED>
+__global__ void __launch_bounds__(256)
+pack_kernel(Lay L, const double *__restrict__ src, double *__restrict__ dst, int flip_y)
 {
     const Grid &g = L.g;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.ndof()) return;
-    const long long n = t / 3;
-    const int d = (int)(t - 3 * n);
-    const long long row = n / (g.ny + 1);
-    const int j = (int)(n - row * (g.ny + 1));
-    const long long p = row * L.pitch + 3LL * j + d;
-    const double s = (flip_y && d == 1) ? -1.0 : 1.0;
-    if (to_padded) padded[p] = s * dense[t];
-    else dense[t] = s * padded[p];
+    const long long rows = (long long)(g.nx + 1) * (g.nz + 1);
+    const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const int n = 3 * (g.ny + 1), lane = threadIdx.x & 31;
+    const long long dense = row * n, padded = row * L.pitch;
+    const double *s = src + (TO_PADDED ? dense : padded);
+    double *d = dst + (TO_PADDED ? padded : dense);
+    for (int q0 = lane; q0 < n; q0 += 256) {
+        double v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = q0 + 32 * e < n ? s[q0 + 32 * e] : 0.0;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int q = q0 + 32 * e;
+            if (q < n) d[q] = flip_y && q % 3 == 1 ? -v[e] : v[e];
+        }
+    }
 }
 
 void launch_pack(const Lay &L, const double *dense, double *padded, int flip_y, cudaStream_t st)
 {
-    const int bs = 256;
-    pack_kernel<<<(unsigned)((L.g.ndof() + bs - 1) / bs), bs, 0, st>>>(L, const_cast<double *>(dense), padded,
-                                                                        flip_y, 1);
+    const long long rows = (long long)(L.g.nx + 1) * (L.g.nz + 1);
+    pack_kernel<true><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(L, dense, padded, flip_y);
     count_launches(1);
 }
 
 void launch_unpack(const Lay &L, const double *padded, double *dense, int flip_y, cudaStream_t st)
 {
-    const int bs = 256;
-    pack_kernel<<<(unsigned)((L.g.ndof() + bs - 1) / bs), bs, 0, st>>>(L, dense, const_cast<double *>(padded),
-                                                                        flip_y, 0);
+    const long long rows = (long long)(L.g.nx + 1) * (L.g.nz + 1);
+    pack_kernel<false><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(L, padded, dense, flip_y);
     count_launches(1);
 }
 
@@ -841,38 +850,52 @@ void launch_coarsest_penalty(const Grid &g, const uint8_t *mask, double *Apk, cu
     count_launches(1);
 }
 
-// Dense coarsest matrix, one thread per row (mgcg1.cu:1747-1806 assembAc).
-__global__ void assemble_dense_kernel(Grid g, const double *__restrict__ A, double *__restrict__ AQ)
+// Dense coarsest matrix (mgcg1.cu:1747-1806 assembAc), a warp per row: the
+// lanes clear the row, then lane l < 27 sums the row's three entries at
+// neighbour node l over the elements the two nodes share.  (A thread per row
+// that cleared and updated it in global memory took 82 us for 675 rows, one
+// dependent read and write after the other; 7 us now.)
+__global__ void __launch_bounds__(256)
+assemble_dense_kernel(Grid g, const double *__restrict__ A, double *__restrict__ AQ)
 {
-    const long long row = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long N = g.ndof();
+    const int N = (int)g.ndof();
+    const int row = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (row >= N) return;
-    const long long n = row / 3;
-    const int d = (int)(row - 3 * n);
+    const int n = row / 3, d = row - 3 * n;
     int i, j, k;
     node_ijk(g, n, i, j, k);
     const long long nel = g.nel();
-    double *out = AQ + row * N;
-    for (long long c = 0; c < N; ++c) out[c] = 0.0;
+    double *out = AQ + (long long)row * N;
+    for (int c = lane; c < N; c += 32) out[c] = 0.0;
+    __syncwarp();
+    if (lane >= 27) return;
+    const int dx = lane / 9 - 1, dz = lane / 3 % 3 - 1, dy = lane % 3 - 1;
+    if (i + dx < 0 || i + dx > g.nx || j + dy < 0 || j + dy > g.ny || k + dz < 0 || k + dz > g.nz) return;
+    double s[3] = {0.0, 0.0, 0.0};
+#pragma unroll
     for (int ex = 0; ex < 2; ++ex)
+#pragma unroll
         for (int ez = 0; ez < 2; ++ez)
+#pragma unroll
             for (int ey = 0; ey < 2; ++ey) {
                 const int ei = i - 1 + ex, ej = j - 1 + ey, ek = k - 1 + ez;
-                if (ei < 0 || ei >= g.nx || ej < 0 || ej >= g.ny || ek < 0 || ek >= g.nz) continue;
+                const int bx = dx + 1 - ex, by = dy + 1 - ey, bz = dz + 1 - ez;   // the neighbour's corner
+                if (ei < 0 || ei >= g.nx || ej < 0 || ej >= g.ny || ek < 0 || ek >= g.nz || bx < 0 || bx > 1 || by < 0 ||
+                    by > 1 || bz < 0 || bz > 1)
+                    continue;
                 const long long e = g.elem(ei, ej, ek);
-                const int a = local_index(1 - ex, 1 - ey, 1 - ez);
-                for (int b = 0; b < 8; ++b) {
-                    const long long nb = g.node(ei + local_x(b), ej + local_y(b), ek + local_z(b));
-                    for (int q = 0; q < 3; ++q)
-                        out[3 * nb + q] += A[(long long)packed_index(3 * a + d, 3 * b + q) * nel + e];
-                }
+                const int a = local_index(1 - ex, 1 - ey, 1 - ez), b = local_index(bx, by, bz);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) s[q] += A[(long long)packed_index(3 * a + d, 3 * b + q) * nel + e];
             }
+    const long long nb = g.node(i + dx, j + dy, k + dz);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) out[3 * nb + q] = s[q];
 }
 
 void launch_assemble_dense(const Grid &g, const double *Apk, double *AQ, cudaStream_t st)
 {
-    const int bs = 64;
-    assemble_dense_kernel<<<(unsigned)((g.ndof() + bs - 1) / bs), bs, 0, st>>>(g, Apk, AQ);
+    assemble_dense_kernel<<<(unsigned)((g.ndof() * 32 + 255) / 256), 256, 0, st>>>(g, Apk, AQ);
     count_launches(1);
 }
 

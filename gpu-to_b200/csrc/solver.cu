@@ -547,6 +547,21 @@ void Solver::apply(const double *u, double *r, double *dot_partial, const int *d
     note(fine_sweep<double>(0, MODE_APPLY, lay[0], elay, CXp, u, nullptr, L[0], r, 1.0, 0.0, dot_partial, done, st));
 }
 
+// The sweep's stores are plain ones, so writing rows without padding costs it
+// nothing and saves the pass that took them from Q (an eighth of the call at
+// 512 x 256 x 256).
+void Solver::apply_dense(const double *u, double *r, cudaStream_t st)
+{
+    if (use_hsweep<double>(g[0]) && L[0].rdiag) {
+        note(launch_hsweep<double>(MODE_APPLY, lay[0], elay, hk, CXp, u, nullptr, L[0].rdiag, mask[0], maskp[0], r, 1.0,
+                                   0.0, nullptr, nullptr, err, st, nullptr, nullptr, nullptr, nullptr,
+                                   opt.sweep_xchunk, false, true));
+        return;
+    }
+    apply(u, Q, nullptr, nullptr, st);
+    launch_unpack(lay[0], Q, r, 0, st);
+}
+
 // One PCG iteration (mgcg1.cu:254-275), every scalar on the device.
 void Solver::iteration(cudaStream_t st)
 {

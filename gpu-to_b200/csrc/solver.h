@@ -102,6 +102,8 @@ struct Solver {
     // Padded-layout preconditioner and operator.
     void vcycle(const double *r, double *z, const int *done, cudaStream_t st);
     void apply(const double *u, double *r, double *dot_partial, const int *done, cudaStream_t st);
+    // K u into a dense vector: the Hadamard-basis sweep writes it itself, else through Q
+    void apply_dense(const double *u, double *r, cudaStream_t st);
     cudaStream_t stream(void *s) const { return s ? (cudaStream_t)s : own_stream; }
     // Fine-operator sweep on a grid with K = sum CX_e Ke: the Hadamard-basis
     // kernel when it applies, else the dense element rows.
