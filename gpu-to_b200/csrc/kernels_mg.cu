@@ -854,7 +854,7 @@ void launch_coarsest_penalty(const Grid &g, const uint8_t *mask, double *Apk, cu
 // lanes clear the row, then lane l < 27 sums the row's three entries at
 // neighbour node l over the elements the two nodes share.  (A thread per row
 // that cleared and updated it in global memory took 82 us for 675 rows, one
-// dependent read and write after the other; 7 us now.)
+// dependent read and write after the other; 8 us now.)
 __global__ void __launch_bounds__(256)
 assemble_dense_kernel(Grid g, const double *__restrict__ A, double *__restrict__ AQ)
 {
@@ -949,86 +949,157 @@ void launch_dense_fix(const Grid &g, const uint8_t *mask, double *AQ, cudaStream
 // place in the lower triangle, 32-column panels (textbook algorithm; the
 // reference factors row by row, one kernel launch per row,
 // mgcg1.cu:2099-2142).  For each panel [c0, c0 + w):
-//   chol_diag_kernel   the w x w diagonal block, factored in shared memory
-//                      (one CTA, a thread per entry);
-//   chol_panel_kernel  each row r below it solves L[r][panel] D^T = A[r][panel]
-//                      (a thread per row, many CTAs);
+//   chol_panel_kernel  every CTA factors the w x w diagonal block for itself in
+//                      one warp, and each of its warps then solves
+//                      L[r][panel] D^T = A[r][panel] for a row r below;
 //   chol_trail_kernel  the trailing lower triangle loses the panel's rank-w
 //                      product, A[r][c] -= sum_k L[r][c0 + k] L[c][c0 + k]
 //                      (a CTA per 32 x 32 tile on or below the diagonal).
-// Each step is a short latency-bound kernel (675 unknowns on the
-// 256 x 128 x 128 grid), so all of them, and the inverse below, run back to
+// All of it is a chain of short latency-bound steps (675 unknowns on the
+// 256 x 128 x 128 grid), so all kernels, and the inverse below, run back to
 // back under programmatic dependent launch: a kernel lets the next one launch
 // at its start and waits for its predecessor before it reads anything.
+// Square roots and quotients are the correctly rounded ones, from an
+// approximate reciprocal square root and fused remainders (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990): a chain of five FMAs instead of two library
+// calls on the pivots' critical path.  Measured for 675 unknowns, kernels
+// serialised: 22 panel steps of 13.4 us and 21 trailing updates of 6.5 us; 16.3
+// us (a CTA with a thread per entry, two divisions per entry and column), 14.0
+// us and 9.0 us as separate diagonal, panel and trailing kernels, with the same
+// bits.  The inverse below took 0.27 ms and takes 0.11 ms (tile_product).
 // info = 1-based index of the first non-positive (or NaN) pivot, 0 on
 // success; once set, every later factor kernel returns at once.
 constexpr int kCholB = 32;
 
-// Column step j: every thread forms the pivot sqrt(D[j][j]) and the scaled
-// entries it needs itself (the same operations on the same values, so the
-// same bits as one thread forming them), the scaled column goes to Lc, and the
-// trailing update writes only columns > j: one barrier per column.
-__global__ void __launch_bounds__(1024) chol_diag_kernel(int n, int c0, int w, double *__restrict__ A,
-                                                         int *__restrict__ info)
+// s / d for y = 1 / d to about 2^-51: the product's remainder corrects it to
+// the rounded quotient (its error before the last rounding is about 2^-103).
+__device__ __forceinline__ double div_by(double s, double d, double y)
 {
-    pdl_wait();
-    pdl_trigger();
-    if (*info) return;
-    __shared__ double D[kCholB][kCholB + 1];
-    __shared__ double Lc[kCholB][kCholB + 1];
-    const int tid = threadIdx.x, r = tid >> 5, c = tid & 31;
-    D[r][c] = (r < w && c <= r) ? A[(long long)(c0 + r) * n + c0 + c] : 0.0;
-    Lc[r][c] = 0.0;
-    __syncthreads();
-    for (int j = 0; j < w; ++j) {
-        const double s = D[j][j];
-        if (!(s > 0.0)) {   // the same value in every thread
-            if (tid == 0) atomicCAS(info, 0, c0 + j + 1);
-            return;
-        }
-        const double d = sqrt(s);
-        if (r < w && r >= j) {
-            const double lrj = r == j ? d : D[r][j] / d;
-            if (c == j) Lc[r][j] = lrj;
-            // trailing update inside the block: D[r][c] -= L[r][j] L[c][j], j < c <= r < w
-            if (c > j && c <= r) D[r][c] = fma(-lrj, D[c][j] / d, D[r][c]);
-        }
-        __syncthreads();
-    }
-    if (r < w && c <= r) A[(long long)(c0 + r) * n + c0 + c] = Lc[r][c];
+    const double q = s * y;
+    return fma(fma(-q, d, s), y, q);
 }
+
+// Pivots in this range keep every product and remainder above clear of
+// overflow and of subnormal numbers; others take sqrt and /.
+__device__ __forceinline__ bool pivot_in_range(double s) { return s > 1e-200 && s < 1e200; }
+
+// The lower triangle of the w x w block in Ds (row-major) -> its factor in Ls,
+// one warp, lane r holding row r in registers: column j's pivot comes by a
+// shuffle, the scaled column goes through shared memory (cb), and every entry
+// loses its products in the order of j.  yd[j] = 1 / L[j][j] for div_by (0
+// when the block must divide).  Returns 0, or the 1-based index of the first
+// bad pivot.
+__device__ __forceinline__ int chol_block(int w, const double (*Ds)[kCholB + 1], double (*Ls)[kCholB + 1],
+                                          double (*cb)[kCholB], double *yd)
+{
+    const int r = threadIdx.x & 31;
+    double D[kCholB];
+#pragma unroll
+    for (int c = 0; c < kCholB; ++c) D[c] = Ds[r][c];
+#pragma unroll
+    for (int j = 0; j < kCholB; ++j) {
+        if (j >= w) break;
+        const double s = __shfl_sync(0xffffffffu, D[j], j);
+        if (!(s > 0.0)) return j + 1;   // the same value in every lane
+        double d, l, y = 0.0;
+        if (pivot_in_range(s)) {
+            y = rsqrt(s);
+            const double g = s * y;
+            d = fma(fma(-g, g, s), 0.5 * y, g);
+            l = div_by(D[j], d, y);
+        } else {
+            d = sqrt(s);
+            l = D[j] / d;
+        }
+        if (r == j) l = d;
+        cb[j & 1][r] = l;
+        if (r == 0) yd[j] = y;
+        if (r >= j) Ls[r][j] = l;
+        __syncwarp();
+#pragma unroll
+        for (int c = j + 1; c < kCholB; ++c) D[c] = fma(-l, cb[j & 1][c], D[c]);   // columns c > r are not used
+    }
+    return 0;
+}
+
+constexpr int kCholPanelWarps = 8;
 
 // A warp per row below the panel: x D^T = a by forward substitution, lane c
 // holding entry c; step k finishes x_k on lane k and broadcasts it, and the
 // later lanes subtract x_k D[c][k] (each lane's updates in order of k, as a
 // thread-per-row substitution applies them).
-constexpr int kCholPanelWarps = 8;
-
+// The other CTAs still read the diagonal block's lower triangle, so CTA 0 puts
+// the factor where nothing reads: strictly lower entries mirrored into the
+// upper triangle, the diagonal into column c0 + w; chol_trail_kernel moves them
+// into place.  Without rows below (one CTA, no trailing step) it stores them
+// directly.
 __global__ void __launch_bounds__(kCholPanelWarps * 32) chol_panel_kernel(int n, int c0, int w,
                                                                          double *__restrict__ A,
-                                                                         const int *__restrict__ info)
+                                                                         int *__restrict__ info)
 {
     pdl_wait();
     pdl_trigger();
-    if (*info) return;
-    __shared__ double D[kCholB][kCholB + 1];
-    for (int idx = threadIdx.x; idx < kCholB * kCholB; idx += kCholPanelWarps * 32) {
+    if (*(volatile int *)info) return;
+    __shared__ double Ds[kCholB][kCholB + 1], Ls[kCholB][kCholB + 1], cb[2][kCholB], yd[kCholB];
+    __shared__ int bad;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int idx = tid; idx < kCholB * kCholB; idx += kCholPanelWarps * 32) {
         const int r = idx / kCholB, c = idx - r * kCholB;
-        D[r][c] = (r < w && c <= r) ? A[(long long)(c0 + r) * n + c0 + c] : 0.0;
+        Ds[r][c] = (r < w && c <= r) ? A[(long long)(c0 + r) * n + c0 + c] : 0.0;
+        Ls[r][c] = 0.0;
+    }
+    const int r = c0 + w + blockIdx.x * kCholPanelWarps + warp;
+    double *row = A + (long long)(r < n ? r : 0) * n + c0;
+    double s = r < n && lane < w ? row[lane] : 0.0;
+    __syncthreads();
+    if (warp == 0) {
+        const int b = chol_block(w, Ds, Ls, cb, yd);
+        if (lane == 0) bad = b;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int r = c0 + w + blockIdx.x * kCholPanelWarps + (threadIdx.x >> 5);
+    if (bad) {
+        if (tid == 0) atomicCAS(info, 0, c0 + bad);
+        return;
+    }
+    const bool below = n - c0 - w > 0;
+    if (blockIdx.x == 0)
+        for (int idx = tid; idx < kCholB * kCholB; idx += kCholPanelWarps * 32) {
+            const int rr = idx / kCholB, c = idx - rr * kCholB;
+            if (rr >= w || c > rr) continue;
+            const long long at = !below ? (long long)(c0 + rr) * n + c0 + c
+                                 : c < rr ? (long long)(c0 + c) * n + c0 + rr : (long long)(c0 + rr) * n + c0 + w;
+            A[at] = Ls[rr][c];
+        }
     if (r >= n) return;   // the same for the whole warp
-    double *row = A + (long long)r * n + c0;
-    double s = lane < w ? row[lane] : 0.0;
     for (int k = 0; k < w; ++k) {
-        double xk = lane == k ? s / D[k][k] : 0.0;
+        const double d = Ls[k][k], y = yd[k];
+        double xk = y != 0.0 ? div_by(s, d, y) : s / d;   // lane k's is used
         xk = __shfl_sync(0xffffffffu, xk, k);
         if (lane == k) s = xk;
-        else if (lane > k) s = fma(-xk, D[lane][k], s);
+        else if (lane > k) s = fma(-xk, Ls[lane][k], s);
     }
     if (lane < w) row[lane] = s;
+}
+
+// A 32 x 32 output tile of a product by 256 threads, 2 x 2 entries each, from
+// k-major operand tiles: pairs of rows and columns come as 16-byte reads, so a
+// warp needs three shared-memory wavefronts per k (a row per thread and four
+// single columns needed five times as many and were what the steps below
+// waited for).  Sums run in order of k.
+constexpr int kTileP = kCholB + 2;   // 16-byte aligned rows
+
+__device__ __forceinline__ void tile_product(const double (*P)[kTileP], const double (*Q)[kTileP], double (&acc)[2][2])
+{
+    const int ti = 2 * (threadIdx.x >> 4), tj = 2 * (threadIdx.x & 15);
+#pragma unroll 8
+    for (int k = 0; k < kCholB; ++k) {
+        const double2 a = *reinterpret_cast<const double2 *>(&P[k][ti]), b = *reinterpret_cast<const double2 *>(&Q[k][tj]);
+        acc[0][0] = fma(a.x, b.x, acc[0][0]);
+        acc[0][1] = fma(a.x, b.y, acc[0][1]);
+        acc[1][0] = fma(a.y, b.x, acc[1][0]);
+        acc[1][1] = fma(a.y, b.y, acc[1][1]);
+    }
 }
 
 // grid (t, t) over the trailing 32 x 32 tiles; tiles above the diagonal return
@@ -1038,30 +1109,41 @@ __global__ void __launch_bounds__(256) chol_trail_kernel(int n, int c0, int w, d
     pdl_wait();
     pdl_trigger();
     if (blockIdx.y > blockIdx.x || *info) return;
-    __shared__ double Ar[kCholB][kCholB + 1];
-    __shared__ double Ac[kCholB][kCholB + 1];
+    __shared__ __align__(16) double P[kCholB][kTileP];
+    __shared__ __align__(16) double Q[kCholB][kTileP];
     const int t0 = c0 + w;
     const int r0 = t0 + blockIdx.x * kCholB, q0 = t0 + blockIdx.y * kCholB;
     for (int idx = threadIdx.x; idx < kCholB * kCholB; idx += 256) {
         const int rr = idx / kCholB, k = idx - rr * kCholB;
-        Ar[rr][k] = (r0 + rr < n && k < w) ? A[(long long)(r0 + rr) * n + c0 + k] : 0.0;
-        Ac[rr][k] = (q0 + rr < n && k < w) ? A[(long long)(q0 + rr) * n + c0 + k] : 0.0;
+        P[k][rr] = (r0 + rr < n && k < w) ? A[(long long)(r0 + rr) * n + c0 + k] : 0.0;
+        Q[k][rr] = (q0 + rr < n && k < w) ? A[(long long)(q0 + rr) * n + c0 + k] : 0.0;
     }
+    const int ti = 2 * (threadIdx.x >> 4), tj = 2 * (threadIdx.x & 15);
+    double old[2][2];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int r = r0 + ti + a, c = q0 + tj + b;
+            old[a][b] = r < n && c <= r ? A[(long long)r * n + c] : 0.0;
+        }
     __syncthreads();
-    const int ty = threadIdx.x >> 3, tx = threadIdx.x & 7;   // 32 rows x 8 threads, 4 columns each
-    double acc[4] = {0, 0, 0, 0};
-#pragma unroll 8
-    for (int k = 0; k < kCholB; ++k) {
-        const double a = Ar[ty][k];
+    double acc[2][2] = {};
+    tile_product(P, Q, acc);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q] = fma(a, Ac[tx * 4 + q][k], acc[q]);
-    }
-    const int r = r0 + ty;
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int col = q0 + tx * 4 + q;
-        if (r < n && col <= r) A[(long long)r * n + col] -= acc[q];
-    }
+        for (int b = 0; b < 2; ++b) {
+            const int r = r0 + ti + a, c = q0 + tj + b;
+            if (r < n && c <= r) A[(long long)r * n + c] = old[a][b] - acc[a][b];
+        }
+    if (blockIdx.x == 0)   // the diagonal block's factor into place (see chol_panel_kernel)
+        for (int idx = threadIdx.x; idx < kCholB * kCholB; idx += 256) {
+            const int rr = idx / kCholB, c = idx - rr * kCholB;
+            if (rr < w && c <= rr)
+                A[(long long)(c0 + rr) * n + c0 + c] =
+                    c < rr ? A[(long long)(c0 + c) * n + c0 + rr] : A[(long long)(c0 + rr) * n + c0 + w];
+        }
 }
 
 void launch_cholesky(int n, double *A, int *info, cudaStream_t st)
@@ -1070,15 +1152,14 @@ void launch_cholesky(int n, double *A, int *info, cudaStream_t st)
     for (int c0 = 0; c0 < n; c0 += kCholB) {
         const int w = (n - c0) < kCholB ? (n - c0) : kCholB;
         const int m = n - c0 - w;   // rows below the panel
-        launch_pdl(chol_diag_kernel, dim3(1), dim3(kCholB * kCholB), 0, st, n, c0, w, A, info);
+        launch_pdl(chol_panel_kernel, dim3((unsigned)std::max(1, (m + kCholPanelWarps - 1) / kCholPanelWarps)),
+                   dim3(kCholPanelWarps * 32), 0, st, n, c0, w, A, info);
         count_launches(1);
         if (m > 0) {
             const int *cinfo = info;
-            launch_pdl(chol_panel_kernel, dim3((unsigned)((m + kCholPanelWarps - 1) / kCholPanelWarps)),
-                       dim3(kCholPanelWarps * 32), 0, st, n, c0, w, A, cinfo);
             const unsigned t = (unsigned)((m + kCholB - 1) / kCholB);
             launch_pdl(chol_trail_kernel, dim3(t, t), dim3(256), 0, st, n, c0, w, A, cinfo);
-            count_launches(2);
+            count_launches(1);
         }
     }
 }
@@ -1123,7 +1204,8 @@ __global__ void __launch_bounds__(kCholB) tri_diag_inverse_kernel(int n, const d
         for (int i = 0; i < w; ++i) Linv[(long long)(b0 + i) * n + b0 + j] = (j <= i) ? X[i][j] : 0.0;
 }
 
-// grid (s / 32 column tiles, s / 32 row tiles, pairs); 32 x 32 output tile per CTA
+// grid (s / 32 column tiles, s / 32 row tiles, pairs); 32 x 32 output tile per
+// CTA, the next k chunk's entries read while the current one is multiplied
 template <int STEP>
 __global__ void __launch_bounds__(256) tri_double_kernel(int n, int s, const double *__restrict__ L,
                                                          double *__restrict__ Linv, double *__restrict__ Tb)
@@ -1134,44 +1216,53 @@ __global__ void __launch_bounds__(256) tri_double_kernel(int n, int s, const dou
     const int sc = min(s, n - rows0);   // rows of C (> 0 for every pair the grid holds)
     const int i0 = blockIdx.y * kCholB, j0 = blockIdx.x * kCholB;
     if (i0 >= sc) return;
-    __shared__ double P[kCholB][kCholB + 1];
-    __shared__ double Q[kCholB][kCholB + 1];
-    const int ty = threadIdx.x >> 3, tx = threadIdx.x & 7;
-    double acc[4] = {0, 0, 0, 0};
+    __shared__ __align__(16) double P[kCholB][kTileP];   // [k][i]
+    __shared__ __align__(16) double Q[kCholB][kTileP];   // [k][j]
+    double acc[2][2] = {};
     // STEP 1: T[i][j] = sum_{k >= j} B[i][k] Ainv[k][j]  (k chunks from j0's on)
     // STEP 2: X[i][j] = -sum_{k <= i} Cinv[i][k] T[k][j] (k chunks up to i0's)
     const int kbeg = STEP == 1 ? j0 : 0;
     const int kend = STEP == 1 ? s : min(i0 + kCholB, sc);
-    for (int k0 = kbeg; k0 < kend; k0 += kCholB) {
-        for (int idx = threadIdx.x; idx < kCholB * kCholB; idx += 256) {
-            const int a = idx / kCholB, b = idx - a * kCholB;
-            const bool pin = i0 + a < sc && k0 + b < kend;   // P[a][b]: row i0 + a, column k0 + b
-            const bool qin = k0 + a < kend;                   // Q[a][b]: row k0 + a, column j0 + b
+    const int a0 = threadIdx.x >> 5, b = threadIdx.x & 31;   // rows a0, a0 + 8, ... and column b of a chunk's tiles
+    double pv[4], qv[4];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int a = a0 + 8 * e;
+            const bool pin = i0 + a < sc && k0 + b < kend;   // row i0 + a, column k0 + b
+            const bool qin = k0 + a < kend;                   // row k0 + a, column j0 + b
             if (STEP == 1) {
-                P[a][b] = pin ? L[(long long)(rows0 + i0 + a) * n + o + k0 + b] : 0.0;
-                Q[a][b] = qin ? Linv[(long long)(o + k0 + a) * n + o + j0 + b] : 0.0;
+                pv[e] = pin ? L[(long long)(rows0 + i0 + a) * n + o + k0 + b] : 0.0;
+                qv[e] = qin ? Linv[(long long)(o + k0 + a) * n + o + j0 + b] : 0.0;
             } else {
-                P[a][b] = pin ? Linv[(long long)(rows0 + i0 + a) * n + rows0 + k0 + b] : 0.0;
-                Q[a][b] = qin ? Tb[(long long)(rows0 + k0 + a) * n + o + j0 + b] : 0.0;
+                pv[e] = pin ? Linv[(long long)(rows0 + i0 + a) * n + rows0 + k0 + b] : 0.0;
+                qv[e] = qin ? Tb[(long long)(rows0 + k0 + a) * n + o + j0 + b] : 0.0;
             }
         }
-        __syncthreads();
-#pragma unroll 8
-        for (int k = 0; k < kCholB; ++k) {
-            const double a = P[ty][k];
+    };
+    fetch(kbeg);
+    for (int k0 = kbeg; k0 < kend; k0 += kCholB) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[q] = fma(a, Q[k][tx * 4 + q], acc[q]);
+        for (int e = 0; e < 4; ++e) {
+            P[b][a0 + 8 * e] = pv[e];
+            Q[a0 + 8 * e][b] = qv[e];
         }
         __syncthreads();
+        if (k0 + kCholB < kend) fetch(k0 + kCholB);
+        tile_product(P, Q, acc);
+        __syncthreads();
     }
-    const int i = i0 + ty;
-    if (i >= sc) return;
+    const int ti = 2 * (threadIdx.x >> 4), tj = 2 * (threadIdx.x & 15);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const long long at = (long long)(rows0 + i) * n + o + j0 + tx * 4 + q;
-        if (STEP == 1) Tb[at] = acc[q];
-        else Linv[at] = -acc[q];
-    }
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int i = i0 + ti + a;
+            if (i >= sc) continue;
+            const long long at = (long long)(rows0 + i) * n + o + j0 + tj + c;
+            if (STEP == 1) Tb[at] = acc[a][c];
+            else Linv[at] = -acc[a][c];
+        }
 }
 
 // The last kernel of the setup's factor chain: it does not release its

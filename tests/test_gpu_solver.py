@@ -82,6 +82,36 @@ def test_mex_entry_matches_reference_golden(oracle, gputo, name):
     assert np.linalg.norm(U - d["U"]) <= 1e-9 * np.linalg.norm(d["U"])
 
 
+@pytest.mark.parametrize("shape,nl", [((4, 4, 4), 3), ((4, 4, 8), 3), ((16, 12, 8), 3), ((30, 10, 10), 2)])
+def test_coarsest_factor_sizes_match_oracle(oracle, gputo, shape, nl):
+    """Coarsest matrices of 24 (less than a panel), 36 (a panel and four rows),
+    180 and 1728 unknowns (partial last panels; up to six doubling levels of the
+    inverse): the oracle's iteration count and U to 1e-9, as for the golden
+    solves."""
+    p = oracle.cantilever(*shape)
+    CX = oracle.simp(oracle.random_density(*shape, seed=6, lo=0.1))[0]
+    U = np.zeros(p.ndof)
+    rr, nit = gputo.mgcg1(p.Ke0, p.F, U, CX, p.fixed, len(p.fixed), *shape, nl, 1e-8, 300, printLev=0)
+    Uo, rro, nito = oracle.mgcg1(p, CX, nl, 1e-8, 300)
+    assert nit == nito and rr < 1e-8
+    assert np.linalg.norm(U - Uo) <= 1e-9 * np.linalg.norm(Uo)
+
+
+def test_coarsest_factor_of_a_tiny_matrix(oracle, gputo):
+    """Moduli of 1e-205 take the pivots out of the range of the short quotients:
+    the solution scales with 1 / E.  The coarsest penalty on the fixed dofs does
+    not, so the preconditioner changes by about its 1e-10: solves to 1e-10 agree
+    to 1e-7."""
+    shape, nl, c = (16, 8, 8), 3, 1e-205
+    p = oracle.cantilever(*shape)
+    CX = oracle.simp(oracle.random_density(*shape, seed=6, lo=0.1))[0]
+    U, V = np.zeros(p.ndof), np.zeros(p.ndof)
+    gputo.mgcg1(p.Ke0, p.F, U, CX, p.fixed, len(p.fixed), *shape, nl, 1e-10, 300, printLev=0)
+    rr, nit = gputo.mgcg1(p.Ke0, p.F, V, CX * c, p.fixed, len(p.fixed), *shape, nl, 1e-10, 300, printLev=0)
+    assert nit > 0 and rr < 1e-10
+    assert np.linalg.norm(V * c - U) <= 1e-7 * np.linalg.norm(U)
+
+
 def test_corner_supports_converged_solution(oracle, gputo):
     d = load_golden("solve_16x8x8_corner_nl3")
     p = _problem(oracle, d)
