@@ -42,7 +42,8 @@ struct Solver {
     int *info = nullptr;
     int *err = nullptr;        // device error flag (bounded waits)
     // device scalars and reduction scratch
-    PcgScalars *sc = nullptr, *h_sc = nullptr;
+    PcgScalars *sc = nullptr, *h_sc = nullptr;   // h_sc[1], h_sc[2]: copies in flight (iterate_ahead)
+    cudaEvent_t ahead_ev[2] = {};
     double *partial = nullptr;
     int partial_cap = 0;
     unsigned *ticket = nullptr;
@@ -94,6 +95,7 @@ struct Solver {
     // (device scalars to h_sc), end (result, status).
     int solve_begin(const double *Fp, double tol, int maxit, cudaStream_t st);
     int solve_poll(cudaStream_t st, bool *finished);
+    int iterate_ahead(int maxit, cudaStream_t st, FILE *log);
     int solve_end(double *Up, double *relres, int *nit, cudaStream_t st);
     void iteration(cudaStream_t st);
     // Element energies of the last solve's U, fused into an FP64 apply (see solver.cu).
