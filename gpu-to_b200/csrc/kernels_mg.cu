@@ -224,8 +224,8 @@ packed_sweep_kernel(Lay L, const T *__restrict__ A, const T *__restrict__ u,
 // kernel's tail), and only then waits for its predecessor before it reads u,
 // f or 1/diag.  Kernels before a sweep that write the matrices (the setup)
 // never release their successors early, so they have completed by then.
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256)
+template <typename T, int MODE, bool EARLY>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 && EARLY ? 1 : 0)
 packed_sweep_slot_kernel(Lay L, const T *__restrict__ A, const T *__restrict__ u, const T *__restrict__ f,
                          const T *__restrict__ rdiag, const uint8_t *__restrict__ mask, T *__restrict__ out,
                          T omega, T prerelax, const int *__restrict__ done)
@@ -243,9 +243,7 @@ packed_sweep_slot_kernel(Lay L, const T *__restrict__ A, const T *__restrict__ u
     const long long nel = g.nel();
     const long long e = slot ? g.elem(ei, ej, ek) : 0;
     const int a = local_index(1 - ex, 1 - ey, 1 - ez);
-    // FP32: all 72 entries in registers before the wait; FP64 loads them after
-    // it (144 registers of entries would halve the CTAs per SM)
-    constexpr bool EARLY = sizeof(T) == 4;
+    // EARLY: all 72 entries in registers before the wait (launch_packed_sweep)
     T am[3][24];   // rows 3 a + d of the slot's element matrix
     auto load_entries = [&]() {
 #pragma unroll
@@ -327,6 +325,21 @@ packed_sweep_slot_kernel(Lay L, const T *__restrict__ A, const T *__restrict__ u
     }
 }
 
+template <typename T, bool EARLY>
+static void slot_sweep(int mode, unsigned nb, const Lay &L, const T *Apk, const T *u, const T *f, const T *rdiag,
+                       const uint8_t *mask, T *out, T omega, T prerelax, const int *done, cudaStream_t st)
+{
+    auto go = [&](auto *kernel) {
+        launch_pdl(kernel, dim3(nb), dim3(256), 0, st, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done);
+    };
+    switch (mode) {
+    case MODE_APPLY: go(packed_sweep_slot_kernel<T, MODE_APPLY, EARLY>); break;
+    case MODE_DEFECT: go(packed_sweep_slot_kernel<T, MODE_DEFECT, EARLY>); break;
+    case MODE_JACOBI: go(packed_sweep_slot_kernel<T, MODE_JACOBI, EARLY>); break;
+    default: go(packed_sweep_slot_kernel<T, MODE_JACOBI_PRE, EARLY>);
+    }
+}
+
 template <typename T>
 void launch_packed_sweep(int mode, const Lay &L, const T *Apk, const T *u, const T *f,
                          const T *rdiag, const uint8_t *mask, T *out, T omega, T prerelax,
@@ -335,19 +348,13 @@ void launch_packed_sweep(int mode, const Lay &L, const T *Apk, const T *u, const
     const int bs = 128;
     if (L.g.nnod() < 65536) {
         const unsigned sb = (unsigned)((L.g.nnod() + 31) / 32);
-        switch (mode) {
-        case MODE_APPLY:
-            launch_pdl(packed_sweep_slot_kernel<T, MODE_APPLY>, dim3(sb), dim3(256), 0, st, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done);
-            break;
-        case MODE_DEFECT:
-            launch_pdl(packed_sweep_slot_kernel<T, MODE_DEFECT>, dim3(sb), dim3(256), 0, st, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done);
-            break;
-        case MODE_JACOBI:
-            launch_pdl(packed_sweep_slot_kernel<T, MODE_JACOBI>, dim3(sb), dim3(256), 0, st, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done);
-            break;
-        default:
-            launch_pdl(packed_sweep_slot_kernel<T, MODE_JACOBI_PRE>, dim3(sb), dim3(256), 0, st, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done);
-        }
+        // FP64's 72 entries take 144 registers, one CTA per SM: early loads pay
+        // while every CTA has an SM of its own (a 64 x 32 x 32 FP64 solve 6.01 ->
+        // 5.67 ms)
+        if (sizeof(T) == 4 || sb <= 148)
+            slot_sweep<T, true>(mode, sb, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done, st);
+        else
+            slot_sweep<T, false>(mode, sb, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done, st);
         count_launches(1);
         return;
     }
@@ -431,12 +438,57 @@ __global__ void restrict_kernel(Lay Lc, Lay Lf, const T *__restrict__ rf,
     restrict_node<T>(Lc, Lf, rf, maskc, fc, i, j, k);
 }
 
+// The same with a thread per value (blockIdx.y = plane): 27 loads in flight
+// instead of 81 one after the other, for grids whose nodes are too few to hide
+// latency.  On large ones the thread per node reads each line fewer times.
+template <typename T>
+__global__ void __launch_bounds__(128)
+restrict_value_kernel(Lay Lc, Lay Lf, const T *__restrict__ rf, const uint8_t *__restrict__ maskc, T *__restrict__ fc,
+                      const int *__restrict__ done)
+{
+    pdl_wait();
+    pdl_trigger();
+    if (done && *done) return;
+    const Grid &gc = Lc.g, &gf = Lf.g;
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), i = (int)blockIdx.y, rowv = 3 * (gc.ny + 1);
+    const int k = t / rowv, c = t - k * rowv, j = c / 3, d = c - 3 * j;
+    if (k > gc.nz) return;
+    const T *src = rf + d;
+    T v[27];
+#pragma unroll
+    for (int di = -1; di <= 1; ++di)
+#pragma unroll
+        for (int dk = -1; dk <= 1; ++dk)
+#pragma unroll
+            for (int dj = -1; dj <= 1; ++dj) {
+                const int fi = 2 * i + di, fk = 2 * k + dk, fj = 2 * j + dj;
+                const bool ok = fi >= 0 && fi <= gf.nx && fk >= 0 && fk <= gf.nz && fj >= 0 && fj <= gf.ny;
+                v[(di + 1) * 9 + (dk + 1) * 3 + dj + 1] = ok ? src[Lf.at(fi, fj, fk)] : T(0);
+            }
+    const unsigned m = maskc[gc.node(i, j, k)];
+    T acc = T(0);
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const T w = T(1.0 / (1 << ((q / 9 != 1) + (q / 3 % 3 != 1) + (q % 3 != 1))));
+        acc = fma(w, v[q], acc);
+    }
+    fc[Lc.at(i, j, k) + d] = ((m >> d) & 1u) ? T(0) : acc;
+}
+
 template <typename T>
 void launch_restrict(const Lay &Lc, const Lay &Lf, const T *rf, const uint8_t *maskc, T *fc,
                      const int *done, cudaStream_t st)
 {
     const int bs = 128;
-    launch_pdl(restrict_kernel<T>, plane_grid(Lc.g, bs), dim3(bs), 0, st, Lc, Lf, rf, maskc, fc, done);
+    // up to 100,000 coarse nodes (measured: 20,000 less good, 64 x 32 x 32 FP64
+    // solves 6.01 -> 5.91 ms, with the prolongation's 5.74 ms)
+    if (Lc.g.nnod() < 100000) {
+        const int values = 3 * (Lc.g.ny + 1) * (Lc.g.nz + 1);
+        launch_pdl(restrict_value_kernel<T>, dim3((unsigned)((values + bs - 1) / bs), (unsigned)(Lc.g.nx + 1)), dim3(bs), 0,
+                   st, Lc, Lf, rf, maskc, fc, done);
+    } else {
+        launch_pdl(restrict_kernel<T>, plane_grid(Lc.g, bs), dim3(bs), 0, st, Lc, Lf, rf, maskc, fc, done);
+    }
     count_launches(1);
 }
 template void launch_restrict<double>(const Lay &, const Lay &, const double *, const uint8_t *,
@@ -531,12 +583,53 @@ __global__ void prolong_cell_kernel(Lay Lf, Lay Lc, const T *__restrict__ uc, co
     }
 }
 
+// The same with a thread per fine value (blockIdx.y = fine plane): up to eight
+// coarse loads and one fine one in flight, for small grids.
+template <typename T>
+__global__ void __launch_bounds__(128)
+prolong_value_kernel(Lay Lf, Lay Lc, const T *__restrict__ uc, const uint8_t *__restrict__ maskf, T *__restrict__ uf,
+                     const int *__restrict__ done)
+{
+    pdl_wait();
+    pdl_trigger();
+    if (done && *done) return;
+    const Grid &gf = Lf.g;
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), i = (int)blockIdx.y, rowv = 3 * (gf.ny + 1);
+    const int k = t / rowv, c = t - k * rowv, j = c / 3, d = c - 3 * j;
+    if (k > gf.nz) return;
+    const int ni = (i & 1) + 1, nk = (k & 1) + 1, nj = (j & 1) + 1;
+    const T *c0 = uc + Lc.at(i >> 1, j >> 1, k >> 1) + d;
+    const long long si = (long long)(Lc.g.nz + 1) * Lc.pitch, sk = Lc.pitch;
+    const long long at = Lf.at(i, j, k) + d;
+    const T v = uf[at];
+    T x[8];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+                x[4 * a + 2 * q + b] = a < ni && q < nk && b < nj ? c0[a * si + q * sk + 3 * b] : T(0);
+    const unsigned m = maskf[gf.node(i, j, k)];
+    T acc = T(0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc += x[q];
+    const T w = T(1) / T(ni * nj * nk);
+    uf[at] = ((m >> d) & 1u) ? T(0) : fma(w, acc, v);
+}
+
 template <typename T>
 void launch_prolong_add(const Lay &Lf, const Lay &Lc, const T *uc, const uint8_t *maskf, T *uf,
                         const int *done, cudaStream_t st)
 {
     const int bs = 128;
-    launch_pdl(prolong_cell_kernel<T>, plane_grid(Lc.g, bs), dim3(bs), 0, st, Lf, Lc, uc, maskf, uf, done);
+    if (Lf.g.nnod() < 300000) {   // fine nodes
+        const int values = 3 * (Lf.g.ny + 1) * (Lf.g.nz + 1);
+        launch_pdl(prolong_value_kernel<T>, dim3((unsigned)((values + bs - 1) / bs), (unsigned)(Lf.g.nx + 1)), dim3(bs), 0,
+                   st, Lf, Lc, uc, maskf, uf, done);
+    } else {
+        launch_pdl(prolong_cell_kernel<T>, plane_grid(Lc.g, bs), dim3(bs), 0, st, Lf, Lc, uc, maskf, uf, done);
+    }
     count_launches(1);
 }
 template void launch_prolong_add<double>(const Lay &, const Lay &, const double *, const uint8_t *,
