@@ -9,8 +9,9 @@
 // 9 (dx+1) + 3 (dz+1) + (dy+1).
 //
 // The 16 -> 32 and 32 -> 64 convolutions and their data gradients are implicit
-// GEMMs on the 5th-generation tensor cores (conv_tc_kernel); the first layer,
-// the 1x1x1 head and the weight gradients run on the CUDA cores.
+// GEMMs on the 5th-generation tensor cores (conv_tc_kernel); so are their
+// weight gradients (wgrad_tc_kernel); the first layer and the 1x1x1 head run on
+// the CUDA cores.
 //
 // Activations and gradients between the layers are stored as "split rows":
 //  * a grid node is row r = guard + ((s (X + 1) + x) (Z + 1) + z) (Y + 1) + y;
@@ -324,10 +325,42 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar)
 
 // K-major BF16 operand without swizzle: 8 rows x 16 bytes contiguous, the
 // next 8 rows 128 bytes on (SBO), the next 8 channels lbo bytes on (LBO).
-__device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo)
+__device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo, uint32_t sbo = 128)
 {
-    return ((uint64_t)(addr >> 4) & 0x3FFFull) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) | ((uint64_t)(128 >> 4) << 32) |
-           ((uint64_t)1 << 46);
+    return ((uint64_t)(addr >> 4) & 0x3FFFull) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
+           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46);
+}
+
+__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+        : "memory");
+}
+
+__device__ __forceinline__ void tc_load16(uint32_t addr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
+}
+
+// The registers of earlier TMEM loads may be read from here on (they pass
+// through, so that no use moves ahead of the wait).
+__device__ __forceinline__ void tc_wait_loads(uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
 }
 
 template <int CK, int CN, int EPI>
@@ -423,12 +456,7 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
                                     a0 + s * C::STAGE + ((part * C::C8 + 2 * ks) * C::RS + dy) * 16, C::RS * 16);
                                 const uint64_t db =
                                     tc_desc(b0 + ((3 * seg + dy) * C::C8 + 2 * ks) * CN * 16, CN * 16);
-                                asm volatile(
-                                    "{\n\t.reg .pred p;\n\t"
-                                    "setp.ne.b32 p, %4, 0;\n\t"
-                                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d),
-                                    "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-                                    : "memory");
+                                tc_mma(d, da, db, idesc, acc);
                                 acc = 1;
                             }
                     tc_commit(&empty[s]);
@@ -455,15 +483,8 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
 #pragma unroll
                 for (int c0 = 0; c0 < CN; c0 += 16) {
                     uint32_t r[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
-                        "tcgen05.wait::ld.sync.aligned;"
-                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                          "=r"(r[14]), "=r"(r[15])
-                        : "r"(tmem + lane_off + (uint32_t)(tb * CN + c0))
-                        : "memory");
+                    tc_load16(tmem + lane_off + (uint32_t)(tb * CN + c0), r);
+                    tc_wait_loads(r);
 #pragma unroll
                     for (int c = 0; c < 16; ++c) acc[c0 + c] += __uint_as_float(r[c]);
                 }
@@ -584,41 +605,282 @@ head_backward_kernel(const float *__restrict__ gy, const float *__restrict__ act
 }
 
 // Weight gradients gw[co][ci][tap] = sum over rows of g[row][co]
-// x[row + offset(tap)][ci] and bias gradients, one CTA per (row range, dx).
-// A thread keeps G output channels x the 9 (dz, dy) taps of one input channel
-// in registers: per row it reads its G gradients (the same for a warp) and
-// three new input values (the dy taps slide along the row), for 9 G FMAs as
-// paired instructions, so it runs near the FMA rate.  The CTAs' sums go to
-// part[range][(co CI + ci) 27 + tap] and are added in a fixed order
-// (sum_parts_kernel).  Eight 33^3 samples: 892, 290 and 153 us for the three
-// layers (the 32 -> 64 one at 53 % of the FMA rate), 8616 us together with one
-// CTA per (co, ci) pair and per sample.  Layer 1 reads its input from the dense [S][4][n].
-constexpr int kWgRows = 48;   // rows staged at a time
+// x[row + offset(tap)][ci] and bias gradients of layers 2 and 3, as GEMMs over
+// the rows: A = g' (M = output channels), B = x (N = input channels), both
+// M- / N-major, straight from the split rows.  A tap's shift by dy is again an
+// operand address 16 bytes on.  A CTA takes a range of 128-row tiles and SEG
+// of the nine (dx, dz) pairs, i.e. 3 SEG taps with a TMEM accumulator each.
+//
+// Both operands have three parts.  16 x 32: M holds all parts of g (96 of 128
+// lanes), N all parts of x: the nine products in one MMA.  32 x 64: M = 128
+// is (hi, mid) of g against all of x, and a second MMA adds (mid, lo) x hi to
+// the columns of x's lo part, where its upper half, lo x hi, belongs; its
+// lower half is the mid x hi that the first one left in the upper lanes of x's
+// hi columns, which are not read.  Left out are lo x mid and lo x lo, below
+// 2^-23 of a product.  A plane of ones in front of the last pair's rows gives
+// the bias gradients: the first group of CTAs takes its last tap 16 columns
+// wider, 8 of ones in front and 8 behind that are not read.
+//
+// Every kWgChunk tiles (256 rows) the accumulators are added into FP32
+// registers, so that the tensor core's truncating adds stay 16 long (with 32
+// the relative error against 64 bits is 1.3 times as large, for 1 % of the time);
+// a tap is drained while the others' MMAs run.  Per CTA the sums over a range go to
+// part[range and lane group][tap][ci][co], added in order by sum_parts_kernel.
+//
+// Bound by the MMAs, whose operands' reads from shared memory (4 KB of A for
+// 32 to 96 columns) outlast the arithmetic: the tensor unit is 71 % busy, at
+// 38 % of its BF16 rate.  A CTA keeps only three (nine) taps, since 512 columns
+// hold no more of them for 32 x 64 and the copies of g would grow.  Eight 33^3
+// samples: 368 and 178 us for layers 3 and 2; 892 and 290 us as FP32 FMAs on
+// the CUDA cores (53 % of their rate), 7.0 ms with a CTA per (co, ci) pair.
+constexpr int kWgChunk = 2;   // tiles per accumulation in TMEM
 
-template <int CO, int CI, int G, bool DENSE>
-__global__ void __launch_bounds__((CO / G) * CI)
-wgrad_kernel(const uint4 *__restrict__ g, const uint4 *__restrict__ xr, const float *__restrict__ xd,
-             float *__restrict__ part, float *__restrict__ bpart, RowGeo q, int tiles_per)
+template <int CO, int CI> struct WgCfg {
+    static constexpr int GP = 3 * CO / 8, XP = 3 * CI / 8;   // planes
+    static constexpr int SEG = CO == 64 ? 1 : 3, T = 3 * SEG, GROUPS = 9 / SEG;
+    static constexpr int SUBS = CO == 64 ? 2 : 3;            // lane groups with sums of their own
+    static constexpr int XR = kRows + 2;
+    static constexpr int GBYTES = GP * kRows * 16, SEGBYTES = XP * XR * 16, ONES = XR * 16;
+    static constexpr int STAGE = GBYTES + SEG * SEGBYTES + ONES, COPIED = GBYTES + SEG * SEGBYTES;
+    static constexpr int NST = 3;
+    static constexpr int N = 3 * CI;
+    static constexpr int COLS = 512;
+    static constexpr int BIAS2 = T * N + 32;                 // columns of lo's bias sums (32 x 64)
+    static constexpr int BARS = NST * STAGE;
+    // the unused last 8 columns of the widened operand read up to a plane past the last stage
+    static constexpr size_t SMEM = BARS + XR * 16 + 16;
+    static_assert(8 * (2 * NST + 2 * T + 1) + 8 <= XR * 16, "barriers");
+    static_assert(BIAS2 + 16 <= COLS && N % 16 == 0, "accumulators");
+    static_assert(CO == 64 || GBYTES + 4 * kRows * 16 <= STAGE, "A's unused planes lie within the stage");
+    static_assert(STAGE % 16 == 0 && BARS % 16 == 0 && SMEM <= 227 * 1024, "shared memory of one CTA");
+    // the rows of pair s within a stage; the plane of ones is in front of the last
+    __host__ __device__ static constexpr int xoff(int s) { return GBYTES + s * SEGBYTES + (s == SEG - 1 ? ONES : 0); }
+    __host__ __device__ static constexpr int dcol(int t) { return t * N + (t == T - 1 ? 16 : 0); }
+};
+
+template <int CO, int CI>
+__global__ void __launch_bounds__(192)
+wgrad_tc_kernel(const uint4 *__restrict__ g, const uint4 *__restrict__ x, float *__restrict__ part,
+                float *__restrict__ bpart, RowGeo q, int tiles_per, int *err)
 {
-    constexpr int NT = (CO / G) * CI, GP = CO + 4, XP = CI + 4;
-    __shared__ __align__(16) float gs[kWgRows][GP];
-    __shared__ __align__(16) float xs[3][kWgRows + 2][XP];
+    using C = WgCfg<CO, CI>;
+    constexpr int T = C::T;
+    extern __shared__ __align__(128) unsigned char sm[];
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + C::BARS), *empty = full + C::NST, *tfull = empty + C::NST,
+             *tempty = tfull + T, *fin = tempty + T;
+    uint32_t *tbase = reinterpret_cast<uint32_t *>(fin + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tbase)),
+                     "r"(C::COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 128) {
+        for (int s = 0; s < C::NST; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int t = 0; t < T; ++t) {
+            mbar_init(&tfull[t], 1);
+            mbar_init(&tempty[t], 128);
+        }
+        mbar_init(fin, 1);
+        fence_barrier_init();
+    }
+    for (int i = tid; i < C::NST * (C::ONES / 16); i += 192) {
+        const int s = i / (C::ONES / 16), k = i - s * (C::ONES / 16);
+        reinterpret_cast<uint4 *>(sm + s * C::STAGE + C::xoff(C::SEG - 1) - C::ONES)[k] =
+            make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tbase;
+    const int grp = (int)blockIdx.y;
+    const bool bias = grp == 0;
+    const int t0 = (int)blockIdx.x * tiles_per, nt = min(tiles_per, q.ntiles - t0);
+    bool bad = false;
+    auto wait = [&](uint64_t *b, uint32_t parity) {
+        if (!bad && !mbar_wait_for(b, parity, kNetWaitNs)) {
+            bad = true;
+            if (err) *(volatile int *)err = GPUTO_ERR_TIMEOUT;
+        }
+    };
+    if (warp == 4) {
+        int it = 0;
+        for (; it < nt; ++it) {
+            const int s = it % C::NST;
+            if (it >= C::NST) wait(&empty[s], (uint32_t)((it / C::NST - 1) & 1));
+            if (__any_sync(0xffffffffu, bad)) {
+                bad = true;
+                break;
+            }
+            if (lane == 0) mbar_arrive_expect_tx(&full[s], C::COPIED);
+            __syncwarp();
+            unsigned char *dst = sm + s * C::STAGE;
+            const long long row = q.guard + (long long)(t0 + it) * kRows;
+            for (int pl = lane; pl < C::GP + C::SEG * C::XP; pl += 32) {
+                if (pl < C::GP) {
+                    bulk_load(dst + pl * (kRows * 16), g + pl * q.R + row, kRows * 16, &full[s]);
+                } else {
+                    const int sg = (pl - C::GP) / C::XP, xp = (pl - C::GP) % C::XP, pair = grp * C::SEG + sg;
+                    bulk_load(dst + C::xoff(sg) + xp * (C::XR * 16),
+                              x + xp * q.R + row + (long long)(pair / 3 - 1) * q.pz + (pair % 3 - 1) * q.py - 1,
+                              C::XR * 16, &full[s]);
+                }
+            }
+        }
+        // copies in flight land before the CTA leaves (they already have unless a wait gave up)
+        if (bad)
+            for (int k = it > C::NST ? it - C::NST : 0; k < it; ++k)
+                mbar_wait_for(&full[k % C::NST], (uint32_t)((k / C::NST) & 1), kNetWaitNs);
+    } else if (warp == 5) {
+        if (lane == 0) {
+            // M = 128, both operands transposed
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((128u >> 4) << 24);
+            auto width = [](int n) { return (uint32_t)(n >> 3) << 17; };
+            const uint32_t s0 = smem_u32(sm);
+            bool issued = false;
+            for (int it = 0; it < nt && !bad; ++it) {
+                const int s = it % C::NST, ch = it / kWgChunk;
+                const bool first = it % kWgChunk == 0, last = it % kWgChunk == kWgChunk - 1 || it == nt - 1;
+                wait(&full[s], (uint32_t)((it / C::NST) & 1));
+                if (bad) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ga = s0 + s * C::STAGE;
+#pragma unroll
+                for (int t = 0; t < T; ++t) {
+                    if (first && ch > 0) {
+                        wait(&tempty[t], (uint32_t)((ch - 1) & 1));
+                        if (bad) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    }
+                    const bool ones = t == T - 1 && bias;
+                    const uint32_t xa = ga + C::xoff(t / 3) + (t % 3) * 16 - (ones ? C::ONES : 0);
+                    const uint32_t d = tmem + C::dcol(t) - (ones ? 8 : 0);
+                    const uint32_t id = idesc | (ones ? width(C::N + 16) : width(C::N));
+#pragma unroll
+                    for (int ks = 0; ks < kRows / 16; ++ks) {
+                        const uint32_t acc = first && ks == 0 ? 0u : 1u;
+                        const uint64_t da = tc_desc(ga + ks * 256, 128, kRows * 16);
+                        tc_mma(d, da, tc_desc(xa + ks * 256, 128, C::XR * 16), id, acc);
+                        if (CO == 64) {
+                            const uint64_t d2 = tc_desc(ga + (CO / 8) * kRows * 16 + ks * 256, 128, kRows * 16);
+                            tc_mma(tmem + C::dcol(t) + 2 * CI, d2,
+                                   tc_desc(ga + C::xoff(t / 3) + (t % 3) * 16 + ks * 256, 128, C::XR * 16),
+                                   idesc | width(CI), 1u);
+                            if (ones)
+                                tc_mma(tmem + C::BIAS2, d2, tc_desc(xa + ks * 256, 128, C::XR * 16),
+                                       idesc | width(16), acc);
+                        }
+                    }
+                    issued = true;
+                    if (last) tc_commit(&tfull[t]);
+                }
+                // only where the producer waits for it: no arrival is left under way at the end
+                if (!bad && it + C::NST < nt) tc_commit(&empty[s]);
+            }
+            // MMAs in flight end before TMEM is freed
+            if (bad && issued) {
+                tc_commit(fin);
+                mbar_wait_for(fin, 0, kNetWaitNs);
+            }
+        }
+    } else {
+        const uint32_t base = tmem + ((uint32_t)(warp * 32) << 16);
+        const bool upper = CO == 64 && warp >= 2;
+        float acc[T][CI], bacc = 0.f;
+#pragma unroll
+        for (int t = 0; t < T; ++t)
+#pragma unroll
+            for (int c = 0; c < CI; ++c) acc[t][c] = 0.f;
+        const int nch = (nt + kWgChunk - 1) / kWgChunk;
+        for (int ch = 0; ch < nch && !bad; ++ch) {
+#pragma unroll
+            for (int t = 0; t < T; ++t) {
+                wait(&tfull[t], (uint32_t)(ch & 1));
+                if (__any_sync(0xffffffffu, bad)) {   // the TMEM loads are warp-wide
+                    bad = true;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int c0 = 0; c0 < CI; c0 += 16) {
+                    uint32_t hi[16], mid[16], lo[16];
+                    tc_load16(base + C::dcol(t) + 2 * CI + c0, lo);
+                    tc_load16(base + C::dcol(t) + CI + c0, mid);
+                    tc_load16(base + C::dcol(t) + c0, hi);
+                    tc_wait_loads(lo);
+                    tc_wait_loads(mid);
+                    tc_wait_loads(hi);
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        float s = __uint_as_float(lo[c]) + __uint_as_float(mid[c]);
+                        if (!upper) s += __uint_as_float(hi[c]);
+                        acc[t][c0 + c] += s;
+                    }
+                }
+                if (t == T - 1 && bias) {
+                    uint32_t o[16];
+                    tc_load16(base + C::dcol(T - 1) - 8, o);
+                    tc_wait_loads(o);
+                    bacc += __uint_as_float(o[0]);
+                    if (upper) {
+                        tc_load16(base + C::BIAS2, o);
+                        tc_wait_loads(o);
+                        bacc += __uint_as_float(o[0]);
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[t])) : "memory");
+            }
+        }
+        const int sub = tid / CO, co = tid % CO;
+        if (!bad && sub < C::SUBS) {
+            const size_t k = (size_t)blockIdx.x * C::SUBS + sub;
+            float *dst = part + (k * 27 + 3 * C::SEG * grp) * (CI * CO) + co;
+#pragma unroll
+            for (int t = 0; t < T; ++t)
+#pragma unroll
+                for (int c = 0; c < CI; ++c) dst[(t * CI + c) * CO] = acc[t][c];
+            if (bias) bpart[k * CO + co] = bacc;
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::COLS) : "memory");
+}
+
+// The same sums of layer 1, whose 4 channels are too few for the tensor cores,
+// one CTA per (row range, dx).  A thread keeps two output channels x the 9
+// (dz, dy) taps of one input channel in registers: per row it reads its two
+// gradients (the same for a warp) and three new input values (the dy taps
+// slide along the row), for 18 FMAs as paired instructions.  The CTAs' sums go
+// to part[range][(co 4 + ci) 27 + tap].  Eight 33^3 samples: 153 us.
+constexpr int kWg1Rows = 48;   // rows staged at a time
+
+__global__ void __launch_bounds__(32)
+wgrad1_kernel(const uint4 *__restrict__ g, const float *__restrict__ xd, float *__restrict__ part,
+              float *__restrict__ bpart, RowGeo q, int tiles_per)
+{
+    constexpr int CO = 16, CI = 4, GP = CO + 4;
+    __shared__ __align__(16) float gs[kWg1Rows][GP];
+    __shared__ __align__(16) float xs[3][kWg1Rows + 2][CI + 4];
     const int tid = threadIdx.x, ci = tid % CI, cg = tid / CI;
     const int dx = (int)blockIdx.y - 1;
-    const long long ntile = (q.rows + kWgRows - 1) / kWgRows;
+    const long long ntile = (q.rows + kWg1Rows - 1) / kWg1Rows, n = (long long)q.X * q.Z * q.Y;
     const long long t0 = (long long)blockIdx.x * tiles_per, t1 = min(t0 + tiles_per, ntile);
-    float2 acc[G / 2][9], bsum[G / 2];
+    float2 acc[9], bsum = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int c = 0; c < G / 2; ++c) {
-        bsum[c] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int t = 0; t < 9; ++t) acc[c][t] = make_float2(0.f, 0.f);
-    }
+    for (int t = 0; t < 9; ++t) acc[t] = make_float2(0.f, 0.f);
     for (long long tile = t0; tile < t1; ++tile) {
-        const long long r0 = tile * kWgRows;
+        const long long r0 = tile * kWg1Rows;
         __syncthreads();
-        for (int i = tid; i < kWgRows * (CO / 8); i += NT) {
-            const int c = i / kWgRows, rr = i - c * kWgRows;
+        for (int i = tid; i < kWg1Rows * (CO / 8); i += 32) {
+            const int c = i / kWg1Rows, rr = i - c * kWg1Rows;
             float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (r0 + rr < q.rows)
 #pragma unroll
@@ -627,27 +889,12 @@ wgrad_kernel(const uint4 *__restrict__ g, const uint4 *__restrict__ xr, const fl
             d[0] = make_float4(v[0], v[1], v[2], v[3]);
             d[1] = make_float4(v[4], v[5], v[6], v[7]);
         }
-        if constexpr (DENSE) {
-            const long long n = (long long)q.X * q.Z * q.Y;
-            for (int i = tid; i < 3 * (kWgRows + 2) * CI; i += NT) {
-                const int rr = i % (kWgRows + 2), rest = i / (kWgRows + 2), c = rest % CI, dz = rest / CI;
-                const long long r = r0 + rr - 1 + (long long)dx * q.pz + (dz - 1) * q.py;
-                int s, x, z, y;
-                const bool in = r >= 0 && row_node(q, r, s, x, z, y);
-                xs[dz][rr][c] = in ? xd[(4LL * s + c) * n + ((long long)x * q.Z + z) * q.Y + y] : 0.f;
-            }
-        } else {
-            for (int i = tid; i < 3 * (kWgRows + 2) * (CI / 8); i += NT) {
-                const int rr = i % (kWgRows + 2), rest = i / (kWgRows + 2), c = rest % (CI / 8), dz = rest / (CI / 8);
-                const long long r = q.guard + r0 + rr - 1 + (long long)dx * q.pz + (dz - 1) * q.py;
-                float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                if (r < q.R)   // the last tile's overhang meets zero gradients
-#pragma unroll
-                    for (int p = 2; p >= 0; --p) add_part(v, xr[(size_t)(p * (CI / 8) + c) * q.R + r]);
-                float4 *d = reinterpret_cast<float4 *>(&xs[dz][rr][8 * c]);
-                d[0] = make_float4(v[0], v[1], v[2], v[3]);
-                d[1] = make_float4(v[4], v[5], v[6], v[7]);
-            }
+        for (int i = tid; i < 3 * (kWg1Rows + 2) * CI; i += 32) {
+            const int rr = i % (kWg1Rows + 2), rest = i / (kWg1Rows + 2), c = rest % CI, dz = rest / CI;
+            const long long r = r0 + rr - 1 + (long long)dx * q.pz + (dz - 1) * q.py;
+            int s, x, z, y;
+            const bool in = r >= 0 && row_node(q, r, s, x, z, y);
+            xs[dz][rr][c] = in ? xd[(4LL * s + c) * n + ((long long)x * q.Z + z) * q.Y + y] : 0.f;
         }
         __syncthreads();
         float xw[3][3];   // [dz][row mod 3]
@@ -657,57 +904,40 @@ wgrad_kernel(const uint4 *__restrict__ g, const uint4 *__restrict__ xr, const fl
             xw[dz][1] = xs[dz][1][ci];
         }
 #pragma unroll 1
-        for (int rb = 0; rb < kWgRows; rb += 3)
+        for (int rb = 0; rb < kWg1Rows; rb += 3)
 #pragma unroll
             for (int u = 0; u < 3; ++u) {
                 const int rr = rb + u;
-                float2 gv[G / 2];
-                if constexpr (G >= 4) {
-#pragma unroll
-                    for (int c = 0; c < G / 4; ++c) {
-                        const float4 f = *reinterpret_cast<const float4 *>(&gs[rr][cg * G + 4 * c]);
-                        gv[2 * c] = make_float2(f.x, f.y);
-                        gv[2 * c + 1] = make_float2(f.z, f.w);
-                    }
-                } else {
-                    gv[0] = *reinterpret_cast<const float2 *>(&gs[rr][cg * G]);
-                }
+                const float2 gv = *reinterpret_cast<const float2 *>(&gs[rr][2 * cg]);
 #pragma unroll
                 for (int dz = 0; dz < 3; ++dz) xw[dz][(u + 2) % 3] = xs[dz][rr + 2][ci];
-                if (dx == -1)
-#pragma unroll
-                    for (int c = 0; c < G / 2; ++c) bsum[c] = __fadd2_rn(bsum[c], gv[c]);
+                if (dx == -1) bsum = __fadd2_rn(bsum, gv);
 #pragma unroll
                 for (int dz = 0; dz < 3; ++dz)
 #pragma unroll
                     for (int dy = 0; dy < 3; ++dy) {
                         const float v = xw[dz][(u + dy) % 3];
-#pragma unroll
-                        for (int c = 0; c < G / 2; ++c)
-                            acc[c][3 * dz + dy] = __ffma2_rn(gv[c], make_float2(v, v), acc[c][3 * dz + dy]);
+                        acc[3 * dz + dy] = __ffma2_rn(gv, make_float2(v, v), acc[3 * dz + dy]);
                     }
             }
     }
     float *dst = part + (size_t)blockIdx.x * (CO * CI * 27) + 9 * blockIdx.y;
 #pragma unroll
-    for (int c = 0; c < G / 2; ++c)
-#pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            dst[((cg * G + 2 * c) * CI + ci) * 27 + t] = acc[c][t].x;
-            dst[((cg * G + 2 * c + 1) * CI + ci) * 27 + t] = acc[c][t].y;
-        }
-    if (dx == -1 && ci == 0)
-#pragma unroll
-        for (int c = 0; c < G / 2; ++c) {
-            bpart[(size_t)blockIdx.x * CO + cg * G + 2 * c] = bsum[c].x;
-            bpart[(size_t)blockIdx.x * CO + cg * G + 2 * c + 1] = bsum[c].y;
-        }
+    for (int t = 0; t < 9; ++t) {
+        dst[(2 * cg * CI + ci) * 27 + t] = acc[t].x;
+        dst[((2 * cg + 1) * CI + ci) * 27 + t] = acc[t].y;
+    }
+    if (dx == -1 && ci == 0) {
+        bpart[(size_t)blockIdx.x * CO + 2 * cg] = bsum.x;
+        bpart[(size_t)blockIdx.x * CO + 2 * cg + 1] = bsum.y;
+    }
 }
 
 // grads[i] += sum over ranges of part[range][i]: a CTA takes 32 entries, its
 // eight warps every eighth range, and the warps' sums are added in order.
+// With co > 0 the parts are in the order [tap][ci][co] of wgrad_tc_kernel.
 __global__ void __launch_bounds__(256)
-sum_parts_kernel(const float *__restrict__ part, int n, int ranges, float *__restrict__ grads)
+sum_parts_kernel(const float *__restrict__ part, int n, int ranges, float *__restrict__ grads, int co = 0, int ci = 0)
 {
     __shared__ float red[8][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
@@ -720,7 +950,7 @@ sum_parts_kernel(const float *__restrict__ part, int n, int ranges, float *__res
     if (w == 0 && i < n) {
         s = red[0][lane];
         for (int k = 1; k < 8; ++k) s += red[k][lane];
-        grads[i] += s;
+        grads[co ? ((i % co) * ci + i / co % ci) * 27 + i / (co * ci) : i] += s;
     }
 }
 
@@ -819,25 +1049,36 @@ void launch_conv(const ConvArgs &a, const RowGeo &q, int sms, cudaStream_t st)
     count_launches(1);
 }
 
-// Row ranges of the weight-gradient kernels (a CTA per range and dx): two CTAs
-// of 256 threads per SM for 64 x 32 channels, and as many more of the smaller
-// CTAs of the other layers (98 ranges for those left most of the chip idle:
-// 353 and 848 us on eight 33^3 samples).
-constexpr int kWgRanges = 98;
-constexpr int kWgMaxWeights = kWgRanges * 64 * 32 * 27, kWgMaxBias = 8 * kWgRanges * 16;
+// Partial sums of the weight gradients: layer 1 in up to 784 row ranges (a CTA
+// of one warp per range and dx; with 98 most of the chip idles, 848 us on
+// eight 33^3 samples), layers 2 and 3 in as many as give every SM one CTA.
+constexpr int kWg1Ranges = 784, kWgMaxCtas = 296;
+constexpr int kWgMaxWeights = std::max({kWg1Ranges * 16 * 4 * 27, kWgMaxCtas / 3 * 3 * 32 * 16 * 27, kWgMaxCtas / 9 * 2 * 64 * 32 * 27});
+constexpr int kWgMaxBias = std::max({kWg1Ranges * 16, kWgMaxCtas / 3 * 3 * 32, kWgMaxCtas / 9 * 2 * 64});
 
-template <int CO, int CI, int G, bool DENSE>
-void launch_wgrad(const uint4 *g, const uint4 *xr, const float *xd, float *part, float *bpart, float *gw, float *gb,
-                  const RowGeo &q, cudaStream_t st)
+void launch_wgrad1(const uint4 *g, const float *x, float *part, float *bpart, float *gw, float *gb, const RowGeo &q,
+                   cudaStream_t st)
 {
-    constexpr int NT = (CO / G) * CI, MAXR = kWgRanges * (256 / NT);   // 98, 196, 784
-    static_assert(MAXR * CO * CI * 27 <= kWgMaxWeights && MAXR * CO <= kWgMaxBias, "partial sums");
-    const long long ntile = (q.rows + kWgRows - 1) / kWgRows;
-    const int per = (int)((ntile + MAXR - 1) / MAXR), ranges = (int)((ntile + per - 1) / per);
-    wgrad_kernel<CO, CI, G, DENSE><<<dim3((unsigned)ranges, 3), NT, 0, st>>>(g, xr, xd, part, bpart, q, per);
-    const int n = CO * CI * 27;
+    const long long ntile = (q.rows + kWg1Rows - 1) / kWg1Rows;
+    const int per = (int)((ntile + kWg1Ranges - 1) / kWg1Ranges), ranges = (int)((ntile + per - 1) / per);
+    wgrad1_kernel<<<dim3((unsigned)ranges, 3), 32, 0, st>>>(g, x, part, bpart, q, per);
+    constexpr int n = 16 * 4 * 27;
     sum_parts_kernel<<<(n + 31) / 32, 256, 0, st>>>(part, n, ranges, gw);
-    sum_parts_kernel<<<(CO + 31) / 32, 256, 0, st>>>(bpart, CO, ranges, gb);
+    sum_parts_kernel<<<1, 256, 0, st>>>(bpart, 16, ranges, gb);
+    count_launches(3);
+}
+
+template <int CO, int CI>
+void launch_wgrad(const uint4 *g, const uint4 *x, float *part, float *bpart, float *gw, float *gb, const RowGeo &q,
+                  int sms, int *err, cudaStream_t st)
+{
+    using C = WgCfg<CO, CI>;
+    const int most = std::max(1, std::min(sms, kWgMaxCtas) / C::GROUPS);
+    const int per = (q.ntiles + most - 1) / most, ranges = (q.ntiles + per - 1) / per;
+    wgrad_tc_kernel<CO, CI><<<dim3((unsigned)ranges, C::GROUPS), 192, C::SMEM, st>>>(g, x, part, bpart, q, per, err);
+    constexpr int n = CO * CI * 27;
+    sum_parts_kernel<<<(n + 31) / 32, 256, 0, st>>>(part, n, ranges * C::SUBS, gw, CO, CI);
+    sum_parts_kernel<<<(CO + 31) / 32, 256, 0, st>>>(bpart, CO, ranges * C::SUBS, gb);
     count_launches(3);
 }
 
@@ -960,6 +1201,8 @@ int init_net_kernels()
     GPUTO_CUDA(set(conv_tc_kernel<32, 64, EPI_HEAD>, ConvCfg<32, 64>::SMEM));
     GPUTO_CUDA(set(conv_tc_kernel<64, 32, EPI_MASK>, ConvCfg<64, 32>::SMEM));
     GPUTO_CUDA(set(conv_tc_kernel<32, 16, EPI_MASK>, ConvCfg<32, 16>::SMEM));
+    GPUTO_CUDA(set(wgrad_tc_kernel<64, 32>, WgCfg<64, 32>::SMEM));
+    GPUTO_CUDA(set(wgrad_tc_kernel<32, 16>, WgCfg<32, 16>::SMEM));
     if (dev < 64) done[dev] = true;
     return GPUTO_OK;
 }
@@ -1058,9 +1301,9 @@ int Net::backward_from(const float *x, const NetDims &d, int S, cudaStream_t st)
     launch_conv<32, 16, EPI_MASK>(a, q, sms, st);
     auto gw = [&](int l) { return grads + param_offset(l, false); };
     auto gb = [&](int l) { return grads + param_offset(l, true); };
-    launch_wgrad<64, 32, 8, false>(g3, rows2, nullptr, wpart, bpart, gw(2), gb(2), q, st);
-    launch_wgrad<32, 16, 4, false>(g2, rows1, nullptr, wpart, bpart, gw(1), gb(1), q, st);
-    launch_wgrad<16, 4, 2, true>(g1, nullptr, x, wpart, bpart, gw(0), gb(0), q, st);
+    launch_wgrad<64, 32>(g3, rows2, wpart, bpart, gw(2), gb(2), q, sms, d_err, st);
+    launch_wgrad<32, 16>(g2, rows1, wpart, bpart, gw(1), gb(1), q, sms, d_err, st);
+    launch_wgrad1(g1, x, wpart, bpart, gw(0), gb(0), q, st);
     return GPUTO_OK;
 }
 

@@ -100,6 +100,36 @@ def test_tiles_and_samples_match_oracle(gputo, dims, ns):
     assert np.abs(g - ref_g).max() <= 1e-3 * np.abs(ref_g).max()
 
 
+@pytest.mark.parametrize("dims,ns", [((7, 12, 31), 40), ((16, 15, 14), 9), ((3, 2, 129), 23)])
+def test_weight_gradients_of_stacked_samples_are_the_sums(gputo, dims, ns):
+    """A pass over many samples, where a block takes several chunks of row tiles
+    (the last one short), gives the sum of the samples' own gradients, which
+    take one or two chunks each.  Activations and their masks are the same bits
+    on both sides.  A chunk of 512 rows is at most 32 truncating FP32 adds, 4e-6
+    of its sum; for random terms that is 4e-6 sqrt(rows / 512) of the total if
+    all chunks err the same way, and as much again for the separate passes."""
+    rng = np.random.default_rng(int(np.prod(dims)) + ns)
+    th = learned.init_params(5)
+    xs = rng.standard_normal((ns, 4) + dims).astype(np.float32)
+    ts = rng.standard_normal((ns, 3) + dims).astype(np.float32)
+    ms = np.ones((ns, 3) + dims, dtype=np.float32)
+    net = gputo.Net(seed=0)
+    net.set_params(th)
+    g, one = (np.zeros(learned.num_params(), dtype=np.float32) for _ in range(2))
+    net.train_step(_f32(xs), _f32(ts), _f32(ms), ns, dims, 0.0, grads_out=g)
+    ref = np.zeros(learned.num_params())
+    for q in range(ns):
+        net.train_step(_f32(xs[q:q + 1]), _f32(ts[q:q + 1]), _f32(ms[q:q + 1]), 1, dims, 0.0, grads_out=one)
+        ref += one
+    tol = 2 * 4e-6 * np.sqrt(ns * np.prod([d + 1 for d in dims]) / 512)
+    o = 0
+    for ci, co, k in ((4, 16, 27), (16, 32, 27), (32, 64, 27), (64, 3, 1)):
+        for n in (ci * co * k, co):
+            assert np.abs(g[o:o + n] - ref[o:o + n]).max() <= tol * np.abs(ref[o:o + n]).max()
+            o += n
+    assert o == g.size
+
+
 def _problem(gputo, shape=(64, 32, 32), nl=4, seed=0):
     import torch
     F, fixed = gputo.cantilever(*shape)
