@@ -283,26 +283,29 @@ struct ConvArgs {
 //
 // Warp 4's first thread issues the copies, warp 5's first thread the MMAs,
 // warps 0-3 add the segment sums from TMEM (double-buffered) into FP32
-// registers and run the epilogue.  Draining every segment keeps the tensor
-// core's accumulation chains short (its adds truncate): the smallest parts go
-// in first, so 3 K / 16 adds per segment happen at full magnitude, and the
-// nine segment sums are rounded FP32 adds.  Against 64 bits the network's
-// error is below that of the FP32 FMA chains (3.3e-7 against 6.4e-7 at 129 x
-// 65 x 65).
+// registers and run the epilogue.  The tensor core's adds truncate, which
+// shrinks every sum a little, and gradients add that up over all nodes.  So a
+// segment has four accumulators, the hi parts of each dy and the mid and lo
+// parts of all: products of hi parts and weights have 16 bits, few of which
+// are lost in the K / 16 adds of a chain, and the four sums are added with
+// rounding.  With one accumulator per segment the output is low by 1.2e-7 and
+// small grids' gradients are off by 4.3e-7; now 3e-8 and 1.5e-7, no more than
+// with FP32 FMA chains (outputs 2.7e-7 against 6.3e-7, relative to the norm),
+// for 10 % of the forward pass.
 //
 // Persistent, weights resident (110 KB for 32 x 64).  Bound by the operand
 // reads from shared memory (4 KB of A and N 32 bytes of B per MMA) and the
 // nine reads of the activations from L2.  Measured at 129 x 65 x 65: 32 -> 64
-// with the head 249 us (0.9 PFLOP/s of BF16 MMAs; 3167 + 50 us as direct
-// FP32 convolutions on the CUDA cores), 16 -> 32 97 us (733 us); data gradients
-// of eight 33^3 samples 230 and 132 us (2988 and 784 us).
+// with the head 280 us (0.8 PFLOP/s of BF16 MMAs; 3167 + 50 us as direct FP32
+// convolutions on the CUDA cores), 16 -> 32 115 us (733 us); data gradients of
+// eight 33^3 samples 238 and 138 us (2988 and 784 us).
 template <int CK, int CN> struct ConvCfg {
     static constexpr int C8 = CK / 8;
     static constexpr int RS = kRows + 2;                    // rows of a segment
     static constexpr int STAGE = 3 * C8 * RS * 16;          // bytes
     static constexpr int BBYTES = 27 * CK * CN * 2;
     static constexpr int NST = CK == 64 ? 2 : 4;
-    static constexpr int COLS = 2 * CN < 32 ? 32 : 2 * CN;  // TMEM columns (a power of two)
+    static constexpr int COLS = 8 * CN;                     // TMEM columns (a power of two): 2 x 4 accumulators
     static constexpr int BARS = BBYTES + NST * STAGE;
     static constexpr size_t SMEM = BARS + 8 * (2 * NST + 5) + 16 + 200 * 4;
     static_assert(BBYTES % 128 == 0 && STAGE % 16 == 0 && BARS % 16 == 0, "bulk copies need 16-byte alignment");
@@ -444,8 +447,7 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
                     if (it >= 2) wait(&tempty[tb], (uint32_t)((it / 2 - 1) & 1));
                     if (bad) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t d = tmem + (uint32_t)(tb * CN);
-                    uint32_t acc = 0;
+                    const uint32_t d = tmem + (uint32_t)(tb * 4 * CN);
 #pragma unroll
                     for (int part = 2; part >= 0; --part)
 #pragma unroll
@@ -456,8 +458,8 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
                                     a0 + s * C::STAGE + ((part * C::C8 + 2 * ks) * C::RS + dy) * 16, C::RS * 16);
                                 const uint64_t db =
                                     tc_desc(b0 + ((3 * seg + dy) * C::C8 + 2 * ks) * CN * 16, CN * 16);
-                                tc_mma(d, da, db, idesc, acc);
-                                acc = 1;
+                                const bool first = ks == 0 && (part == 0 || (part == 2 && dy == 0));
+                                tc_mma(d + (part ? 3 : dy) * CN, da, db, idesc, first ? 0u : 1u);
                             }
                     tc_commit(&empty[s]);
                     tc_commit(&tfull[tb]);
@@ -482,11 +484,15 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int c0 = 0; c0 < CN; c0 += 16) {
-                    uint32_t r[16];
-                    tc_load16(tmem + lane_off + (uint32_t)(tb * CN + c0), r);
-                    tc_wait_loads(r);
+                    uint32_t r[4][16];
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) acc[c0 + c] += __uint_as_float(r[c]);
+                    for (int p = 0; p < 4; ++p) tc_load16(tmem + lane_off + (uint32_t)((4 * tb + p) * CN + c0), r[p]);
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) tc_wait_loads(r[p]);
+#pragma unroll
+                    for (int c = 0; c < 16; ++c)
+                        acc[c0 + c] += (__uint_as_float(r[0][c]) + __uint_as_float(r[1][c])) +
+                                       (__uint_as_float(r[2][c]) + __uint_as_float(r[3][c]));
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[tb])) : "memory");
