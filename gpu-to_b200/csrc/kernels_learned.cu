@@ -108,15 +108,15 @@ RowGeo row_geo(const NetDims &d, int S)
     return q;
 }
 
-// Row r (without the guard) -> sample, node; false on padding rows.
+// Row r (without the guard) -> sample, node; false on padding rows.  In 32
+// bits: 2^31 rows of the first layer alone (96 bytes each) would be 206 GB.
 __device__ __forceinline__ bool row_node(const RowGeo &q, long long r, int &s, int &x, int &z, int &y)
 {
-    const long long line = r / q.py;
-    y = (int)(r - line * q.py);
-    const long long plane = line / (q.Z + 1);
+    const uint32_t r32 = (uint32_t)r, line = r32 / (uint32_t)q.py, plane = line / (uint32_t)(q.Z + 1);
+    y = (int)(r32 - line * q.py);
     z = (int)(line - plane * (q.Z + 1));
-    s = (int)(plane / (q.X + 1));
-    x = (int)(plane - (long long)s * (q.X + 1));
+    s = (int)(plane / (uint32_t)(q.X + 1));
+    x = (int)(plane - (uint32_t)s * (q.X + 1));
     return s < q.S && x < q.X && z < q.Z && y < q.Y;
 }
 
@@ -298,13 +298,14 @@ struct ConvArgs {
 // nine reads of the activations from L2.  Measured at 129 x 65 x 65: 32 -> 64
 // with the head 280 us (0.8 PFLOP/s of BF16 MMAs; 3167 + 50 us as direct FP32
 // convolutions on the CUDA cores), 16 -> 32 115 us (733 us); data gradients of
-// eight 33^3 samples 238 and 138 us (2988 and 784 us).
+// eight 33^3 samples 232 and 91 us (2988 and 784 us).
 template <int CK, int CN> struct ConvCfg {
     static constexpr int C8 = CK / 8;
     static constexpr int RS = kRows + 2;                    // rows of a segment
     static constexpr int STAGE = 3 * C8 * RS * 16;          // bytes
     static constexpr int BBYTES = 27 * CK * CN * 2;
-    static constexpr int NST = CK == 64 ? 2 : 4;
+    // three stages let two CTAs of 32 -> 16 share an SM (91 us; 132 us with four)
+    static constexpr int NST = CK == 64 ? 2 : CN == 16 ? 3 : 4;
     static constexpr int COLS = 8 * CN;                     // TMEM columns (a power of two): 2 x 4 accumulators
     static constexpr int BARS = BBYTES + NST * STAGE;
     static constexpr size_t SMEM = BARS + 8 * (2 * NST + 5) + 16 + 200 * 4;
@@ -865,7 +866,9 @@ wgrad_tc_kernel(const uint4 *__restrict__ g, const uint4 *__restrict__ x, float 
 // (dz, dy) taps of one input channel in registers: per row it reads its two
 // gradients (the same for a warp) and three new input values (the dy taps
 // slide along the row), for 18 FMAs as paired instructions.  The CTAs' sums go
-// to part[range][(co 4 + ci) 27 + tap].  Eight 33^3 samples: 153 us.
+// to part[range][(co 4 + ci) 27 + tap].  Bound by the staging's latency: with
+// the index arithmetic of every channel of its own and in 64 bits, eight 33^3
+// samples took 158 us, now 70 us; tiles of 96 or 30 rows 5 and 15 us more.
 constexpr int kWg1Rows = 48;   // rows staged at a time
 
 __global__ void __launch_bounds__(32)
@@ -895,12 +898,18 @@ wgrad1_kernel(const uint4 *__restrict__ g, const float *__restrict__ xd, float *
             d[0] = make_float4(v[0], v[1], v[2], v[3]);
             d[1] = make_float4(v[4], v[5], v[6], v[7]);
         }
-        for (int i = tid; i < 3 * (kWg1Rows + 2) * CI; i += 32) {
-            const int rr = i % (kWg1Rows + 2), rest = i / (kWg1Rows + 2), c = rest % CI, dz = rest / CI;
+#pragma unroll
+        for (int k = 0; k < (3 * (kWg1Rows + 2) + 31) / 32; ++k) {
+            const int i = tid + 32 * k, dz = i / (kWg1Rows + 2), rr = i - dz * (kWg1Rows + 2);
+            if (dz > 2) break;
             const long long r = r0 + rr - 1 + (long long)dx * q.pz + (dz - 1) * q.py;
             int s, x, z, y;
-            const bool in = r >= 0 && row_node(q, r, s, x, z, y);
-            xs[dz][rr][c] = in ? xd[(4LL * s + c) * n + ((long long)x * q.Z + z) * q.Y + y] : 0.f;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r >= 0 && row_node(q, r, s, x, z, y)) {
+                const float *p = xd + 4LL * s * n + ((long long)x * q.Z + z) * q.Y + y;
+                v = make_float4(p[0], p[n], p[2 * n], p[3 * n]);
+            }
+            *reinterpret_cast<float4 *>(xs[dz][rr]) = v;
         }
         __syncthreads();
         float xw[3][3];   // [dz][row mod 3]
