@@ -174,8 +174,9 @@ pack_weights_kernel(const float *__restrict__ w2, const float *__restrict__ w3, 
 // writes the split rows of its 16 channels (zeros on padding).  4 x 27 x 16
 // FMAs per node are too few channels for the tensor cores.  A thread takes
 // kC1R rows a CTA width apart, which share each weight read: with one row the
-// kernel was bound by those reads (94 us at 129 x 65 x 65, 72 us now).
-constexpr int kC1R = 4;
+// kernel was bound by those reads (94 us at 129 x 65 x 65, 66 us now); four rows
+// take 154 registers and leave too few warps (72 us).
+constexpr int kC1R = 2;
 
 __global__ void __launch_bounds__(128)
 conv1_kernel(const float *__restrict__ xin, const float *__restrict__ w, const float *__restrict__ b,
@@ -1192,7 +1193,7 @@ int Net::reserve(const NetDims &d, int S, bool train)
         if (!s) s = grow(&g2, cap[6], 12 * plane);
         if (!s) s = grow(&g1, cap[7], 6 * plane);
         if (!s) s = grow(&wpart, cap[8], sizeof(float) * ((size_t)kWgMaxWeights + kWgMaxBias +
-                                                          (size_t)2 * sms * kHeadPart));
+                                                          (size_t)4 * sms * kHeadPart));
     }
     return s;
 }
@@ -1296,7 +1297,8 @@ int Net::backward_from(const float *x, const NetDims &d, int S, cudaStream_t st)
     const RowGeo q = row_geo(d, S);
     const float *p = params;
     float *bpart = wpart + kWgMaxWeights, *hpart = bpart + kWgMaxBias;
-    const int hb = std::min(q.ntiles, 2 * sms);
+    // four CTAs fit an SM and wait on memory: 67 us with two, 48 with four (eight 33^3 samples)
+    const int hb = std::min(q.ntiles, 4 * sms);
     head_backward_kernel<<<hb, 256, 0, st>>>(gy, act3, p + param_offset(3, false), g3, hpart, q);
     // the head's 192 weights and 3 biases are adjacent in grads
     sum_parts_kernel<<<(kHeadPart + 31) / 32, 256, 0, st>>>(hpart, kHeadPart, hb, grads + param_offset(3, false));
