@@ -441,6 +441,7 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
                 (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(CN >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
             const uint32_t b0 = smem_u32(sB), a0 = smem_u32(sA);
             wait(bbar, 0);
+            const int mine = 9 * ((q.ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x);
             int it = 0;
             for (int tile = blockIdx.x; tile < q.ntiles && !bad; tile += gridDim.x)
                 for (int seg = 0; seg < 9; ++seg, ++it) {
@@ -463,7 +464,8 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
                                 const bool first = ks == 0 && (part == 0 || (part == 2 && dy == 0));
                                 tc_mma(d + (part ? 3 : dy) * CN, da, db, idesc, first ? 0u : 1u);
                             }
-                    tc_commit(&empty[s]);
+                    // only where the producer waits for it: no arrival is left under way at the end
+                    if (it + C::NST < mine) tc_commit(&empty[s]);
                     tc_commit(&tfull[tb]);
                 }
             // MMAs in flight end before TMEM is freed
@@ -787,7 +789,7 @@ wgrad_tc_kernel(const uint4 *__restrict__ g, const uint4 *__restrict__ x, float 
                     issued = true;
                     if (last) tc_commit(&tfull[t]);
                 }
-                // only where the producer waits for it: no arrival is left under way at the end
+                // only where the producer waits for it, as in conv_tc_kernel
                 if (!bad && it + C::NST < nt) tc_commit(&empty[s]);
             }
             // MMAs in flight end before TMEM is freed
