@@ -294,9 +294,11 @@ struct ConvArgs {
 // with FP32 FMA chains (outputs 2.7e-7 against 6.3e-7, relative to the norm),
 // for 10 % of the forward pass.
 //
-// Persistent, weights resident (110 KB for 32 x 64).  Bound by the operand
-// reads from shared memory (4 KB of A and N 32 bytes of B per MMA) and the
-// nine reads of the activations from L2.  Measured at 129 x 65 x 65: 32 -> 64
+// Persistent, weights resident (110 KB for 32 x 64).  Copies, MMAs and drains
+// overlap but share the shared memory and TMEM ports, and none of them alone
+// is the bound: a forward pass at 129 x 65 x 65 takes 465 us, 384 with a third
+// of the MMAs, 399 without drains and epilogue, 303 without both, which is the
+// nine reads of the activations (978 MB at about 6.5 TB/s).  Measured at 129 x 65 x 65: 32 -> 64
 // with the head 280 us (0.8 PFLOP/s of BF16 MMAs; 3167 + 50 us as direct FP32
 // convolutions on the CUDA cores), 16 -> 32 115 us (733 us); data gradients of
 // eight 33^3 samples 232 and 91 us (2988 and 784 us).
@@ -637,9 +639,8 @@ head_backward_kernel(const float *__restrict__ gy, const float *__restrict__ act
 // a tap is drained while the others' MMAs run.  Per CTA the sums over a range go to
 // part[range and lane group][tap][ci][co], added in order by sum_parts_kernel.
 //
-// Bound by the MMAs, whose operands' reads from shared memory (4 KB of A for
-// 32 to 96 columns) outlast the arithmetic: the tensor unit is 71 % busy, at
-// 38 % of its BF16 rate.  A CTA keeps only three (nine) taps, since 512 columns
+// Bound by the MMAs: the tensor unit is 71 % busy, at 38 % of its BF16 rate,
+// with 4 KB of A to read for 32 to 96 columns.  A CTA keeps only three (nine) taps, since 512 columns
 // hold no more of them for 32 x 64 and the copies of g would grow.  Eight 33^3
 // samples: 368 and 178 us for layers 3 and 2; 892 and 290 us as FP32 FMAs on
 // the CUDA cores (53 % of their rate), 7.0 ms with a CTA per (co, ci) pair.
