@@ -1,5 +1,4 @@
 // The C ABI of include/gputo.h.
-#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -321,7 +320,7 @@ int gputo_net_forward_dev(gputo_net *h, const float *x, int X, int Z, int Y, flo
     if (!h || !x || !y || X < 1 || Z < 1 || Y < 1) return GPUTO_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     int s = gputo::init_net_kernels();
-    if (!s) s = h->n.forward(x, gputo::NetDims{X, Z, Y}, 1, y, false, st);
+    if (!s) s = h->n.forward(x, gputo::NetDims{X, Z, Y}, y, st);
     if (s) return s;
     GPUTO_CUDA(cudaStreamSynchronize(st));
     GPUTO_CUDA(cudaGetLastError());
@@ -338,10 +337,8 @@ int gputo_net_train_step_dev(gputo_net *h, const float *x, const float *t, const
     int s = gputo::init_net_kernels();
     if (s) return s;
     GPUTO_CUDA(cudaMemsetAsync(h->n.loss_acc, 0, sizeof(double), st));
-    const int group = h->n.group(d, nsamples);
-    for (int q = 0; q < nsamples; q += group) {
-        s = h->n.accumulate(x + (size_t)q * 4 * n, t + (size_t)q * 3 * n, m + (size_t)q * 3 * n, d,
-                            std::min(group, nsamples - q), st);
+    for (int q = 0; q < nsamples; ++q) {
+        s = h->n.accumulate(x + (size_t)q * 4 * n, t + (size_t)q * 3 * n, m + (size_t)q * 3 * n, d, st);
         if (s) return s;
     }
     if (grads_out)
@@ -357,8 +354,6 @@ int gputo_net_train_step_dev(gputo_net *h, const float *x, const float *t, const
     GPUTO_CUDA(cudaMemcpyAsync(&l, h->n.loss_acc, sizeof(double), cudaMemcpyDeviceToHost, st));
     GPUTO_CUDA(cudaStreamSynchronize(st));
     GPUTO_CUDA(cudaGetLastError());
-    s = h->n.check();
-    if (s) return s;
     if (loss) *loss = l / nsamples;
     return GPUTO_OK;
 }

@@ -415,7 +415,6 @@ struct NetDims {
 
 // The network's parameters, Adam state and work buffers on one device.  The
 // formats of the buffers are described in kernels_learned.cu.
-constexpr int kNetGroup = 256;    // samples of one training pass over the network, at most
 constexpr int kNetPart = 2048;    // doubles of loss reduction scratch
 
 struct Net {
@@ -423,14 +422,15 @@ struct Net {
     float *params = nullptr, *grads = nullptr, *m1 = nullptr, *m2 = nullptr;
     double *part = nullptr, *loss_acc = nullptr;   // loss reduction scratch, summed loss
     float *gscale = nullptr;
-    void *img = nullptr;                           // BF16 weight operands of the tensor-core convolutions
-    uint4 *rows1 = nullptr, *rows2 = nullptr;      // activations of layers 1 and 2 (split rows)
-    uint4 *g3 = nullptr, *g2 = nullptr, *g1 = nullptr;   // gradients at the outputs of layers 3, 2 and 1 (split rows)
-    float *act3 = nullptr;                         // layer 3's activations, FP32 rows (training)
-    float *y = nullptr, *gy = nullptr;             // output and its gradient, dense [S][3][n]
-    float *wpart = nullptr;                        // partial weight gradients
-    size_t cap[9] = {};
+    // inference: BF16 weight operands of the tensor-core convolutions, activations of layers 1 and 2 (split rows)
+    void *img = nullptr;
+    uint4 *rows1 = nullptr, *rows2 = nullptr;
+    size_t cap[2] = {};
     int *h_err = nullptr, *d_err = nullptr;        // mapped host flag of the bounded waits
+    // training: act[0] = input (not owned), act[1..4] owned, gradient ping-pong of 64 channels each
+    float *act[5] = {};
+    float *gA = nullptr, *gB = nullptr;
+    long long cap_n = 0;
     long long step = 0;
     std::vector<void *> owned;
 
@@ -438,15 +438,16 @@ struct Net {
     static long long param_offset(int layer, bool bias);
     ~Net();
     int create(unsigned long long seed);
-    int reserve(const NetDims &d, int S, bool train);   // work buffers (never inside a stream capture)
-    // samples that one training pass takes of ns (about a million rows at most)
-    int group(const NetDims &d, int ns) const;
-    // y = net(x) of S stacked samples (yout may be null: the output stays in y); train keeps what the backward needs
-    int forward(const float *x, const NetDims &d, int S, float *yout, bool train, cudaStream_t st);
-    // S samples' masked mean-square losses added to *loss_acc, their gradients to grads
-    int accumulate(const float *x, const float *t, const float *m, const NetDims &d, int S, cudaStream_t st);
-    // gradient of the last training forward's output in gy -> added to grads
-    int backward_from(const float *x, const NetDims &d, int S, cudaStream_t st);
+    int reserve(const NetDims &d);         // inference buffers (never inside a stream capture)
+    int reserve_train(long long nodes);    // training buffers
+    // y = net(x)
+    int forward(const float *x, const NetDims &d, float *y, cudaStream_t st);
+    // the same in the training's arithmetic: activations in act[1..3], output in act[4]
+    int train_forward(const float *x, const NetDims &d, cudaStream_t st);
+    // one sample's masked mean-square loss added to *loss_acc, its gradient to grads
+    int accumulate(const float *x, const float *t, const float *m, const NetDims &d, cudaStream_t st);
+    // gradient of the last training forward's output in gA ([3][n]) -> added to grads
+    int backward_from(const NetDims &d, cudaStream_t st);
     // Adam step with the mean gradient of nsamples accumulated samples; clears grads
     int adam(float lr, int nsamples, cudaStream_t st);
     // status of the kernels' bounded waits since the last check (after a synchronisation)

@@ -456,7 +456,7 @@ void Solver::learned_correction(double *z, const int *done, cudaStream_t st)
     launch_restrict<float>(lay[1], lay[0], Lf[0].f, mask[1], Lf[1].f, done, st);
     launch_restrict<float>(lay[2], lay[1], Lf[1].f, mask[2], Lf[2].f, done, st);
     launch_net_features(lay[2], Lf[2].f, Lf[2].diag, dens2, net_x, nullptr, net_s, done, st);
-    note(net->forward(net_x, nd, 1, net_y, false, st));
+    note(net->forward(net_x, nd, net_y, st));
     launch_net_output(lay[2], net_y, Lf[2].diag, net_s, mask[2], Lf[2].u0, done, st);
     cudaMemsetAsync(Lf[1].u0, 0, sizeof(float) * lay[1].size(), st);
     launch_prolong_add<float>(lay[1], lay[2], Lf[2].u0, mask[1], Lf[1].u0, done, st);
@@ -483,18 +483,18 @@ int Solver::net_train_energy(Net *n, const float *x, const float *gt, int ns, fl
 {
     if (!n || !net_x || ns < 1 || redisc()) return GPUTO_ERR_ARG;
     int s = init_net_kernels();
-    if (!s) s = n->reserve(nd, 1, true);
+    if (!s) s = n->reserve_train(nd.n());
     if (s) return s;
     const long long nn = nd.n();
     GPUTO_CUDA(cudaMemsetAsync(n->loss_acc, 0, sizeof(double), st));
     for (int q = 0; q < ns; ++q) {
-        s = n->forward(x + (size_t)q * 4 * nn, nd, 1, nullptr, true, st);
+        s = n->train_forward(x + (size_t)q * 4 * nn, nd, st);
         if (s) return s;
-        launch_net_to_padded(lay[2], n->y, Lf[2].diag, mask[2], Lf[2].u0, st);
+        launch_net_to_padded(lay[2], n->act[4], Lf[2].diag, mask[2], Lf[2].u0, st);
         apply_level_f32(2, Lf[2].u0, Lf[2].u1, st);
-        s = launch_net_energy(lay[2], n->y, Lf[2].u1, Lf[2].diag, gt + (size_t)q * 3 * nn, mask[2], n->gy, n->part,
+        s = launch_net_energy(lay[2], n->act[4], Lf[2].u1, Lf[2].diag, gt + (size_t)q * 3 * nn, mask[2], n->gA, n->part,
                               kNetPart, n->loss_acc, st);
-        if (!s) s = n->backward_from(x + (size_t)q * 4 * nn, nd, 1, st);
+        if (!s) s = n->backward_from(nd, st);
         if (s) return s;
     }
     if (grads_out)
@@ -510,7 +510,7 @@ int Solver::net_train_energy(Net *n, const float *x, const float *gt, int ns, fl
     GPUTO_CUDA(cudaStreamSynchronize(st));
     GPUTO_CUDA(cudaGetLastError());
     if (loss) *loss = l / ns;
-    return n->check();
+    return GPUTO_OK;
 }
 
 int Solver::attach_net(Net *n, int mode)
@@ -532,7 +532,7 @@ int Solver::attach_net(Net *n, int mode)
         }
         // everything the captured iteration needs exists before any capture
         int s = init_net_kernels();
-        if (!s) s = n->reserve(nd, 1, false);
+        if (!s) s = n->reserve(nd);
         if (s) return s;
     }
     net = n;

@@ -149,3 +149,78 @@ def init_params(seed=0):
         std = np.sqrt(2.0 / fan_in) * (0.1 if l == 3 else 1.0)
         parts += [rng.standard_normal(int(np.prod(ws))) * std, np.zeros(bs[0])]
     return np.concatenate(parts).astype(np.float32)
+
+
+# ---------------------------------------------------------------------------
+# the training step in FP32, each sum in the order the kernels take it
+# ---------------------------------------------------------------------------
+
+def fma32(a, b, c):
+    """float32 fused multiply-add, rounded once: the product is exact in float64, the float64 sum is rounded to odd
+    (its error decides the last bit), and rounding that to float32 gives the rounding of the exact value."""
+    p = a.astype(np.float64) * b
+    c = c.astype(np.float64)
+    s = p + c
+    t = s - p
+    err = (p - (s - t)) + (c - t)
+    even = (s.view(np.int64) & 1) == 0
+    s = np.where((err != 0) & even, np.nextafter(s, np.where(err > 0, np.inf, -np.inf)), s)
+    return s.astype(np.float32)
+
+
+def _conv32(x, w, acc, k):
+    """acc[co] = fma(w[co, ci, tap], x[ci](node + offset), acc[co]) over ci, then taps."""
+    for ci in range(x.shape[0]):
+        for t, d in enumerate(_taps(k)):
+            acc = fma32(w[:, ci, t][:, None, None, None], _shift(x[ci], d)[None], acc)
+    return acc
+
+
+def _threads32(v):
+    """Sum of 256 per-thread values [256, ...]: a butterfly in each warp of 32, then the warps in order."""
+    v = v.reshape((8, 32) + v.shape[1:])
+    for o in (16, 8, 4, 2, 1):
+        v = v + v[:, np.arange(32) ^ o]
+    s = np.zeros(v.shape[2:], np.float32)
+    for w in range(8):
+        s = s + v[w, 0]
+    return s
+
+
+def train_gradients_fp32(xs, ts, ms, theta):
+    """Summed parameter gradients of the masked mean-square losses of the samples, as the training kernels form them:
+    forward and data gradients one FMA chain per value, weight gradients per (co, ci, tap) over the nodes n, n + 256,
+    ... of each of 256 threads, samples one after the other."""
+    layers = [(bf16_round(w), b) for w, b in unpack(theta)]
+    total = [(np.zeros(w.shape, np.float32), np.zeros(b.shape, np.float32)) for w, b in layers]
+    for x, t, m in zip(xs, ts, ms):
+        acts = [x.astype(np.float32)]
+        for l, (w, b) in enumerate(layers):
+            h = _conv32(acts[l], w, np.broadcast_to(b[:, None, None, None], (len(b),) + x.shape[1:]), KSIZE[l])
+            acts.append(np.maximum(h, np.float32(0)) if l < 3 else h)
+        n = int(np.prod(x.shape[1:]))
+        scale = np.float32(2.0 / max(float(m.astype(np.float64).sum()), 1.0))
+        g = scale * m * (acts[4] - t)
+        for l in range(3, -1, -1):
+            w, _ = layers[l]
+            if l < 3:
+                g = np.where(acts[l + 1] > 0, g, np.float32(0))
+            co, ci = w.shape[:2]
+            gf = g.reshape(co, n)
+            xt = np.stack([_shift(acts[l], d).reshape(ci, n) for d in _taps(KSIZE[l])], 2)   # [ci][node][tap]
+            acc = np.zeros((256, co, ci, w.shape[2]), np.float32)
+            bacc = np.zeros((256, co), np.float32)
+            for n0 in range(0, n, 256):
+                c = min(256, n - n0)
+                gv = gf[:, n0:n0 + c].T
+                acc[:c] = fma32(gv[:, :, None, None], xt[:, n0:n0 + c].transpose(1, 0, 2)[:, None], acc[:c])
+                bacc[:c] += gv
+            gw, gb = total[l]
+            total[l] = (gw + _threads32(acc), gb + _threads32(bacc))
+            if l > 0:
+                back = np.zeros((ci,) + x.shape[1:], np.float32)
+                for c in range(co):
+                    for q, d in enumerate(_taps(KSIZE[l])):
+                        back = fma32(w[c, :, q][:, None, None, None], _shift(g[c], tuple(-v for v in d))[None], back)
+                g = back
+    return np.concatenate([a.reshape(-1) for wb in total for a in wb])

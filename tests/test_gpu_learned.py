@@ -130,6 +130,26 @@ def test_weight_gradients_of_stacked_samples_are_the_sums(gputo, dims, ns):
     assert o == g.size
 
 
+@pytest.mark.parametrize("dims,ns", [((7, 6, 9), 2), ((5, 1, 3), 3)])
+def test_training_keeps_the_order_of_its_sums(gputo, dims, ns):
+    """A training amplifies the last bit of a gradient (Adam divides it by its own size, the weights are rounded to
+    BF16), so the gradients of every step of one are pinned bit for bit to the FP32 sums in their order: more nodes
+    than a CTA has threads, and fewer."""
+    rng = np.random.default_rng(int(np.prod(dims)))
+    xs = rng.standard_normal((ns, 4) + dims).astype(np.float32)
+    ts = rng.standard_normal((ns, 3) + dims).astype(np.float32)
+    ms = (rng.random((ns, 3) + dims) > 0.3).astype(np.float32)
+    net = gputo.Net(seed=0)
+    th = learned.init_params(11)
+    th[-3:] = [0.1, -0.2, 0.3]
+    net.set_params(th)
+    for step in range(4):
+        ref = learned.train_gradients_fp32(xs, ts, ms, net.get_params())
+        g = np.zeros(learned.num_params(), dtype=np.float32)
+        net.train_step(_f32(xs), _f32(ts), _f32(ms), ns, dims, 1e-3, grads_out=g)
+        assert np.array_equal(g, ref), (step, np.abs(g - ref).max(), np.abs(ref).max())
+
+
 def _problem(gputo, shape=(64, 32, 32), nl=4, seed=0):
     import torch
     F, fixed = gputo.cantilever(*shape)

@@ -45,3 +45,34 @@ def test_bf16_rounding_is_round_to_nearest_even():
 
 def test_parameter_count_matches_library(gputo):
     assert gputo.Net.num_params() == learned.num_params() == 71155
+
+
+def test_fp32_training_order_agrees_with_the_gradients():
+    """The restatement of the training kernels' FP32 sums against the plain gradients: chains of up to 1728 products
+    rounded to 2^-24 each, 1e-4 of the largest."""
+    rng = np.random.default_rng(8)
+    dims, th = (3, 4, 23), learned.init_params(6)
+    xs = rng.standard_normal((2, 4) + dims).astype(np.float32)
+    ts = rng.standard_normal((2, 3) + dims).astype(np.float32)
+    ms = (rng.random((2, 3) + dims) > 0.3).astype(np.float32)
+    ref = 0.0
+    for x, t, m in zip(xs, ts, ms):
+        y, acts = learned.forward(x, th, dtype=np.float64)
+        ref = ref + learned.backward(acts, th, learned.loss(y, t, m)[1])
+    g = learned.train_gradients_fp32(xs, ts, ms, th)
+    assert g.dtype == np.float32
+    assert np.abs(g - ref).max() <= 1e-4 * np.abs(ref).max()
+
+
+def test_fma32_rounds_once():
+    """Against exact rational arithmetic."""
+    from fractions import Fraction
+    rng = np.random.default_rng(9)
+    a, b, c = (rng.standard_normal(2000).astype(np.float32) for _ in range(3))
+    c *= np.float32(2.0) ** rng.integers(-30, 30, 2000).astype(np.float32)
+    got = learned.fma32(a, b, c)
+    for x, y, z, r in zip(a, b, c, got):
+        e = Fraction(float(x)) * Fraction(float(y)) + Fraction(float(z))
+        lo, hi = np.nextafter(r, np.float32(-np.inf)), np.nextafter(r, np.float32(np.inf))
+        d = abs(e - Fraction(float(r)))
+        assert d <= abs(e - Fraction(float(lo))) and d <= abs(e - Fraction(float(hi)))
