@@ -64,6 +64,32 @@ def test_projection_loop_sizes_and_betas(oracle, gputo, torch, n, beta):
     np.testing.assert_allclose(P.cpu().numpy(), oracle.prj(xt, eta, beta), rtol=0, atol=1e-12 * max(1.0, beta))
 
 
+@pytest.mark.parametrize("beta", [1e-12, 1e-9, 1e-5, 0.01, 0.3, 0.49])
+def test_projection_of_small_betas(oracle, gputo, torch, beta):
+    """beta near zero, where the projection is the identity and tanh(beta (v - eta)) has to keep its relative
+    accuracy.  The volume is that of eta = 0.45, so below 1e-3 the first threshold stays.  The mean of the projection is
+    exact to a few 2^-53 on both sides: eta agrees to 1e-15 over its derivative."""
+    xt = np.random.default_rng(17).random(60001)
+    volfrac, eta0 = oracle.prj(xt, 0.45, beta).mean(), 0.55
+    eta = eta0
+    for _ in range(60):
+        f = oracle.prj(xt, eta, beta).mean() - volfrac
+        if abs(f) <= 1e-6:
+            break
+        eta = eta - f / oracle.deta(xt, eta, beta).mean()
+    assert abs(f) <= 1e-6
+    X = torch.as_tensor(xt, dtype=torch.float64, device="cuda")
+    P = torch.empty_like(X)
+    eta_g = gputo.heaviside_dev(X, P, volfrac, beta, eta0)
+    if eta == eta0:
+        assert eta_g == eta0
+    else:
+        assert abs(eta_g - eta) <= 1e-15 / abs(oracle.deta(xt, eta, beta).mean())
+    # eight roundings of values up to 1, and a shift of eta moves a projected value by at most |beta| of it
+    np.testing.assert_allclose(P.cpu().numpy(), oracle.prj(xt, eta, beta), rtol=0,
+                               atol=2e-15 + abs(beta) * abs(eta_g - eta))
+
+
 @pytest.mark.parametrize("n", [1, 700, 4097, 300001])
 def test_oc_loop_sizes(oracle, gputo, torch, n):
     """The OC update on fewer elements than a CTA, a partial last pass and
