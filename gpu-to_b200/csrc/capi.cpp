@@ -320,11 +320,13 @@ int gputo_net_forward_dev(gputo_net *h, const float *x, int X, int Z, int Y, flo
     if (!h || !x || !y || X < 1 || Z < 1 || Y < 1) return GPUTO_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     int s = gputo::init_net_kernels();
-    if (!s) s = h->n.forward(x, gputo::NetDims{X, Z, Y}, y, st);
+    const gputo::NetDims d{X, Z, Y};
+    if (!s) s = h->n.work.reserve(d);
+    if (!s) s = h->n.forward(h->n.work, x, d, y, st);
     if (s) return s;
     GPUTO_CUDA(cudaStreamSynchronize(st));
     GPUTO_CUDA(cudaGetLastError());
-    return h->n.check();
+    return h->n.work.check();
 }
 
 int gputo_net_train_step_dev(gputo_net *h, const float *x, const float *t, const float *m, int nsamples, int X,

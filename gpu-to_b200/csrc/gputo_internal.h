@@ -413,8 +413,23 @@ struct NetDims {
     __host__ __device__ long long n() const { return (long long)X * Z * Y; }
 };
 
-// The network's parameters, Adam state and work buffers on one device.  The
-// formats of the buffers are described in kernels_learned.cu.
+// Work buffers of an inference, whose formats kernels_learned.cu describes.
+// Each solver that a network is attached to has its own set: solvers that
+// share a network run at the same time (the members of a batch do).
+struct NetWork {
+    void *img = nullptr;                           // BF16 weight operands of the tensor-core convolutions
+    uint4 *rows1 = nullptr, *rows2 = nullptr;      // activations of layers 1 and 2 (split rows)
+    long long cap_rows = 0;
+    int *h_err = nullptr, *d_err = nullptr;        // mapped host flag of the bounded waits
+
+    ~NetWork() { release(); }
+    void release();
+    int reserve(const NetDims &d);   // never inside a stream capture, nor while a captured graph uses the buffers
+    // status of the kernels' bounded waits since the last check (after a synchronisation)
+    int check();
+};
+
+// The network's parameters, Adam state and training buffers on one device.
 constexpr int kNetPart = 2048;    // doubles of loss reduction scratch
 
 struct Net {
@@ -422,11 +437,7 @@ struct Net {
     float *params = nullptr, *grads = nullptr, *m1 = nullptr, *m2 = nullptr;
     double *part = nullptr, *loss_acc = nullptr;   // loss reduction scratch, summed loss
     float *gscale = nullptr;
-    // inference: BF16 weight operands of the tensor-core convolutions, activations of layers 1 and 2 (split rows)
-    void *img = nullptr;
-    uint4 *rows1 = nullptr, *rows2 = nullptr;
-    size_t cap[2] = {};
-    int *h_err = nullptr, *d_err = nullptr;        // mapped host flag of the bounded waits
+    NetWork work;                                  // of the calls on the network itself
     // training: act[0] = input (not owned), act[1..4] owned, gradient ping-pong of 64 channels each
     float *act[5] = {};
     float *gA = nullptr, *gB = nullptr;
@@ -438,10 +449,9 @@ struct Net {
     static long long param_offset(int layer, bool bias);
     ~Net();
     int create(unsigned long long seed);
-    int reserve(const NetDims &d);         // inference buffers (never inside a stream capture)
     int reserve_train(long long nodes);    // training buffers
-    // y = net(x)
-    int forward(const float *x, const NetDims &d, float *y, cudaStream_t st);
+    // y = net(x), w reserved for d
+    int forward(NetWork &w, const float *x, const NetDims &d, float *y, cudaStream_t st) const;
     // the same in the training's arithmetic: activations in act[1..3], output in act[4]
     int train_forward(const float *x, const NetDims &d, cudaStream_t st);
     // one sample's masked mean-square loss added to *loss_acc, its gradient to grads
@@ -450,8 +460,6 @@ struct Net {
     int backward_from(const NetDims &d, cudaStream_t st);
     // Adam step with the mean gradient of nsamples accumulated samples; clears grads
     int adam(float lr, int nsamples, cudaStream_t st);
-    // status of the kernels' bounded waits since the last check (after a synchronisation)
-    int check();
 };
 
 int init_net_kernels();

@@ -810,7 +810,6 @@ Net::~Net()
     for (int l = 1; l <= 4; ++l) cudaFree(act[l]);
     cudaFree(gA);
     cudaFree(gB);
-    if (h_err) cudaFreeHost(h_err);
 }
 
 int Net::create(unsigned long long seed)
@@ -827,12 +826,6 @@ int Net::create(unsigned long long seed)
     owned.push_back(part);
     loss_acc = part + kNetPart;   // part: kNetPart doubles of reduction scratch
     gscale = reinterpret_cast<float *>(loss_acc + 1);
-    GPUTO_CUDA(cudaMalloc(&img, 2 * (size_t)(kImg2 + kImg3)));
-    owned.push_back(img);
-    // where a kernel's bounded wait reports that it gave up: read by the host after a synchronisation
-    GPUTO_CUDA(cudaHostAlloc((void **)&h_err, sizeof(int), cudaHostAllocMapped));
-    *h_err = 0;
-    GPUTO_CUDA(cudaHostGetDevicePointer((void **)&d_err, h_err, 0));
     // He-normal initial weights (last layer scaled by 0.1), zero biases;
     // a fixed generator so that a seed reproduces the network
     std::vector<float> h((size_t)np, 0.f);
@@ -854,24 +847,37 @@ int Net::create(unsigned long long seed)
     return GPUTO_OK;
 }
 
-// Inference buffers.  They only grow; a buffer that is outgrown stays allocated
-// until the network goes, since a solver's captured graph may still use it.
-int Net::reserve(const NetDims &d)
+void NetWork::release()
 {
-    const RowGeo q = row_geo(d);
-    auto grow = [&](uint4 **p, size_t &cap, size_t bytes) -> int {
-        if (bytes <= cap) return GPUTO_OK;
-        void *v = nullptr;
-        GPUTO_CUDA(cudaMalloc(&v, bytes));
-        owned.push_back(v);
-        *p = (uint4 *)v;
-        cap = bytes;
-        return GPUTO_OK;
-    };
-    const size_t plane = 16 * (size_t)q.R;
-    int s = grow(&rows1, cap[0], 6 * plane);
-    if (!s) s = grow(&rows2, cap[1], 12 * plane);
-    return s;
+    cudaFree(img);
+    cudaFree(rows1);
+    cudaFree(rows2);
+    if (h_err) cudaFreeHost(h_err);
+    img = nullptr;
+    rows1 = rows2 = nullptr;
+    h_err = d_err = nullptr;
+    cap_rows = 0;
+}
+
+int NetWork::reserve(const NetDims &d)
+{
+    if (!h_err) {
+        // where a kernel's bounded wait reports that it gave up: read by the host after a synchronisation
+        GPUTO_CUDA(cudaHostAlloc((void **)&h_err, sizeof(int), cudaHostAllocMapped));
+        *h_err = 0;
+        GPUTO_CUDA(cudaHostGetDevicePointer((void **)&d_err, h_err, 0));
+    }
+    if (!img) GPUTO_CUDA(cudaMalloc(&img, 2 * (size_t)(kImg2 + kImg3)));
+    const long long rows = row_geo(d).R;
+    if (rows <= cap_rows) return GPUTO_OK;
+    cudaFree(rows1);
+    cudaFree(rows2);
+    rows1 = rows2 = nullptr;
+    cap_rows = 0;
+    GPUTO_CUDA(cudaMalloc(&rows1, 16 * 6 * (size_t)rows));
+    GPUTO_CUDA(cudaMalloc(&rows2, 16 * 12 * (size_t)rows));
+    cap_rows = rows;
+    return GPUTO_OK;
 }
 
 int Net::reserve_train(long long n)
@@ -906,36 +912,36 @@ int init_net_kernels()
     return GPUTO_OK;
 }
 
-int Net::check()
+int NetWork::check()
 {
-    if (!*(volatile int *)h_err) return GPUTO_OK;
+    if (!h_err || !*(volatile int *)h_err) return GPUTO_OK;
     const int e = *(volatile int *)h_err;
     *(volatile int *)h_err = 0;
     set_error("a bounded wait of the network's convolution gave up");
     return e;
 }
 
-int Net::forward(const float *x, const NetDims &d, float *y, cudaStream_t st)
+int Net::forward(NetWork &w, const float *x, const NetDims &d, float *y, cudaStream_t st) const
 {
-    int s = reserve(d);
-    if (s) return s;
     const RowGeo q = row_geo(d);
+    if (q.R > w.cap_rows) return GPUTO_ERR_ARG;
     const float *p = params;
-    GuardSets gs{{rows1, rows2}, {6, 12}};
+    GuardSets gs{{w.rows1, w.rows2}, {6, 12}};
     zero_guards_kernel<<<dim3(64, 2), 256, 0, st>>>(gs, q);
     pack_weights_kernel<<<(kImg2 + kImg3 + 255) / 256, 256, 0, st>>>(p + param_offset(1, false), p + param_offset(2, false),
-                                                                    (__nv_bfloat16 *)img);
-    conv1_kernel<<<(q.ntiles + kC1R - 1) / kC1R, 128, 0, st>>>(x, p + param_offset(0, false), p + param_offset(0, true), rows1, q);
+                                                                    (__nv_bfloat16 *)w.img);
+    conv1_kernel<<<(q.ntiles + kC1R - 1) / kC1R, 128, 0, st>>>(x, p + param_offset(0, false), p + param_offset(0, true),
+                                                               w.rows1, q);
     count_launches(3);
-    const uint4 *im = reinterpret_cast<const uint4 *>(img);
+    const uint4 *im = reinterpret_cast<const uint4 *>(w.img);
     ConvArgs a{};
-    a.err = d_err;
-    a.a = rows1;
+    a.err = w.d_err;
+    a.a = w.rows1;
     a.img = im;
     a.bias = p + param_offset(1, true);
-    a.out = rows2;
+    a.out = w.rows2;
     launch_conv<16, 32, EPI_RELU>(a, q, sms, st);
-    a.a = rows2;
+    a.a = w.rows2;
     a.img = im + kImg2 / 8;
     a.bias = p + param_offset(2, true);
     a.out = nullptr;

@@ -272,7 +272,7 @@ int Solver::check_error_flags(cudaStream_t st)
         cudaMemsetAsync(err, 0, sizeof(int), st);
         return h_err;
     }
-    return net ? net->check() : GPUTO_OK;
+    return net_work.check();
 }
 
 int Solver::setup(const double *CX_in, cudaStream_t st)
@@ -456,7 +456,7 @@ void Solver::learned_correction(double *z, const int *done, cudaStream_t st)
     launch_restrict<float>(lay[1], lay[0], Lf[0].f, mask[1], Lf[1].f, done, st);
     launch_restrict<float>(lay[2], lay[1], Lf[1].f, mask[2], Lf[2].f, done, st);
     launch_net_features(lay[2], Lf[2].f, Lf[2].diag, dens2, net_x, nullptr, net_s, done, st);
-    note(net->forward(net_x, nd, net_y, st));
+    note(net->forward(net_work, net_x, nd, net_y, st));
     launch_net_output(lay[2], net_y, Lf[2].diag, net_s, mask[2], Lf[2].u0, done, st);
     cudaMemsetAsync(Lf[1].u0, 0, sizeof(float) * lay[1].size(), st);
     launch_prolong_add<float>(lay[1], lay[2], Lf[2].u0, mask[1], Lf[1].u0, done, st);
@@ -532,7 +532,7 @@ int Solver::attach_net(Net *n, int mode)
         }
         // everything the captured iteration needs exists before any capture
         int s = init_net_kernels();
-        if (!s) s = n->reserve(nd);
+        if (!s) s = net_work.reserve(nd);
         if (s) return s;
     }
     net = n;
@@ -542,6 +542,7 @@ int Solver::attach_net(Net *n, int mode)
     const bool want = net_mode == 1;
     if (want != net_on) drop_graphs();
     net_on = want;
+    if (!n) net_work.release();
     return GPUTO_OK;
 }
 

@@ -65,6 +65,7 @@ struct Solver {
     bool net_on = false;       // part of the captured iteration
     int ref_plain_nit = -1, ref_net_nit = -1, net_solves = 0;
     float *net_x = nullptr, *net_y = nullptr, *dens2 = nullptr, *net_s = nullptr;
+    NetWork net_work;          // this solver's own: others may run the same network meanwhile
     NetDims nd{};
     int attach_net(Net *n, int mode);
     void learned_correction(double *z, const int *done, cudaStream_t st);

@@ -357,7 +357,10 @@ void gputo_net_destroy(gputo_net *net);
 int gputo_net_get_params(const gputo_net *net, float *host);
 /* Replaces the parameters and resets the optimizer state. */
 int gputo_net_set_params(gputo_net *net, const float *host);
-/* y[3][n] = net(x[4][n]) on device buffers, n = X Z Y. */
+/* y[3][n] = net(x[4][n]) on device buffers, n = X Z Y.  This call and the
+ * training steps work in buffers of the network: one at a time per network.
+ * Solvers it is attached to have their own and may run at the same time (in a
+ * batch, or on other streams), as long as nothing changes its parameters. */
 int gputo_net_forward_dev(gputo_net *net, const float *x, int X, int Z, int Y, float *y, void *stream);
 /* One training step on nsamples samples stored back to back (x: [4][n] each,
  * target t and loss mask m: [3][n] each): the masked mean-square losses and

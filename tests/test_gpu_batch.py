@@ -41,6 +41,27 @@ def test_batch_matches_individual_solves(gputo, precision):
     assert nits2 == nits and all(torch.equal(a, c) for a, c in zip(Us, Us2))
 
 
+def test_batch_members_may_share_a_network(gputo):
+    """Two members of different grids with the same network attached run their inferences side by side in one graph:
+    each has work buffers of its own, so their results are those of single solves, bit for bit (12 iterations, whether
+    or not the untrained network helps them converge)."""
+    import torch
+    net = gputo.Net(seed=3)
+    members = [_member(gputo, sh, 4, sd, 1) for sh, sd in (((64, 32, 32), 1), ((48, 24, 40), 2))]
+    ref = []
+    for s, F in members:
+        s.set_net(net, 1)
+        U = torch.zeros_like(F)
+        rr, nit = s.solve(F, U, 1e-30, 12)
+        ref.append((U, rr, nit))
+    b = gputo.Batch([s for s, _ in members])
+    for _ in range(3):
+        Us = [torch.zeros_like(F) for _, F in members]
+        rrs, nits = b.solve([F for _, F in members], Us, 1e-30, 12, check_every=5)
+        for (U0, rr0, nit0), U, rr, nit in zip(ref, Us, rrs, nits):
+            assert (rr, nit) == (rr0, nit0) and torch.equal(U, U0)
+
+
 def test_autotune_picks_a_converging_option_and_keeps_the_solution(gputo):
     import torch
     s, F = _member(gputo, (64, 32, 32), 4, 5, 1)
