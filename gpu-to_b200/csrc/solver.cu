@@ -539,9 +539,8 @@ int Solver::attach_net(Net *n, int mode)
     net_mode = n ? mode : 0;
     ref_plain_nit = ref_net_nit = -1;
     net_solves = 0;
-    const bool want = net_mode == 1;
-    if (want != net_on) drop_graphs();
-    net_on = want;
+    net_on = net_mode == 1;
+    drop_graphs();   // a captured iteration holds the last network's parameters
     if (!n) net_work.release();
     return GPUTO_OK;
 }

@@ -235,3 +235,25 @@ def test_learned_correction_gain_and_fallback(gputo, tmp_path):
             "gain_iterations": plain_nit - net_nit}
     (tmp_path / "learned_gain.json").write_text(json.dumps(gain))
     print("learned correction:", gain)
+
+
+def test_attaching_another_network_replaces_the_captured_one(gputo):
+    """Solves run captured iterations: after a second network is attached in the first one's place, they are those of a
+    solver that only ever had the second (8 iterations, bit for bit)."""
+    import torch
+    nets = [gputo.Net(seed=q) for q in (1, 2)]
+
+    def run(s, F):
+        U = torch.zeros_like(F)
+        return s.solve(F, U, 1e-30, 8), U
+
+    s, F = _problem(gputo, (32, 16, 16), 3)
+    s.set_net(nets[0], 1)
+    (r0, n0), U0 = run(s, F)
+    s.set_net(nets[1], 1)
+    (r1, n1), U1 = run(s, F)
+    s2, _ = _problem(gputo, (32, 16, 16), 3)
+    s2.set_net(nets[1], 1)
+    (r2, n2), U2 = run(s2, F)
+    assert (r1, n1) == (r2, n2) and torch.equal(U1, U2)
+    assert not torch.equal(U0, U1)
