@@ -197,8 +197,15 @@ struct HadamardKe {
 };
 bool hadamard_ke(const double *Ke, HadamardKe *hk);
 int init_hsweep_kernels();
-// Test hook of the Hadamard-basis sweeps' bounded waits (see
-// gputo_debug_set_sweep_fault in gputo.h).
+// Test hook of the bounded waits (gputo_debug_set_sweep_fault in gputo.h): the
+// ring stage whose copies a launch leaves unissued (-1: none; the looping
+// design kernels leave out a CTA's arrival instead) and how long each wait
+// lasts before it gives up.
+struct SweepFaultHook {
+    int skip_stage = -1;
+    uint32_t wait_ns = 2000000000u;
+};
+SweepFaultHook sweep_fault_hook();
 int set_sweep_fault_hook(int skip_stage, unsigned wait_us);
 template <typename T> bool hsweep_fits(const Grid &g);
 // The paired FP32 sweep (two element columns per lane, ny <= 512) is built

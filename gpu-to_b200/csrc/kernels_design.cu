@@ -791,21 +791,33 @@ void launch_simp(long long n, const double *x, double penal, double E0, double E
 // ---------------------------------------------------------------------------
 constexpr int kLoopThreads = 512;
 constexpr int kLoopPerSm = 2;
-constexpr uint64_t kLoopWaitNs = 2000000000ull;   // a grid barrier gives up after 2 s
 
 struct LoopSync {
     unsigned arrived, left, failed;   // zero between launches
 };
 
+// How long a grid barrier waits before it gives up (2 s but in tests), and
+// whether the last CTA leaves out its first arrival (test hook).
+struct LoopWait {
+    uint32_t wait_ns;
+    int skip;
+};
+
+static LoopWait loop_wait()
+{
+    const SweepFaultHook h = sweep_fault_hook();
+    return LoopWait{h.wait_ns, h.skip_stage >= 0};
+}
+
 // All CTAs of the launch have arrived (round: 1, 2, ... in every CTA alike).
 // False when the wait gave up.
-__device__ __forceinline__ bool grid_barrier(LoopSync *sync, unsigned round)
+__device__ __forceinline__ bool grid_barrier(LoopSync *sync, unsigned round, LoopWait lw)
 {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        atomicAdd(&sync->arrived, 1u);
+        if (!lw.skip || round > 1 || blockIdx.x != gridDim.x - 1) atomicAdd(&sync->arrived, 1u);
         const unsigned want = round * gridDim.x;
         unsigned seen;
         uint64_t t0 = 0;
@@ -817,7 +829,7 @@ __device__ __forceinline__ bool grid_barrier(LoopSync *sync, unsigned round)
                 uint64_t t;
                 asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
                 if (t0 == 0) t0 = t;
-                else if (t - t0 > kLoopWaitNs) {
+                else if (t - t0 > lw.wait_ns) {
                     ok = 0;
                     break;
                 }
@@ -905,7 +917,7 @@ __device__ __forceinline__ double oc_candidate(double x, double ocp, double lmid
 
 __global__ void __launch_bounds__(kLoopThreads, kLoopPerSm)
 oc_update_kernel(long long n, const double *__restrict__ x, const double *dc, const double *dv0, double *ocp,
-                 double move, double volfrac, double *xnew, double *partial, LoopSync *sync, int max_steps,
+                 double move, double volfrac, double *xnew, double *partial, LoopSync *sync, LoopWait lw, int max_steps,
                  OcState *state)
 {
     __shared__ double tot[kOcCand];
@@ -923,7 +935,7 @@ oc_update_kernel(long long n, const double *__restrict__ x, const double *dc, co
             s[0] += v;
         }
         loop_partials<1>(s, partial);
-        ok = grid_barrier(sync, ++round);
+        ok = grid_barrier(sync, ++round, lw);
         loop_totals<1>(partial, tot);
         l2 = (tot[0] / (double)n) / volfrac;
         lmid = 0.5 * (l1 + l2);
@@ -959,7 +971,7 @@ oc_update_kernel(long long n, const double *__restrict__ x, const double *dc, co
         }
         double *part = partial + (size_t)(round & 1) * kOcCand * gridDim.x;   // the slowest CTA may still read the last
         loop_partials<kOcCand>(s, part);
-        ok = grid_barrier(sync, ++round);
+        ok = grid_barrier(sync, ++round, lw);
         loop_totals<kOcCand>(part, tot);
         int m = 0;
 #pragma unroll
@@ -1031,7 +1043,7 @@ __device__ __forceinline__ double dprj_v(double v, double eta, double beta)
 // formulas.  The design itself is projected with tanh.
 __global__ void __launch_bounds__(kLoopThreads, kLoopPerSm)
 projection_kernel(long long n, const double *__restrict__ xt, double beta, double volfrac, double eta, double *ex,
-                  double *partial, LoopSync *sync, int max_steps, ProjState *state, double *__restrict__ xphys,
+                  double *partial, LoopSync *sync, LoopWait lw, int max_steps, ProjState *state, double *__restrict__ xphys,
                   double *__restrict__ dprj)
 {
     __shared__ double tot[2];
@@ -1077,7 +1089,7 @@ projection_kernel(long long n, const double *__restrict__ xt, double beta, doubl
         }
         double *part = partial + (size_t)(round & 1) * 2 * gridDim.x;
         loop_partials<2>(s, part);
-        ok = grid_barrier(sync, ++round);
+        ok = grid_barrier(sync, ++round, lw);
         loop_totals<2>(part, tot);
         const double f = (t0 + tot[0] / (double)n) / den - volfrac;   // mean(prj) - volfrac
         if (fabs(f) > 1e-6) {
@@ -1117,7 +1129,8 @@ int launch_heaviside(long long n, const double *xt, double volfrac, double beta,
 {
     ProjState *ps = (ProjState *)state;
     LoopSync *ls = (LoopSync *)sync;
-    void *args[] = {&n, &xt, &beta, &volfrac, &eta0, &ex, &partial, &ls, &max_steps, &ps, &xphys, &dprj};
+    LoopWait lw = loop_wait();
+    void *args[] = {&n, &xt, &beta, &volfrac, &eta0, &ex, &partial, &ls, &lw, &max_steps, &ps, &xphys, &dprj};
     GPUTO_CUDA(cudaLaunchCooperativeKernel((const void *)projection_kernel, dim3((unsigned)loop_blocks(n)),
                                            dim3(kLoopThreads), args, 0, st));
     count_launches(1);
@@ -1146,7 +1159,8 @@ int launch_oc_update(long long n, const double *x, const double *dc, const doubl
 {
     OcState *os = (OcState *)state;
     LoopSync *ls = (LoopSync *)sync;
-    void *args[] = {&n, &x, &dc, &dv0, &ocp, &move, &volfrac, &xnew, &partial, &ls, &max_steps, &os};
+    LoopWait lw = loop_wait();
+    void *args[] = {&n, &x, &dc, &dv0, &ocp, &move, &volfrac, &xnew, &partial, &ls, &lw, &max_steps, &os};
     GPUTO_CUDA(cudaLaunchCooperativeKernel((const void *)oc_update_kernel, dim3((unsigned)loop_blocks(n)),
                                            dim3(kLoopThreads), args, 0, st));
     count_launches(1);

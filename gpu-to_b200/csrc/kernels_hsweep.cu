@@ -1164,21 +1164,8 @@ int hztiles_wz(const Grid &g, int WZ)
 }
 template <typename T> int hztiles(const Grid &g) { return hztiles_wz(g, hwz<T>()); }
 
-// Test hook for the bounded waits (gputo_debug_set_sweep_fault): the ring
-// stage whose copies a launch leaves unissued (-1: none) and how long each
-// wait of the march lasts before the CTA gives up (2 s by default).
-struct SweepFaultHook {
-    int skip_stage = -1;
-    uint32_t wait_ns = 2000000000u;
-};
 std::mutex g_hook_mu;
 SweepFaultHook g_hook;
-
-SweepFaultHook sweep_fault_hook()
-{
-    std::lock_guard<std::mutex> lock(g_hook_mu);
-    return g_hook;
-}
 
 struct HState {
     bool init = false, ok = false, ok2 = false;
@@ -1518,6 +1505,13 @@ bool hadamard_ke(const double *Ke, HadamardKe *hk)
     for (int q = 0; q < 8; ++q) hk->c[q] = v[q];
     hk->ok = true;
     return true;
+}
+
+// The hook's values, read at each launch.
+SweepFaultHook sweep_fault_hook()
+{
+    std::lock_guard<std::mutex> lock(g_hook_mu);
+    return g_hook;
 }
 
 int set_sweep_fault_hook(int skip_stage, unsigned wait_us)

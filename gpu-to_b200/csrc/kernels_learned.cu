@@ -52,7 +52,6 @@ __host__ __device__ constexpr int net_k(int l) { return l == 3 ? 1 : 3; }
 __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 constexpr int kRows = 128;                       // rows of one tile (TMEM lanes)
-constexpr uint32_t kNetWaitNs = 2000000000u;     // bounded waits give up after 2 s
 
 // Eight FP32 values -> their three BF16 parts, eight per 16-byte row entry
 // (the same truncating split as kernels_tc.cu's).
@@ -262,6 +261,8 @@ struct ConvArgs {
     const float *w4, *b4;    // EPI_HEAD
     float *y;                // EPI_HEAD: dense output [3][n]
     int *err;                // set when a bounded wait gives up
+    uint32_t wait_ns;        // how long that takes
+    int skip_stage;          // ring stage whose copies are left unissued (test hook; -1: none)
 };
 
 // One convolution as an implicit GEMM: D[row][N] = sum over 27 taps, K input
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
     const uint32_t tmem = *tbase;
     bool bad = false;
     auto wait = [&](uint64_t *b, uint32_t parity) {
-        if (!bad && !mbar_wait_for(b, parity, kNetWaitNs)) {
+        if (!bad && !mbar_wait_for(b, parity, A.wait_ns)) {
             bad = true;
             if (A.err) *(volatile int *)A.err = GPUTO_ERR_TIMEOUT;
         }
@@ -410,16 +411,15 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
                         q.guard + (long long)tile * kRows + (long long)(seg / 3 - 1) * q.pz + (seg % 3 - 1) * q.py - 1;
                     mbar_arrive_expect_tx(&full[s], C::STAGE);
                     unsigned char *dst = sA + s * C::STAGE;
-                    for (int pl = 0; pl < 3 * C::C8; ++pl)
-                        bulk_load(dst + pl * (C::RS * 16), A.a + pl * q.R + row, C::RS * 16, &full[s]);
+                    if (s != A.skip_stage)
+                        for (int pl = 0; pl < 3 * C::C8; ++pl)
+                            bulk_load(dst + pl * (C::RS * 16), A.a + pl * q.R + row, C::RS * 16, &full[s]);
                     ++issued;
                 }
-            // copies in flight land before the CTA leaves (they already have unless a wait gave up)
-            if (bad) {
-                mbar_wait_for(bbar, 0, kNetWaitNs);
-                for (int k = issued > C::NST ? issued - C::NST : 0; k < issued; ++k)
-                    mbar_wait_for(&full[k % C::NST], (uint32_t)((k / C::NST) & 1), kNetWaitNs);
-            }
+            // copies in flight land before the CTA leaves, whichever warp's wait gave up
+            mbar_wait_for(bbar, 0, A.wait_ns);
+            for (int k = issued > C::NST ? issued - C::NST : 0; k < issued; ++k)
+                mbar_wait_for(&full[k % C::NST], (uint32_t)((k / C::NST) & 1), A.wait_ns);
         }
     } else if (warp == 5) {
         if (lane == 0) {
@@ -454,8 +454,8 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
                     if (it + C::NST < mine) tc_commit(&empty[s]);
                     tc_commit(&tfull[tb]);
                 }
-            // MMAs in flight end before TMEM is freed
-            if (bad && it > 0) mbar_wait_for(&tfull[(it - 1) & 1], (uint32_t)(((it - 1) / 2) & 1), kNetWaitNs);
+            // MMAs in flight end before TMEM is freed, whichever warp's wait gave up
+            if (it > 0) mbar_wait_for(&tfull[(it - 1) & 1], (uint32_t)(((it - 1) / 2) & 1), A.wait_ns);
         }
     } else {
         const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
@@ -936,6 +936,9 @@ int Net::forward(NetWork &w, const float *x, const NetDims &d, float *y, cudaStr
     const uint4 *im = reinterpret_cast<const uint4 *>(w.img);
     ConvArgs a{};
     a.err = w.d_err;
+    const SweepFaultHook hook = sweep_fault_hook();
+    a.wait_ns = hook.wait_ns;
+    a.skip_stage = hook.skip_stage;
     a.a = w.rows1;
     a.img = im;
     a.bias = p + param_offset(1, true);

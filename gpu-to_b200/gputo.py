@@ -634,7 +634,9 @@ def _ptr_stream(stream):
 def debug_set_sweep_fault(skip_stage=-1, wait_us=0):
     """Test hook: Hadamard-basis sweeps launched afterwards leave ring stage
     skip_stage unissued and give up each wait after wait_us microseconds
-    (gputo_debug_set_sweep_fault); (-1, 0) restores normal operation."""
+    (gputo_debug_set_sweep_fault), the network's inference likewise, and the
+    OC update and the Heaviside threshold miss one arrival at a grid barrier;
+    (-1, 0) restores normal operation."""
     _check(_lib.gputo_debug_set_sweep_fault(int(skip_stage), int(wait_us)), "gputo_debug_set_sweep_fault")
 
 

@@ -265,7 +265,9 @@ int gputo_solver_time_kernel(gputo_solver *s, int which, int reps, double *ms_pe
  * after this call leave the tile copies of ring stage 'skip_stage' unissued
  * (its mbarrier armed, nothing in flight), and every wait of their march
  * gives up after 'wait_us' microseconds; the sweep then ends early and the
- * call reports GPUTO_ERR_TIMEOUT, with the context still usable.
+ * call reports GPUTO_ERR_TIMEOUT, with the context still usable.  The learned
+ * correction's inference does the same; the OC update and the Heaviside
+ * threshold leave out one CTA's arrival at their first grid barrier instead.
  * gputo_debug_set_sweep_fault(-1, 0) restores normal operation (waits give up
  * after 2 s).  Affects launches, not CUDA graphs captured earlier.  Not for
  * production use. */

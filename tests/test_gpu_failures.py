@@ -15,7 +15,9 @@ CUDA context) still gives correct results:
  * a bounded wait that runs out: the test hook leaves one ring stage of the
    fine sweep armed with no copy in flight, so its mbarrier phase never
    completes; every wait gives up after 200 us, the sweep ends early and the
-   apply reports GPUTO_ERR_TIMEOUT.  The reference has no bounded waits.
+   apply reports GPUTO_ERR_TIMEOUT.  The same for the ring of the network's
+   convolutions, and for a CTA's arrival at the grid barriers of the OC update
+   and the Heaviside threshold.  The reference has no bounded waits.
 """
 import numpy as np
 import pytest
@@ -136,3 +138,49 @@ def test_bounded_wait_runs_out_and_the_context_stays_usable(oracle, gputo, torch
     rr, nit = s.solve(Fd, U, 1e-8, 300)
     assert rr0 < 1e-8 and (rr, nit) == (rr0, nit0)
     assert torch.equal(U, U0)   # the solver is deterministic: the same solve, bit for bit
+
+
+def test_network_waits_run_out_and_the_context_stays_usable(gputo, torch):
+    """The inference's convolutions, several tiles per CTA and fewer: the waits for a ring stage that never lands give
+    up, copies and MMAs in flight end and the tensor memory is freed, so that the next calls give the same bits."""
+    net = gputo.Net(seed=4)
+    for dims in ((40, 33, 65), (3, 4, 5)):
+        n = int(np.prod(dims))
+        x = torch.as_tensor(np.random.default_rng(n).standard_normal(4 * n), dtype=torch.float32, device="cuda")
+        ok, y, again = (torch.empty(3 * n, dtype=torch.float32, device="cuda") for _ in range(3))
+        net.forward(x, dims, ok)
+        for stage in (0, 3):
+            gputo.debug_set_sweep_fault(skip_stage=stage, wait_us=200)
+            try:
+                with pytest.raises(gputo.GputoError) as e:
+                    net.forward(x, dims, y)
+                assert e.value.status == gputo.GPUTO_ERR_TIMEOUT
+            finally:
+                gputo.debug_set_sweep_fault(-1, 0)
+            net.forward(x, dims, again)
+            assert torch.equal(again, ok)
+
+
+@pytest.mark.parametrize("n", [300, 500001])
+def test_design_loop_barriers_run_out_and_the_next_call_is_right(gputo, torch, n):
+    """One CTA and many: a grid barrier that misses an arrival gives up in every CTA, the call reports it, and the
+    counters are ready for the next call."""
+    rng = np.random.default_rng(n)
+    x, dc, dv, xt = (torch.as_tensor(a, dtype=torch.float64, device="cuda") for a in
+                     (rng.random(n), -np.exp(rng.standard_normal(n)), np.full(n, 1.0 / n), rng.random(n)))
+    out, P = torch.empty_like(x), torch.empty_like(x)
+    calls = [(lambda: gputo.oc_update_dev(x, dc, dv, out, 0.3, 0.2), out),
+             (lambda: gputo.heaviside_dev(xt, P, 0.4, 4.0, 0.5), P)]
+    for call, res in calls:
+        r0 = call()
+        ref = res.clone()
+        gputo.debug_set_sweep_fault(skip_stage=0, wait_us=200)
+        try:
+            with pytest.raises(gputo.GputoError) as e:
+                call()
+            assert e.value.status == gputo.GPUTO_ERR_TIMEOUT
+        finally:
+            gputo.debug_set_sweep_fault(-1, 0)
+        for _ in range(2):
+            res.zero_()
+            assert call() == r0 and torch.equal(res, ref)
