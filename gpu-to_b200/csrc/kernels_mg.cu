@@ -1133,9 +1133,8 @@ __global__ void __launch_bounds__(kCholPanelWarps * 32) chol_panel_kernel(int n,
 {
     pdl_wait();
     pdl_trigger();
-    if (*(volatile int *)info) return;
     __shared__ double Ds[kCholB][kCholB + 1], Ls[kCholB][kCholB + 1], cb[2][kCholB], yd[kCholB];
-    __shared__ int bad;
+    __shared__ int failed, bad;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int idx = tid; idx < kCholB * kCholB; idx += kCholPanelWarps * 32) {
         const int r = idx / kCholB, c = idx - r * kCholB;
@@ -1145,7 +1144,10 @@ __global__ void __launch_bounds__(kCholPanelWarps * 32) chol_panel_kernel(int n,
     const int r = c0 + w + blockIdx.x * kCholPanelWarps + warp;
     double *row = A + (long long)(r < n ? r : 0) * n + c0;
     double s = r < n && lane < w ? row[lane] : 0.0;
+    // one thread decides for the CTA: another one of this launch may be setting it
+    if (tid == 0) failed = *(volatile int *)info;
     __syncthreads();
+    if (failed) return;
     if (warp == 0) {
         const int b = chol_block(w, Ds, Ls, cb, yd);
         if (lane == 0) bad = b;

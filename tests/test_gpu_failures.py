@@ -106,6 +106,34 @@ def test_nan_stiffness_is_caught_by_the_coarsest_factor(oracle, gputo):
     assert nit == nito and np.linalg.norm(U2 - Uo) <= 1e-9 * np.linalg.norm(Uo)
 
 
+@pytest.mark.parametrize("where", [0, -1])
+def test_bad_pivot_of_a_wide_panel_is_reported_alike_every_time(gputo, torch, where):
+    """An indefinite stiffness in the first and in the last panels of a coarsest matrix of 4131 unknowns, whose panel
+    steps run hundreds of CTAs that all meet the bad pivot: the same status and pivot in every call, and the next
+    hierarchy is the one from before."""
+    shape = (32, 16, 16)
+    F, fixed = gputo.cantilever(*shape)
+    s = gputo.Solver(*shape, 2, gputo.default_options())
+    s.set_problem(gputo.hex8_stiffness(), fixed)
+    CX = torch.full((int(np.prod(shape)),), 0.5, dtype=torch.float64, device="cuda")
+    r = torch.as_tensor(np.random.default_rng(1).standard_normal(F.size), dtype=torch.float64, device="cuda")
+    z0, z1 = torch.empty_like(r), torch.empty_like(r)
+    s.setup(CX)
+    s.vcycle(r, z0)
+    bad = CX.clone().reshape(32, -1)
+    bad[-4 if where else 2:][:4] = -0.5
+    told = set()
+    for _ in range(8):
+        with pytest.raises(gputo.GputoError) as e:
+            s.setup(bad.reshape(-1))
+        assert e.value.status == gputo.GPUTO_ERR_NOT_SPD
+        told.add(gputo.lib().gputo_last_error())
+    assert len(told) == 1
+    s.setup(CX)
+    s.vcycle(r, z1)
+    assert torch.equal(z0, z1)
+
+
 @pytest.mark.parametrize("prec,pairs", [("fp64", 0), ("fp32", 0), ("fp32", 1)])
 def test_bounded_wait_runs_out_and_the_context_stays_usable(oracle, gputo, torch, prec, pairs):
     """pairs: the FP32 sweep variant (one or two element columns per lane)."""
