@@ -740,6 +740,7 @@ struct Scratch {
         GPUTO_CUDA(cudaMemset(err, 0, sizeof(int)));
         GPUTO_CUDA(cudaMemset(ticket, 0, 16));
         GPUTO_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        static_assert(2048 >= gputo::kEnergyCtas, "a slot per CTA");
         GPUTO_CUDA(cudaMalloc(&partial, sizeof(double) * 2048));   // last: it says that all is there
         return GPUTO_OK;
     }

@@ -336,6 +336,8 @@ bool element_energy_tc_fits(const Grid &g);   // 32-bit dof indexing
 void launch_element_energy_tc(const Grid &g, const double *U, const double *CX, const double *dsK,
                               double *ce, double *dc, double *partial, double *compliance, int *err,
                               cudaStream_t st);
+// partial: max(kEnergyCtas, nblocks) doubles; nblocks: CTAs of the dense kernel.
+constexpr int kEnergyCtas = 1184;
 void launch_element_energy_blocks(const Grid &g, const double *U, const double *CX,
                                   const double *dsK, double *ce, double *dc, double *partial,
                                   unsigned *ticket, double *compliance, int nblocks,

@@ -245,7 +245,11 @@ static int chunk_planes(int nx, long long tiles, long long slots, int extra)
     return best;
 }
 
-// One partial slot per CTA: at most nblocks CTAs.
+// One partial slot per CTA: kEnergyCtas of them, or nblocks for the dense
+// kernel.  The plan's CTAs are the launch's: with the dense kernel's count of
+// 256-thread CTAs as their limit a CTA ran many short chunks, each filling the
+// ring anew (allocation-free call on 9 x 2 x 300 elements 255 us, now 39; 64 x
+// 32 x 32 55 and 35; 40 and 42 with a thread per element).
 void launch_element_energy_blocks(const Grid &g, const double *U, const double *CX,
                                   const double *dsK, double *ce, double *dc, double *partial,
                                   unsigned *ticket, double *compliance, int nblocks,
@@ -263,7 +267,7 @@ void launch_element_energy_blocks(const Grid &g, const double *U, const double *
         const long long tiles = (long long)ntj * ntk;
         const int xc = chunk_planes(g.nx, tiles, (512 / kEnT) * 148, 5);
         const long long items = tiles * ((g.nx + xc - 1) / xc);
-        element_energy_march_kernel<<<(unsigned)std::min<long long>(items, nblocks), kEnT, 0, st>>>(
+        element_energy_march_kernel<<<(unsigned)std::min<long long>(items, kEnergyCtas), kEnT, 0, st>>>(
             g, make_hc<double>(hk), xc, ntj, ntk, items, U, CX, dsK, ce, dc, partial, ticket, compliance);
     } else {
         element_energy_kernel<<<(unsigned)nblocks, 256, 0, st>>>(g, U, CX, dsK, ce, dc, partial, ticket, compliance);
@@ -276,7 +280,7 @@ void launch_element_energy(const Grid &g, const double *U, const double *CX, con
                            double *compliance, cudaStream_t st)
 {
     long long nb = (g.nel() + 255) / 256;
-    if (nb > 1184) nb = 1184;
+    if (nb > kEnergyCtas) nb = kEnergyCtas;
     if (nb < 1) nb = 1;
     launch_element_energy_blocks(g, U, CX, dsK, ce, dc, partial, ticket, compliance, (int)nb, st);
 }

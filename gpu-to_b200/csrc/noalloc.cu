@@ -15,9 +15,11 @@
 
 namespace gputo {
 
-// One partial sum per CTA; each CTA covers kNoAllocElemsPerCta elements.
+// One partial sum per CTA.  The dense kernel (a Ke without the cube element's
+// pattern) takes one CTA per kNoAllocElemsPerCta elements.
 constexpr int kNoAllocSlots = 8192;
 constexpr long long kNoAllocElemsPerCta = 2048;   // 256 threads x 8 elements
+static_assert(kNoAllocSlots >= kEnergyCtas, "a slot per CTA of the marching kernel");
 constexpr long long kNoAllocMaxElements = kNoAllocSlots * kNoAllocElemsPerCta;  // 16,777,216
 
 struct NoAllocScratch {

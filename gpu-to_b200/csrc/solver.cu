@@ -191,6 +191,7 @@ int Solver::create(int nelx, int nely, int nelz, int nl_, const gputo_options *o
                             2 * hsweep_blocks<float>(g[0], MODE_JACOBI_DOT, 8, true),
                             2 * hsweep_blocks<float>(g[0], MODE_JACOBI_DOT, 0, true),
                             2 * hsweep_blocks<double>(g[0], MODE_ENERGY), 1 << 12});
+    static_assert((1 << 12) >= kEnergyCtas, "a slot per CTA of the energy pass");
     ALLOC(partial, partial_cap);
     ALLOC(ticket, 4);
     ALLOC(sc, 1);

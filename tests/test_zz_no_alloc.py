@@ -75,3 +75,22 @@ def test_noalloc_rejects_grids_above_its_scratch(gputo):
                                                1, 1, 1, 512, 256, 256, 1, 1, ctypes.byref(c), None)
     assert st == gputo.GPUTO_ERR_ARG
     assert b"16,777,216" in lib.gputo_last_error()
+
+
+@pytest.mark.parametrize("shape", [(24, 16, 16), (64, 32, 32), (9, 2, 300), (128, 64, 64)])
+def test_both_entry_points_run_the_same_ctas(gputo, shape):
+    """The energy pass is planned for the CTAs it launches, whichever entry point: the compliance is the same partial
+    sums in the same order, so the same bits (a plan for hundreds of CTAs run on a few took up to six times as
+    long)."""
+    import torch
+    lib = gputo.lib()
+    nel, ndof = int(np.prod(shape)), 3 * int(np.prod([d + 1 for d in shape]))
+    Ke0 = np.ascontiguousarray(gputo.hex8_stiffness().reshape(-1))
+    rng = np.random.default_rng(5)
+    dev = dict(dtype=torch.float64, device="cuda")
+    U, CX = torch.as_tensor(rng.standard_normal(ndof), **dev), torch.as_tensor(rng.uniform(0.05, 1.0, nel), **dev)
+    ce, dc = torch.empty(nel, **dev), torch.empty(nel, **dev)
+    torch.cuda.synchronize()
+    c = [_call(lib, f, Ke0, U, CX, CX, shape, ce, dc)
+         for f in ("gputo_compliance_sens_dev", "gputo_compliance_sens_noalloc_dev")]
+    assert c[0] == c[1]
