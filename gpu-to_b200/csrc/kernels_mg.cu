@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "gputo_internal.h"
+#include "rounded.h"
 
 namespace gputo {
 
@@ -1052,30 +1053,17 @@ void launch_dense_fix(const Grid &g, const uint8_t *mask, double *AQ, cudaStream
 // 256 x 128 x 128 grid), so all kernels, and the inverse below, run back to
 // back under programmatic dependent launch: a kernel lets the next one launch
 // at its start and waits for its predecessor before it reads anything.
-// Square roots and quotients are the correctly rounded ones, from an
-// approximate reciprocal square root and fused remainders (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34, 1990): a chain of five FMAs instead of two library
-// calls on the pivots' critical path.  Measured for 675 unknowns, kernels
-// serialised: 22 panel steps of 13.4 us and 21 trailing updates of 6.5 us; 16.3
-// us (a CTA with a thread per entry, two divisions per entry and column), 14.0
-// us and 9.0 us as separate diagonal, panel and trailing kernels, with the same
-// bits.  The inverse below took 0.27 ms and takes 0.11 ms (tile_product).
+// Square roots and quotients come from rounded.h.  Measured for 675 unknowns,
+// kernels serialised: 22 panel steps of 13.4 us and 21 trailing updates of 6.5
+// us; 16.3 us (a CTA with a thread per entry, two divisions per entry and
+// column), 14.0 us and 9.0 us as separate diagonal, panel and trailing kernels,
+// with the same bits.  The inverse below took 0.27 ms and takes 0.11 ms
+// (tile_product).  Every CTA of a panel step factors the diagonal block again,
+// which pays at all sizes: a whole setup takes 1.6, 8.8 and 91 ms with 1728,
+// 4131 and 10,125 coarse unknowns, 3.8, 19 and 199 ms as separate kernels.
 // info = 1-based index of the first non-positive (or NaN) pivot, 0 on
 // success; once set, every later factor kernel returns at once.
 constexpr int kCholB = 32;
-
-// s / d for y = 1 / d to about 2^-51: the product's remainder corrects it to
-// the rounded quotient (its error before the last rounding is about 2^-103).
-__device__ __forceinline__ double div_by(double s, double d, double y)
-{
-    const double q = s * y;
-    return fma(fma(-q, d, s), y, q);
-}
-
-// Pivots in this range keep every product and remainder above clear of
-// overflow and of subnormal numbers; others take sqrt and /.
-__device__ __forceinline__ bool pivot_in_range(double s) { return s > 1e-200 && s < 1e200; }
 
 // The lower triangle of the w x w block in Ds (row-major) -> its factor in Ls,
 // one warp, lane r holding row r in registers: column j's pivot comes by a
@@ -1098,8 +1086,7 @@ __device__ __forceinline__ int chol_block(int w, const double (*Ds)[kCholB + 1],
         double d, l, y = 0.0;
         if (pivot_in_range(s)) {
             y = rsqrt(s);
-            const double g = s * y;
-            d = fma(fma(-g, g, s), 0.5 * y, g);
+            d = sqrt_by(s, y);
             l = div_by(D[j], d, y);
         } else {
             d = sqrt(s);
