@@ -224,9 +224,14 @@ packed_sweep_kernel(Lay L, const T *__restrict__ A, const T *__restrict__ u,
 // launch (griddepcontrol.launch_dependents: its entry loads overlap this
 // kernel's tail), and only then waits for its predecessor before it reads u,
 // f or 1/diag.  Kernels before a sweep that write the matrices (the setup)
-// never release their successors early, so they have completed by then.
-template <typename T, int MODE, bool EARLY>
-__global__ void __launch_bounds__(256, sizeof(T) == 8 && EARLY ? 1 : 0)
+// never release their successors early, so they have completed by then.  In
+// FP64 the entries take 144 registers and a CTA fills an SM (206 to 254
+// registers a thread), with the loads before the wait as with them after it:
+// an iteration of FP64 solves takes 441 us at 128 x 64 x 64 (299 CTAs on its
+// largest such level; 458 with them after the wait) and 776 us at 160 x 80 x
+// 80 (788), and a 64 x 32 x 32 solve 5.67 ms (6.01).
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 1 : 0)
 packed_sweep_slot_kernel(Lay L, const T *__restrict__ A, const T *__restrict__ u, const T *__restrict__ f,
                          const T *__restrict__ rdiag, const uint8_t *__restrict__ mask, T *__restrict__ out,
                          T omega, T prerelax, const int *__restrict__ done)
@@ -244,20 +249,15 @@ packed_sweep_slot_kernel(Lay L, const T *__restrict__ A, const T *__restrict__ u
     const long long nel = g.nel();
     const long long e = slot ? g.elem(ei, ej, ek) : 0;
     const int a = local_index(1 - ex, 1 - ey, 1 - ez);
-    // EARLY: all 72 entries in registers before the wait (launch_packed_sweep)
     T am[3][24];   // rows 3 a + d of the slot's element matrix
-    auto load_entries = [&]() {
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
+    for (int d = 0; d < 3; ++d)
 #pragma unroll
-            for (int col = 0; col < 24; ++col)
-                am[d][col] = slot ? A[(long long)packed_index(3 * a + d, col) * nel + e] : T(0);
-    };
-    if (EARLY) load_entries();
+        for (int col = 0; col < 24; ++col)
+            am[d][col] = slot ? A[(long long)packed_index(3 * a + d, col) * nel + e] : T(0);
     pdl_trigger();
     pdl_wait();
     if (done && *done) return;
-    if (!EARLY) load_entries();
     // warp 0's epilogue operands, loaded together with the products' inputs
     // instead of after the slot sum
     T fe[3] = {T(0), T(0), T(0)}, re[3] = {T(0), T(0), T(0)}, ue[3] = {T(0), T(0), T(0)};
@@ -326,21 +326,6 @@ packed_sweep_slot_kernel(Lay L, const T *__restrict__ A, const T *__restrict__ u
     }
 }
 
-template <typename T, bool EARLY>
-static void slot_sweep(int mode, unsigned nb, const Lay &L, const T *Apk, const T *u, const T *f, const T *rdiag,
-                       const uint8_t *mask, T *out, T omega, T prerelax, const int *done, cudaStream_t st)
-{
-    auto go = [&](auto *kernel) {
-        launch_pdl(kernel, dim3(nb), dim3(256), 0, st, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done);
-    };
-    switch (mode) {
-    case MODE_APPLY: go(packed_sweep_slot_kernel<T, MODE_APPLY, EARLY>); break;
-    case MODE_DEFECT: go(packed_sweep_slot_kernel<T, MODE_DEFECT, EARLY>); break;
-    case MODE_JACOBI: go(packed_sweep_slot_kernel<T, MODE_JACOBI, EARLY>); break;
-    default: go(packed_sweep_slot_kernel<T, MODE_JACOBI_PRE, EARLY>);
-    }
-}
-
 template <typename T>
 void launch_packed_sweep(int mode, const Lay &L, const T *Apk, const T *u, const T *f,
                          const T *rdiag, const uint8_t *mask, T *out, T omega, T prerelax,
@@ -349,13 +334,15 @@ void launch_packed_sweep(int mode, const Lay &L, const T *Apk, const T *u, const
     const int bs = 128;
     if (L.g.nnod() < 65536) {
         const unsigned sb = (unsigned)((L.g.nnod() + 31) / 32);
-        // FP64's 72 entries take 144 registers, one CTA per SM: early loads pay
-        // while every CTA has an SM of its own (a 64 x 32 x 32 FP64 solve 6.01 ->
-        // 5.67 ms)
-        if (sizeof(T) == 4 || sb <= 148)
-            slot_sweep<T, true>(mode, sb, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done, st);
-        else
-            slot_sweep<T, false>(mode, sb, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done, st);
+        auto go = [&](auto *kernel) {
+            launch_pdl(kernel, dim3(sb), dim3(256), 0, st, L, Apk, u, f, rdiag, mask, out, omega, prerelax, done);
+        };
+        switch (mode) {
+        case MODE_APPLY: go(packed_sweep_slot_kernel<T, MODE_APPLY>); break;
+        case MODE_DEFECT: go(packed_sweep_slot_kernel<T, MODE_DEFECT>); break;
+        case MODE_JACOBI: go(packed_sweep_slot_kernel<T, MODE_JACOBI>); break;
+        default: go(packed_sweep_slot_kernel<T, MODE_JACOBI_PRE>);
+        }
         count_launches(1);
         return;
     }
