@@ -277,8 +277,8 @@ struct ConvArgs {
 // of each dy and the mid and lo parts of all: products of hi parts and weights
 // have 16 bits, few of which are lost in the K / 16 adds of a chain, and the
 // four sums are added with rounding.  With one accumulator per segment the
-// output is low by 1.2e-7; now by 3e-8, and its error against 64 bits is 2.7e-7
-// of the norm (6.3e-7 with FP32 FMA chains), for 10 % of the forward pass.
+// output is low by 1.2e-7; now by 3e-8, and its error against 64 bits is 1.6e-7
+// of the norm (4.1e-7 with FP32 FMA chains), for 10 % of the forward pass.
 //
 // Persistent, weights resident (110 KB for 32 x 64).  Copies, MMAs and drains
 // overlap but share the shared memory and TMEM ports, and none of them alone
@@ -286,8 +286,8 @@ struct ConvArgs {
 // of the MMAs, 399 without drains and epilogue, 303 without both.  Of those 303
 // about 76 are the first layer, the rest the nine reads of the activations
 // (0.49 GB for 16 -> 32 and 0.98 GB for 32 -> 64).  Measured at 129 x 65 x 65:
-// 32 -> 64 with the head 280 us (0.8 PFLOP/s of BF16 MMAs; 3167 + 50 us as
-// direct FP32 convolutions on the CUDA cores), 16 -> 32 115 us (733 us).
+// 32 -> 64 with the head 270 us (0.8 PFLOP/s of BF16 MMAs; 3167 + 50 us as
+// direct FP32 convolutions on the CUDA cores), 16 -> 32 112 us (733 us).
 template <int CK, int CN> struct ConvCfg {
     static constexpr int C8 = CK / 8;
     static constexpr int RS = kRows + 2;                    // rows of a segment
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(192) conv_tc_kernel(ConvArgs A, RowGeo q)
 // are coalesced along Y.  Weight gradients are reduced per (co, ci) pair by
 // one CTA in a fixed order, so training is deterministic.  Bound by FP32 FMAs
 // and, in the weight gradients, by their index arithmetic: eight 33^3 samples
-// take 15.5 ms, of which the weight gradients 8.6, the data gradients 3.8 and
+// take 15.7 ms, of which the weight gradients 8.6, the data gradients 3.8 and
 // the forward passes 2.4 ms.  (On the tensor cores a step took 1.4 ms, but its
 // sums differ in their last bits, and with them every later step.)
 // ---------------------------------------------------------------------------
