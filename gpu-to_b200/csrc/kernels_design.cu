@@ -134,28 +134,32 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // 114 x 82 x 50 31 us; 148, 92 and 62 us with a thread per element gathering
 // its 24 corner values and a one-thread sum of the CTAs' partials.  Tiles of 8
 // rows took 82, 67 and 33 us.
-constexpr int kEnY = 32, kEnZ = 4, kEnT = 32 * kEnZ, kEnRing = 4;
-constexpr int kEnRow = 3 * (kEnY + 1), kEnPlane = kEnRow * (kEnZ + 1), kEnPos = (kEnPlane + kEnT - 1) / kEnT;
+// Thin grids have tiles of their own (FIXED = false, energy_tile()).
+constexpr int kEnY = 32, kEnZ = 4, kEnT = kEnY * kEnZ, kEnRing = 4;
 
+template <bool FIXED>
 __global__ void __launch_bounds__(kEnT, 512 / kEnT)
-element_energy_march_kernel(Grid g, HC<double> hc, int xc, int ntj, int ntk, long long nitems,
+element_energy_march_kernel(Grid g, HC<double> hc, int ty_, int tz_, int xc, int ntj, int ntk, long long nitems,
                             const double *__restrict__ U, const double *__restrict__ CX,
                             const double *__restrict__ dsK, double *__restrict__ ce, double *__restrict__ dc,
                             double *__restrict__ partial, unsigned *ticket, double *compliance)
 {
-    __shared__ double ring[kEnRing][kEnPlane];
-    const int tid = threadIdx.x, l = tid & 31, w = tid >> 5;
+    // values of a plane tile: 3 (ty + 1) (tz + 1) is largest at 1 x kEnT columns
+    constexpr int kMax = FIXED ? 3 * (kEnY + 1) * (kEnZ + 1) : 3 * 2 * (kEnT + 1), kPos = (kMax + kEnT - 1) / kEnT;
+    __shared__ double ring[kEnRing][kMax];
+    const int ty = FIXED ? kEnY : ty_, tz = FIXED ? kEnZ : tz_, row = 3 * (ty + 1), plane = row * (tz + 1);
+    const int tid = threadIdx.x, w = tid / ty, l = tid - w * ty;
     const long long ps = 3LL * (g.ny + 1) * (g.nz + 1);   // values per node plane
     double csum = 0.0;
     for (long long item = blockIdx.x; item < nitems; item += gridDim.x) {
         const long long tile = item % ((long long)ntj * ntk);
         const int i0 = (int)(item / ((long long)ntj * ntk)) * xc, i1 = min(i0 + xc, g.nx);
-        const int j0 = (int)(tile % ntj) * kEnY, k0 = (int)(tile / ntj) * kEnZ;
+        const int j0 = (int)(tile % ntj) * ty, k0 = (int)(tile / ntj) * tz;
         const int np = i1 - i0 + 1;
-        long long off[kEnPos];   // this thread's values of a plane tile, clamped to the grid
+        long long off[kPos];   // this thread's values of a plane tile, clamped to the grid
 #pragma unroll
-        for (int q = 0; q < kEnPos; ++q) {
-            const int p = tid + kEnT * q, kk = p / kEnRow, c = p - kk * kEnRow;
+        for (int q = 0; q < kPos; ++q) {
+            const int p = tid + kEnT * q, kk = p / row, c = p - kk * row;
             const int v = min(3 * j0 + c, 3 * g.ny + 2);
             off[q] = (long long)min(k0 + kk, g.nz) * (3 * (g.ny + 1)) + v;
         }
@@ -164,13 +168,13 @@ element_energy_march_kernel(Grid g, HC<double> hc, int xc, int ntj, int ntk, lon
                 const double *src = U + (i0 + t) * ps;
                 double *dst = ring[t % kEnRing];
 #pragma unroll
-                for (int q = 0; q < kEnPos; ++q)
-                    if (tid + kEnT * q < kEnPlane) cp_async8(dst + tid + kEnT * q, src + off[q]);
+                for (int q = 0; q < kPos; ++q)
+                    if (tid + kEnT * q < plane) cp_async8(dst + tid + kEnT * q, src + off[q]);
             }
             cp_async_commit();
         };
         const int j = j0 + l, k = k0 + w;
-        const bool mine = j < g.ny && k < g.nz;
+        const bool mine = j < g.ny && k < g.nz && (FIXED || w < tz);
         const long long es = (long long)g.ny * g.nz;
         long long e = (long long)i0 * es + (long long)k * g.ny + j;   // element in front of plane t
         __syncthreads();   // the ring is free
@@ -180,13 +184,13 @@ element_energy_march_kernel(Grid g, HC<double> hc, int xc, int ntj, int ntk, lon
             cp_async_wait<kEnRing - 2>();
             __syncthreads();   // plane t has landed for everyone; slot (t - 1) is free
             fetch(t + kEnRing - 1);
-            const double *P = ring[t % kEnRing] + w * kEnRow + 3 * l;
+            const double *P = ring[t % kEnRing] + (FIXED ? w : min(w, tz - 1)) * row + 3 * l;
 #pragma unroll
             for (int cy = 0; cy < 2; ++cy)
 #pragma unroll
                 for (int cz = 0; cz < 2; ++cz)
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) F[(2 * cy + cz) * 4 + d] = P[cz * kEnRow + 3 * cy + d];
+                    for (int d = 0; d < 3; ++d) F[(2 * cy + cz) * 4 + d] = P[cz * row + 3 * cy + d];
             face_h(F);
         };
         auto element = [&](const double (&Fp)[HF], const double (&Fn)[HF], double cx, double ds) {
@@ -245,6 +249,21 @@ static int chunk_planes(int nx, long long tiles, long long slots, int extra)
     return best;
 }
 
+// Columns of a CTA of the energy pass.  Up to 16 elements along y, or two along
+// z, 32 x 4 columns would lie outside the grid for the most part, so a CTA
+// takes all of that direction and what its threads allow of the other.
+static void energy_tile(const Grid &g, int &ty, int &tz)
+{
+    ty = kEnY, tz = kEnZ;
+    if (g.ny <= 16) {
+        ty = g.ny;
+        tz = std::min(kEnT / ty, g.nz);
+    } else if (g.nz <= 2) {
+        tz = g.nz;
+        ty = std::min(kEnT / tz, g.ny);
+    }
+}
+
 // One partial slot per CTA: kEnergyCtas of them, or nblocks for the dense
 // kernel.  The plan's CTAs are the launch's: with the dense kernel's count of
 // 256-thread CTAs as their limit a CTA ran many short chunks, each filling the
@@ -263,12 +282,15 @@ void launch_element_energy_blocks(const Grid &g, const double *U, const double *
         hk = g_design_hk[dev < 64 ? dev : 63];
     }
     if (hk.ok) {
-        const int ntj = (g.ny + kEnY - 1) / kEnY, ntk = (g.nz + kEnZ - 1) / kEnZ;
+        int ty, tz;
+        energy_tile(g, ty, tz);
+        const int ntj = (g.ny + ty - 1) / ty, ntk = (g.nz + tz - 1) / tz;
         const long long tiles = (long long)ntj * ntk;
         const int xc = chunk_planes(g.nx, tiles, (512 / kEnT) * 148, 5);
         const long long items = tiles * ((g.nx + xc - 1) / xc);
-        element_energy_march_kernel<<<(unsigned)std::min<long long>(items, kEnergyCtas), kEnT, 0, st>>>(
-            g, make_hc<double>(hk), xc, ntj, ntk, items, U, CX, dsK, ce, dc, partial, ticket, compliance);
+        auto *kernel = ty == kEnY && tz == kEnZ ? element_energy_march_kernel<true> : element_energy_march_kernel<false>;
+        kernel<<<(unsigned)std::min<long long>(items, kEnergyCtas), kEnT, 0, st>>>(
+            g, make_hc<double>(hk), ty, tz, xc, ntj, ntk, items, U, CX, dsK, ce, dc, partial, ticket, compliance);
     } else {
         element_energy_kernel<<<(unsigned)nblocks, 256, 0, st>>>(g, U, CX, dsK, ce, dc, partial, ticket, compliance);
     }

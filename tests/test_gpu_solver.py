@@ -8,6 +8,8 @@ mixed-precision solves agree with an FP64 solve to 1e-10 within 1e-6 in
 compliance and relative displacement L2, at tol 1e-8 on a small grid and at
 tol 1e-6 (the benchmark's tolerance) on the 256x128x128 benchmark workload.
 """
+import time
+
 import numpy as np
 import pytest
 from conftest import load_golden
@@ -251,6 +253,39 @@ def test_element_energy_tiles_and_chunks(oracle, gputo, torch, shape):
     assert np.abs(ce.cpu().numpy() - ce_ref).max() <= 1e-12 * np.abs(ce_ref).max()
     assert np.abs(dc.cpu().numpy() - dsK * ce_ref).max() <= 1e-12 * np.abs(dsK * ce_ref).max()
     assert abs(c - CX @ ce_ref) <= 1e-12 * abs(CX @ ce_ref)
+
+
+@pytest.mark.parametrize("shape", [(5, 1, 200), (5, 1, 1), (6, 3, 90), (3, 16, 17), (3, 17, 9), (4, 300, 1), (3, 131, 2),
+                                   (40, 4, 4), (40, 100, 1)])
+def test_element_energy_thin_grids(oracle, gputo, torch, shape):
+    """Tiles of whole rows along y or z: several along the other direction, a ragged last one, threads to spare."""
+    test_element_energy_tiles_and_chunks(oracle, gputo, torch, shape)
+
+
+def _call_ms(torch, call):
+    """Median time of 20 calls (they synchronise)."""
+    for _ in range(3):
+        call()
+    ts = []
+    for _ in range(20):
+        t0 = time.perf_counter()
+        call()
+        ts.append(time.perf_counter() - t0)
+    return 1e3 * sorted(ts)[10]
+
+
+@pytest.mark.parametrize("thin", [(1024, 1, 1024), (512, 4, 512), (1024, 1024, 1)])
+def test_element_energy_of_thin_grids_takes_no_longer(gputo, torch, thin):
+    """As many elements as 128 x 64 x 128, and 1.4 times the bytes at one element across: at most twice the time (14
+    times with 32 x 4 columns per CTA whatever the grid)."""
+    def ms(shape):
+        nel, ndof = int(np.prod(shape)), 3 * int(np.prod([d + 1 for d in shape]))
+        U = torch.randn(ndof, dtype=torch.float64, device="cuda")
+        CX, ce, dc = (torch.rand(nel, dtype=torch.float64, device="cuda") for _ in range(3))
+        torch.cuda.synchronize()
+        Ke = gputo.hex8_stiffness()
+        return _call_ms(torch, lambda: gputo.compliance_sens_dev(Ke, U, CX, CX, *shape, ce, dc))
+    assert ms(thin) <= 2 * ms((128, 64, 128))
 
 
 @pytest.mark.parametrize("rmin", [3 ** 0.5, 2 * 3 ** 0.5, 1.2, 2.5, 4.5, 0.9])
