@@ -310,6 +310,21 @@ def test_density_filter_matches_oracle(oracle, gputo, rmin, shape):
     assert np.abs(got2 - out2).max() <= 1e-13 * np.abs(out2).max()
 
 
+@pytest.mark.parametrize("nz", [3, 8, 9, 16, 17])
+def test_density_filter_of_flat_grids(oracle, gputo, nz):
+    """Radius 2 with one, two and four rows per thread, at the heights where that changes."""
+    test_density_filter_matches_oracle(oracle, gputo, 2.5, (21, 35, nz))
+
+
+def test_density_filter_of_flat_grids_takes_no_longer(gputo, torch):
+    """As many elements as 200^3, and the same bytes: at most 1.8 times the time (2.5 times with tiles of 32 rows)."""
+    x, out, div = (torch.rand(200 ** 3, dtype=torch.float64, device="cuda") + 0.5 for _ in range(3))
+    torch.cuda.synchronize()
+    ms = [_call_ms(torch, lambda: gputo.density_filter_dev(x, out, *shape, 2.5, divisor=div, normalize=False))
+          for shape in ((1000, 1000, 8), (200, 200, 200))]
+    assert ms[0] <= 1.8 * ms[1]
+
+
 def test_bad_arguments_return_status(oracle, gputo):
     p = oracle.cantilever(16, 8, 8)
     CX = np.ones(p.nel)
