@@ -426,8 +426,8 @@ struct NetDims {
 // Each solver that a network is attached to has its own set: solvers that
 // share a network run at the same time (the members of a batch do).
 struct NetWork {
-    void *img = nullptr;                           // BF16 weight operands of the tensor-core convolutions
-    uint4 *rows1 = nullptr, *rows2 = nullptr;      // activations of layers 1 and 2 (split rows)
+    void *img = nullptr;                           // BF16 weight operands of the tensor-core convolutions, and behind them
+    uint4 *rows1 = nullptr, *rows2 = nullptr;      // the activations of layers 1 and 2 (split rows)
     long long cap_rows = 0;
     int *h_err = nullptr, *d_err = nullptr;        // mapped host flag of the bounded waits
 

@@ -37,6 +37,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <functional>
+#include <mutex>
 #include <vector>
 
 #include "gputo_internal.h"
@@ -847,12 +849,57 @@ int Net::create(unsigned long long seed)
     return GPUTO_OK;
 }
 
+// Mapped host flags for the bounded waits.  Allocating mapped memory takes 1 to
+// 3 ms, more than the rest of a small network's first pass, so one page serves
+// the process: a slot per NetWork, given back with it, and memory of its own
+// for those that find no slot.
+namespace {
+struct FlagPage {
+    static constexpr int kSlots = 1024;
+    std::mutex mu;
+    int *page = nullptr;
+    std::vector<int *> free;
+
+    int *take()
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!page) {
+            if (cudaHostAlloc((void **)&page, kSlots * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) !=
+                cudaSuccess) {
+                page = nullptr;
+                return nullptr;
+            }
+            for (int i = kSlots; i-- > 0;) free.push_back(page + i);
+        }
+        int *f = nullptr;
+        if (!free.empty()) {
+            f = free.back();
+            free.pop_back();
+        } else if (cudaHostAlloc((void **)&f, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            return nullptr;
+        }
+        *f = 0;
+        return f;
+    }
+    void give_back(int *f)
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (std::less_equal<int *>()(page, f) && std::less<int *>()(f, page + kSlots)) free.push_back(f);
+        else cudaFreeHost(f);
+    }
+};
+
+FlagPage &flag_page()
+{
+    static FlagPage *p = new FlagPage;   // outlives every network
+    return *p;
+}
+}  // namespace
+
 void NetWork::release()
 {
-    cudaFree(img);
-    cudaFree(rows1);
-    cudaFree(rows2);
-    if (h_err) cudaFreeHost(h_err);
+    cudaFree(img);   // waits for kernels that may still write the flag
+    if (h_err) flag_page().give_back(h_err);
     img = nullptr;
     rows1 = rows2 = nullptr;
     h_err = d_err = nullptr;
@@ -863,19 +910,21 @@ int NetWork::reserve(const NetDims &d)
 {
     if (!h_err) {
         // where a kernel's bounded wait reports that it gave up: read by the host after a synchronisation
-        GPUTO_CUDA(cudaHostAlloc((void **)&h_err, sizeof(int), cudaHostAllocMapped));
-        *h_err = 0;
+        h_err = flag_page().take();
+        if (!h_err) GPUTO_CUDA(cudaErrorMemoryAllocation);
         GPUTO_CUDA(cudaHostGetDevicePointer((void **)&d_err, h_err, 0));
     }
-    if (!img) GPUTO_CUDA(cudaMalloc(&img, 2 * (size_t)(kImg2 + kImg3)));
     const long long rows = row_geo(d).R;
     if (rows <= cap_rows) return GPUTO_OK;
-    cudaFree(rows1);
-    cudaFree(rows2);
+    cudaFree(img);
+    img = nullptr;
     rows1 = rows2 = nullptr;
     cap_rows = 0;
-    GPUTO_CUDA(cudaMalloc(&rows1, 16 * 6 * (size_t)rows));
-    GPUTO_CUDA(cudaMalloc(&rows2, 16 * 12 * (size_t)rows));
+    constexpr size_t wbytes = 2 * (size_t)(kImg2 + kImg3);
+    static_assert(wbytes % 256 == 0, "the rows behind it start as aligned as the allocation");
+    GPUTO_CUDA(cudaMalloc(&img, wbytes + 16 * 18 * (size_t)rows));
+    rows1 = reinterpret_cast<uint4 *>((char *)img + wbytes);
+    rows2 = rows1 + 6 * rows;
     cap_rows = rows;
     return GPUTO_OK;
 }

@@ -13,6 +13,7 @@
 import json
 import os
 import sys
+import time
 
 import numpy as np
 import pytest
@@ -257,3 +258,50 @@ def test_attaching_another_network_replaces_the_captured_one(gputo):
     (r2, n2), U2 = run(s2, F)
     assert (r1, n1) == (r2, n2) and torch.equal(U1, U2)
     assert not torch.equal(U0, U1)
+
+
+def test_networks_beyond_the_page_of_flags(gputo):
+    """More networks at a time than the process keeps flags for: each reports its own failed pass, and none of the
+    others, also where a flag has had another owner."""
+    import torch
+    dims, n = (3, 4, 5), 60
+    x = torch.as_tensor(np.random.default_rng(1).standard_normal(4 * n), dtype=torch.float32, device="cuda")
+    ok, y = (torch.empty(3 * n, dtype=torch.float32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    for count in (1030, 3):
+        nets = [gputo.Net(seed=5) for _ in range(count)]
+        for net in nets:
+            net.forward(x, dims, ok)
+        for net in (nets[0], nets[-1]):
+            gputo.debug_set_sweep_fault(skip_stage=0, wait_us=200)
+            try:
+                with pytest.raises(gputo.GputoError) as e:
+                    net.forward(x, dims, y)
+                assert e.value.status == gputo.GPUTO_ERR_TIMEOUT
+            finally:
+                gputo.debug_set_sweep_fault(-1, 0)
+            for other in (nets[1], nets[-2], net):
+                other.forward(x, dims, y)
+                assert torch.equal(y, ok)
+        for net in nets:
+            net.close()
+
+
+def test_first_pass_of_a_small_network(gputo):
+    """A new network's first pass on a small grid allocates once: less than half of what making the network takes (as
+    long as that, and longer, when it allocates host memory that the device can write)."""
+    import torch
+    dims, n = (9, 9, 9), 729
+    x, y = (torch.rand(c * n, device="cuda") for c in (4, 3))
+    torch.cuda.synchronize()
+    made, first = [], []
+    for _ in range(12):
+        t = [time.perf_counter()]
+        net = gputo.Net(seed=6)
+        t.append(time.perf_counter())
+        net.forward(x, dims, y)
+        t.append(time.perf_counter())
+        net.close()
+        made.append(t[1] - t[0])
+        first.append(t[2] - t[1])
+    assert np.median(first) <= 0.5 * np.median(made)
