@@ -1061,20 +1061,36 @@ __device__ __forceinline__ double dprj_v(double v, double eta, double beta)
     return beta * (1.0 - t * t) / (tanh(beta * eta) + tanh(beta * (1.0 - eta)));
 }
 
-// The Newton sums need, per element, t = tanh(beta (v - eta)) and sech^2 times
-// sinh(v beta) sinh((1 - v) beta).  With E = exp(2 beta v), which does not
-// change between the steps (one exponential per element, kept in ex), and
-// a = E exp(-2 beta eta), q = 1 / (a + 1):
-//   t = (a - 1) q,
-//   sech^2 sinh sinh = 2 q^2 (a cosh(beta) - (a E exp(-beta) + exp(beta - 2 beta eta)) / 2),
-// one division instead of a tanh, a cosh and two sinh.  The exponentials'
-// rounding is that of an argument 2^-53 / (2 beta) away, so for beta from 0.5
-// on it is that of v and eta themselves (the mean's error against 80 bits is
-// 2e-17 either way at 0.5 and 1, 1e-17 against 1e-19 at 200); below, a - 1
-// loses the bits that tanh keeps (error 3e-17 against 3e-18 at 0.25, 2e-11 at
-// 1e-6, and no threshold is found at 1e-10).  So beta below 0.5 or above 300,
-// and elements whose E leaves 1e-150 .. 1e150 (or a passes it), take the direct
-// formulas.  The design itself is projected with tanh.
+// The Newton sums need, per element, t = tanh(beta (v - eta)) and deta, which
+// is -beta / sinh(beta) times sech^2 times sinh(v beta) sinh((1 - v) beta).
+// Both come from one value per element that does not change between the steps
+// (kept in ex), with one division instead of a tanh, a cosh and two sinh:
+//  * beta < 2: from V = tanh(beta v), with H = tanh(beta eta), D = tanh(beta)
+//    and u = 1 - V H,
+//      t = (V - H) / u,  deta = -(beta / D) (1 - H^2) V (D - V) / u^2;
+//  * beta from 2 to 300: from E = exp(2 beta v), with a = E exp(-2 beta eta)
+//    and q = 1 / (a + 1),
+//      t = (a - 1) q,
+//      sech^2 sinh sinh = 2 q^2 (a cosh(beta) - (a E exp(-beta) + exp(beta - 2 beta eta)) / 2).
+// As beta goes to zero a - 1 loses the bits of t that V - H keeps, and as V and
+// H go to one u loses those that a keeps.  The error that each leaves in eta,
+// against 80 bits and over that of the direct formulas, is 0.9 to 1.1 for the
+// first form from 0.02 to 1.9, and for the second 1.2 at 2, 1.2 to 1.5 (below
+// one ulp of eta) from 4 to 300, but 1.5 at 1, 2.4 at 0.5 and 26 at 0.02.
+// Other betas, and elements out of the range in which a form is good, take the
+// direct formulas.  The design itself is projected with tanh.
+
+// exp(x y) with the rounding of the product made up for: at large exponents it
+// is many times that of exp.
+__device__ __forceinline__ double exp_product(double x, double y)
+{
+    const double p = x * y, e = exp(p);
+    return fma(e, fma(x, y, -p), e);
+}
+
+enum ProjForm { PROJ_TANH, PROJ_EXP, PROJ_DIRECT };
+
+template <int FORM>
 __global__ void __launch_bounds__(kLoopThreads, kLoopPerSm)
 projection_kernel(long long n, const double *__restrict__ xt, double beta, double volfrac, double eta, double *ex,
                   double *partial, LoopSync *sync, LoopWait lw, int max_steps, ProjState *state, double *__restrict__ xphys,
@@ -1082,19 +1098,23 @@ projection_kernel(long long n, const double *__restrict__ xt, double beta, doubl
 {
     __shared__ double tot[2];
     const long long i0 = (long long)blockIdx.x * kLoopThreads + threadIdx.x, st = (long long)gridDim.x * kLoopThreads;
-    const bool fast_beta = beta >= 0.5 && beta <= 300.0;
     unsigned round = 0;
     bool ok = true, done = false;
     int steps = 0;
     for (int k = 0; k < max_steps && ok && !done; ++k) {
         const double t0 = tanh(beta * eta), den = t0 + tanh(beta * (1.0 - eta));
-        const double c = exp(-2.0 * beta * eta), eb = exp(beta), emb = exp(-beta), ch = 0.5 * (eb + emb);
+        const double t1 = FORM == PROJ_TANH ? tanh(beta) : 0.0, c = FORM == PROJ_EXP ? exp_product(-2.0 * beta, eta) : 0.0;
+        const double eb = exp(beta), emb = exp(-beta), ch = 0.5 * (eb + emb);
         const double half_ceb = 0.5 * c * eb, half_emb = 0.5 * emb;
-        const double kd = -2.0 * beta / sinh(beta);
+        const double kd = FORM == PROJ_TANH ? -(beta / t1) * (1.0 - t0 * t0) : -2.0 * beta / sinh(beta);
         double s[2] = {0.0, 0.0};   // sums of tanh(beta (v - eta)) and of deta
         auto add = [&](long long i, double E) {
-            const double a = E * c;
-            if (E > 1e-150 && E < 1e150 && a < 1e150) {
+            const double a = FORM == PROJ_TANH ? fma(-E, t0, 1.0) : E * c;   // u of the first form
+            if (FORM == PROJ_TANH && a > 0.01 && fabs(E) < 1.0) {
+                const double q = 1.0 / a;
+                s[0] = fma(E - t0, q, s[0]);
+                s[1] = fma(kd * (q * q), E * (t1 - E), s[1]);
+            } else if (FORM == PROJ_EXP && E > 1e-150 && E < 1e150 && a < 1e150) {
                 const double q = 1.0 / (a + 1.0);
                 s[0] = fma(a - 1.0, q, s[0]);
                 s[1] = fma(kd * (q * q), fma(a, ch, -fma(a * E, half_emb, half_ceb)), s[1]);
@@ -1103,6 +1123,9 @@ projection_kernel(long long n, const double *__restrict__ xt, double beta, doubl
                 s[1] += deta_v(xt[i], eta, beta);
             }
         };
+        auto once = [&](double v) {
+            return FORM == PROJ_TANH ? tanh(beta * v) : FORM == PROJ_EXP ? exp_product(2.0 * beta, v) : 0.0;
+        };
         // two elements in flight per thread
         for (long long i = i0; i < n; i += 2 * st) {
             const long long j = i + st;
@@ -1110,8 +1133,8 @@ projection_kernel(long long n, const double *__restrict__ xt, double beta, doubl
             double E, F = 0.0;
             if (k == 0) {
                 const double u = xt[i], v = two ? xt[j] : 0.0;
-                E = fast_beta ? exp(2.0 * beta * u) : 0.0;
-                F = fast_beta ? exp(2.0 * beta * v) : 0.0;
+                E = once(u);
+                F = once(v);
                 ex[i] = E;
                 if (two) ex[j] = F;
             } else {
@@ -1165,7 +1188,10 @@ int launch_heaviside(long long n, const double *xt, double volfrac, double beta,
     LoopSync *ls = (LoopSync *)sync;
     LoopWait lw = loop_wait();
     void *args[] = {&n, &xt, &beta, &volfrac, &eta0, &ex, &partial, &ls, &lw, &max_steps, &ps, &xphys, &dprj};
-    GPUTO_CUDA(cudaLaunchCooperativeKernel((const void *)projection_kernel, dim3((unsigned)loop_blocks(n)),
+    const void *kernel = beta < 2.0      ? (const void *)projection_kernel<PROJ_TANH>
+                         : beta <= 300.0 ? (const void *)projection_kernel<PROJ_EXP>
+                                         : (const void *)projection_kernel<PROJ_DIRECT>;
+    GPUTO_CUDA(cudaLaunchCooperativeKernel(kernel, dim3((unsigned)loop_blocks(n)),
                                            dim3(kLoopThreads), args, 0, st));
     count_launches(1);
     return GPUTO_OK;
