@@ -84,6 +84,11 @@ class ClockSampler:
                 stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
+            # nvidia-smi may take longer to start than a short timed region lasts
+            end = time.time() + 5
+            while not self.lines and self.proc.poll() is None and time.time() < end:
+                time.sleep(0.01)
+            self.lines.clear()
         except Exception:
             self.proc = None
         return self
